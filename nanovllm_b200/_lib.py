@@ -9,9 +9,10 @@ import ctypes
 import os
 from ctypes import c_char_p, c_double, c_float, c_int32, c_int64, c_void_p
 
-from .build import LIB_PATH, build
+from .build import build, build_native
 
 _lib = None
+_native = None
 
 # name -> (restype, argtypes); mirrors include/b200_attn.h one to one
 SIGNATURES = {
@@ -63,6 +64,17 @@ def load():
         fn.argtypes = args
     _lib = lib
     return lib
+
+
+def native():
+    """The compiled binding of the hot entry points (csrc/native.cpp), built like load() if it is missing or stale."""
+    global _native
+    if _native is None:
+        load()
+        build_native()
+        from . import _native as module
+        _native = module
+    return _native
 
 
 class B200AttnError(RuntimeError):

@@ -9,7 +9,7 @@ What it replaces in nano-vllm's model runner, per decode step:
 * the graph branch of `ModelRunner.run_model` (:193-203): seven device operations that move those
   tensors into the graph's static buffers.
 
-Here the step is packed with numpy into ONE persistent pinned record (layout: include/b200_attn.h,
+Here the step is packed by compiled code (csrc/native.cpp) into ONE persistent pinned record (layout: include/b200_attn.h,
 b200_unpack_decode_metadata), copied once, and scattered into the graph buffers by one kernel.  The
 values are the reference's, bit for bit: input_ids = last tokens, positions = len - 1,
 context_lens = len, slot = last block id * block_size + tokens in the last block - 1, block-table rows
@@ -19,8 +19,6 @@ padded with -1 to the longest row of the step.
 keeps the reference's own run_model and reads views of the copied record.
 """
 from __future__ import annotations
-
-from itertools import chain
 
 import numpy as np
 import torch
@@ -40,6 +38,7 @@ class DecodeMetadataStager:
         self._host = [torch.empty(words, dtype=torch.int32, pin_memory=pin) for _ in range(2)]
         self._np = [h.numpy() for h in self._host]
         self._dev = [torch.empty(words, dtype=torch.int32, device=self.device) for _ in range(2)] if pin else [None, None]
+        self._native = _lib.native()
         self._turn = 0
         self.batch = 0
         self.width = 0
@@ -47,35 +46,10 @@ class DecodeMetadataStager:
     # ---- host side (no GPU needed) ---------------------------------------------------------------------
     def pack(self, seqs) -> np.ndarray:
         """Fills the next pinned record from the scheduler's sequences; returns it as int32 words."""
-        bs = len(seqs)
-        if bs > self.max_batch:
-            raise ValueError(f"decode batch {bs} exceeds the stager's capacity {self.max_batch}")
-        self._turn ^= 1
-        rec = self._np[self._turn]
-        tables = [s.block_table for s in seqs]
-        nblk = np.fromiter(map(len, tables), dtype=np.int64, count=bs)
-        w = int(nblk.max()) if bs else 0
-        if w > self.max_blocks:
-            raise ValueError(f"block table of {w} blocks exceeds the stager's capacity {self.max_blocks}")
-        total = int(nblk.sum())
-        flat = np.fromiter(chain.from_iterable(tables), dtype=np.int32, count=total)
-        ntok = np.fromiter(map(len, seqs), dtype=np.int64, count=bs)
-        ids64 = rec[:2 * bs].view(np.int64)
-        pos64 = rec[2 * bs:4 * bs].view(np.int64)
-        ids64[:] = np.fromiter((s.last_token for s in seqs), dtype=np.int64, count=bs)
-        pos64[:] = ntok - 1
-        ends = np.cumsum(nblk)
-        # Sequence.last_block_num_tokens (nanovllm/engine/sequence.py:60-62) with num_blocks = ceil(len / block_size)
-        last_tokens = ntok - ((ntok + self.block_size - 1) // self.block_size - 1) * self.block_size
-        rec[4 * bs:5 * bs] = flat[ends - 1].astype(np.int64) * self.block_size + last_tokens - 1
-        rec[5 * bs:6 * bs] = ntok
-        bt = rec[6 * bs:6 * bs + bs * w].reshape(bs, w)
-        bt.fill(-1)
-        rows = np.repeat(np.arange(bs), nblk)
-        cols = np.arange(total) - np.repeat(ends - nblk, nblk)
-        bt[rows, cols] = flat
-        self.batch, self.width = bs, w
-        return rec[:6 * bs + bs * w]
+        turn = self._turn ^ 1
+        bs, w = self._native.pack_decode(seqs, self._host[turn], self.max_batch, self.max_blocks, self.block_size)
+        self._turn, self.batch, self.width = turn, bs, w
+        return self._np[turn][:6 * bs + bs * w]
 
     def record_views(self, rec):
         """(input_ids, positions, slot_mapping, context_lens, block_tables) as views of a packed record
@@ -88,21 +62,13 @@ class DecodeMetadataStager:
     # ---- device side -----------------------------------------------------------------------------------
     def to_device(self) -> torch.Tensor:
         """One host-to-device copy of the record packed last; returns the device record."""
-        n = 6 * self.batch + self.batch * self.width
-        dev = self._dev[self._turn]
-        dev[:n].copy_(self._host[self._turn][:n], non_blocking=True)
-        return dev[:n]
+        return self._native.upload_record(self._host[self._turn], self._dev[self._turn], 6 * self.batch + self.batch * self.width)
 
     def unpack_into(self, dev_record, input_ids, positions, slot_mapping, context_lens, block_tables):
         """One launch: the device record into the graph's static buffers, with the reference's effect
         (nanovllm/engine/model_runner.py:196-202)."""
-        assert block_tables.stride(1) == 1 and input_ids.dtype == torch.int64 and positions.dtype == torch.int64
-        assert slot_mapping.numel() == context_lens.numel() and input_ids.numel() >= self.batch
-        lib = _lib.load()
-        _lib.check(lib.b200_unpack_decode_metadata(
-            dev_record.data_ptr(), self.batch, self.width, slot_mapping.numel(), block_tables.stride(0),
-            input_ids.data_ptr(), positions.data_ptr(), slot_mapping.data_ptr(), context_lens.data_ptr(),
-            block_tables.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        self._native.unpack_decode_metadata(dev_record, self.batch, self.width, input_ids, positions, slot_mapping,
+                                            context_lens, block_tables)
 
 
 def install_into(model_runner_cls, context_module):
