@@ -22,7 +22,7 @@ HEADER = os.path.join(os.path.dirname(PKG_DIR), "include", "b200_attn.h")
 LIB_PATH = os.path.join(PKG_DIR, "libb200attn.so")
 NATIVE_SOURCE = os.path.join(CSRC, "native.cpp")
 NATIVE_PATH = os.path.join(PKG_DIR, "_native" + sysconfig.get_config_var("EXT_SUFFIX"))
-SOURCES = ["host.cu", "store_kvcache.cu", "decode_attn.cu", "prefill_attn_mma.cu", "prefill_attn_tc2.cu", "prefill_attn.cu", "qk_norm_rope_store.cu", "decode_metadata.cu", "small_allreduce.cu"]
+SOURCES = ["host.cu", "store_kvcache.cu", "decode_attn.cu", "decode_cluster.cu", "prefill_attn_mma.cu", "prefill_attn_tc2.cu", "prefill_attn.cu", "qk_norm_rope_store.cu", "decode_metadata.cu", "small_allreduce.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-shared", "-Xcompiler", "-fPIC"]
 

@@ -46,6 +46,24 @@ int make_tokens_heads_map_cols32(CUtensorMap* map, const void* base, uint64_t to
 
 #ifdef __CUDACC__
 
+// Launch with programmatic stream serialization: the kernel may start while the one in front of it in the stream still
+// runs, if that one lets it (griddepcontrol.launch_dependents), and waits for it itself (griddepcontrol.wait).
+template <typename... Params, typename... Args>
+inline cudaError_t launch_early(void (*kernel)(Params...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream,
+                                Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // ---------------------------------------------------------------------------------------------
 // Bounded waiting.  Every spin in this library gives up after kSpinLimitCycles (about a second)
 // and reports through a status word instead of hanging the GPU.
@@ -74,6 +92,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// The same without suspending the thread.
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
       : "r"(smem_u32(bar)), "r"(parity)

@@ -2,191 +2,199 @@
 // nanovllm/layers/attention.py:71-74).
 //
 // HBM-bound: every K and V byte of every context token is read exactly once.  Design:
-//  * Work unit = one 64-token tile of one (sequence, kv head).  The tiles of all sequences and
-//    heads form one flat list (sequence -> head -> tile), derived on the device from context_lens
-//    by a block scan in every CTA: the launch geometry never depends on device data, as CUDA-graph
-//    replay requires.  The list is cut into contiguous PIECES: one equal static piece per CTA
-//    of the persistent grid (2 CTAs per SM) covering about 70 % of the tiles, then one larger and
-//    four smaller pieces per CTA handed out through an atomic ticket counter, so that CTAs that
-//    stream faster take more of the tail and all finish together.
-//  * The producer warp (one elected lane) walks its pieces.  For every (sequence, head) segment it
-//    publishes a descriptor in shared memory, bulk-copies the segment's G query rows into a small
-//    ring, and issues the TMA tile loads (two 64x64 boxes for K, two for V, 128-byte swizzle;
-//    16-token boxes for the ragged last tile of a sequence) into a ring of stages guarded by
-//    full/empty mbarriers.  The descriptor and the query rows ride on the full-barrier of the
-//    segment's first tile, and metadata of the next segment is fetched one segment ahead, so the
-//    ring never drains at sequence or piece boundaries.
+//  * Work unit = one (sequence, kv head) pair, whole, or, where a pair is longer than half of a CTA's equal share of
+//    the batch, one of the equal parts it is cut into.  Persistent CTAs (2 per SM) take the units longest first: the
+//    first ones statically, the others through an atomic ticket, so that CTAs that stream faster take more and the
+//    short units level the end.  Order and cuts are derived on the device from context_lens by every CTA alike: the
+//    launch geometry never depends on device data, as CUDA-graph replay requires.  (Equal static pieces of
+//    one flat tile list, the earlier form, cut nearly every pair of a batch of a few hundred pairs and paid for it
+//    with partials at the end of the launch; whole pairs in HBM order also stream faster: 176 -> 164 us on 256
+//    sequences of 100 .. 2048 tokens, 16/8 heads, 7.0 TB/s.)  Batches with few pairs go to decode_cluster.cu.
+//  * The producer warp (one elected lane) walks the CTA's units.  For every unit it publishes a descriptor in shared
+//    memory, bulk-copies the G query rows into a small ring, and issues the TMA tile loads (64 tokens: two 64x64
+//    boxes for K, two for V, 128-byte swizzle; 16-token boxes for the ragged last tile of a sequence) into a
+//    ring of stages guarded by full/empty mbarriers.  The descriptor and the query rows ride on the full-barrier of the
+//    unit's first tile, and the next unit and its metadata are fetched one unit ahead, so the ring never drains at
+//    unit boundaries.
 //  * Four consumer warps take 16 tokens of each tile: QK^T and PV on mma.sync.m16n8k16 (the G
 //    query heads of the kv head are rows of the 16-row A operand), online softmax in fp32 with
-//    quad shuffles.  At the end of a segment they only drop their running (m, l, O) into shared
-//    memory and go on with the next tile.
-//  * An epilogue warp combines the four warps' states and writes the bf16 row, or, where a piece
-//    boundary cuts the (sequence, head), a partial (m, l, unnormalised O) to the workspace; the
-//    last piece to arrive (one atomic counter per (sequence, head), reset by that warp) merges the
-//    partials.  No CTA ever waits for another; every mbarrier wait is bounded.
+//    quad shuffles.  At the end of a unit they only drop their running (m, l, O) into shared
+//    memory and go on with the next tile; the CTA's last unit they finish themselves.
+//  * An epilogue warp combines the four warps' states and writes the bf16 row, or, for a part of a cut pair, a
+//    partial (m, l, unnormalised O) to the workspace; the last part to arrive (one atomic counter per pair, reset by
+//    that warp) merges the partials.  No CTA ever waits for another; every mbarrier wait is bounded.
 #include "../../include/b200_attn.h"
-#include "kernels.cuh"
+#include "decode_common.cuh"
 
 namespace b200 {
 extern std::atomic<long long> g_launches;
 
-constexpr int kTile = 64;                       // tokens per stage
-constexpr int kSubTileBytes = kTile * 128;      // 64 tokens x 64 dims bf16
-constexpr int kStageBytes = 4 * kSubTileBytes;  // K lo, K hi, V lo, V hi
 constexpr int kDecStages = 3;
-constexpr int kDecConsumerWarps = 4;
-constexpr int kDecConsumers = kDecConsumerWarps * 32;
 constexpr int kDecProducerWarp = kDecConsumerWarps;
 constexpr int kDecEpilogueWarp = kDecConsumerWarps + 1;
 constexpr int kDecThreads = kDecConsumers + 64;
+constexpr int kDecWarps = kDecThreads / 32;
 constexpr int kDecMaxBatch = 512;               // per launch; the host splits larger batches
 constexpr int kDecPer = (kDecMaxBatch + kDecThreads - 1) / kDecThreads;
-constexpr int kMaxG = 16;
-constexpr int kWsStatusBytes = 256;  // header: word 0 is the ticket counter of the piece scheduler
+constexpr int kWsStatusBytes = 256;  // header: word 0 is the ticket counter of the scheduler
 constexpr int kWsCounterInts = kDecMaxBatch * 128;   // arrival counters: fixed region, up to 128 kv heads
-constexpr int kSegRing = kDecStages + 1;   // segment descriptors / query rows in flight
+constexpr int kUnitRing = kDecStages + 1;  // unit descriptors / query rows in flight
 constexpr int kDecPending = 8;             // partials written but not yet counted, per CTA
-// Geometry of the dynamic tail of the piece scheduler (measured on B200): used from 256 tiles per CTA;
-// one piece of 15 % and four of 3.75 % of a CTA's equal share are handed out through tickets.
-constexpr int kDynFactor = 256, kDynBigPct = 15, kDynSmallPct100 = 375, kDynSmallN = 4;
+constexpr int kDecClasses = 64;            // length classes of the sort
+constexpr int kSortRows = kDecPer * kDecWarps;
+constexpr int kDecMinPart = 4;             // tiles: shorter parts would cost more to merge than to stream
+constexpr int kPartialSlots = 12;          // of the workspace, per CTA of the grid
 static __device__ int g_status_decode = 0;
 
-struct DecodeParams {
-  const __nv_bfloat16* q;
-  long long q_row_stride;
-  __nv_bfloat16* out;
-  const int* context_lens;
-  const int* block_tables;
-  long long bt_row_stride;
-  int bt_cols;
-  int batch, H, Hkv, G;
-  int block_size;
-  long long num_blocks;
-  float scale_log2;
-  int n_merge;    // hand-off buffers between the consumer warps and the epilogue warp (1 or 2)
-  int dyn_factor; // work per CTA (tiles) from which the dynamic tail is used
-  int big_pct, small_pct100, small_n;  // geometry of the dynamic tail
-  float* ws_o;    // [2 * pieces][G][128] unnormalised partial outputs
-  float* ws_ml;   // [2 * pieces][G][2]   running max (log2 domain) and sum
-  int* counters;  // [batch * Hkv], zero between launches
-  unsigned int* ticket;  // piece scheduler, zero between launches
-};
-
-
-// One (sequence, kv head) segment inside one piece, as the producer hands it to the other warps.
-struct SegDesc {
-  int seq;               // -1: no more work for this CTA
-  int h;
-  int t0, t1;            // tiles [t0, t1) of the (sequence, head) that lie in the piece
-  int nt;                // tiles of the whole (sequence, head)
+// One unit as the producer hands it to the other warps.
+struct UnitDesc {
+  int seq, h;
+  int t0, t1;            // tiles [t0, t1) of the pair
   int len;               // context length, clamped to the block table's capacity
-  int slot;              // workspace slot for a partial: 2 * piece + (does the piece start inside it ? 0 : 1)
-  int pad;
-  long long seg_start;   // flat position of tile 0 of the (sequence, head)
+  int parts;             // parts the pair is cut into (1: whole)
+  int part0, slot;       // workspace slots of the pair's first part and of this one (consecutive parts: Hkv apart)
 };
 
-// How the flat tile list [0, T) is cut into pieces.  Pieces are numbered in list order:
-//   [0, g)            static, one per CTA, equal sizes, together the first Ts tiles;
-//   [g, g + nb)       "big" dynamic pieces of Cb tiles;
-//   [g + nb, total)   "small" dynamic pieces of Cs tiles, ending exactly at T.
-// Every CTA computes the same geometry from T and the grid size.
-struct DecPieces {
-  long long T, Ts, Tb_end;
-  int g, nb, ns, Cb, Cs;
-  __device__ __forceinline__ int dynamic() const { return nb + ns; }
-  __device__ __forceinline__ long long start(int i) const {
-    if (i < g) return static_cast<long long>(i) * Ts / g;
-    if (i < g + nb) return Ts + static_cast<long long>(i - g) * Cb;
-    return Tb_end + static_cast<long long>(i - g - nb) * Cs;
-  }
-  __device__ __forceinline__ int of(long long x) const {
-    if (x < Ts) return static_cast<int>(((x + 1) * g - 1) / Ts);
-    if (x < Tb_end) return g + static_cast<int>((x - Ts) / Cb);
-    return g + nb + static_cast<int>((x - Tb_end) / Cs);
+// The units of a launch, the same in every CTA.  Chunk x of [0, chunks) in order of length is part (x - base[r]) of the
+// r-th longest sequence; unit u is kv head u % Hkv of chunk u / Hkv.
+struct DecUnits {
+  const unsigned short *order, *base, *nt;   // shared memory: sequences by length, first chunk of each, tiles by sequence
+  const unsigned char* tail;                 // tokens of a sequence's last tile - 1
+  int cap;                                   // tiles a part may have
+  int live;                                  // sequences with tokens
+  bool split, wide;                          // some pair is cut; some tile count does not fit 16 bits
+  __device__ __forceinline__ UnitDesc get(const DecodeParams& p, int u) const {
+    UnitDesc d;
+    const int x = u / p.Hkv;
+    d.h = u - x * p.Hkv;
+    int r = x, part = 0;
+    if (split) {
+      int lo = 0, hi = live;
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (base[mid] <= x) lo = mid; else hi = mid;
+      }
+      r = lo;
+      part = x - base[r];
+    }
+    d.seq = order[r];
+    int n = nt[d.seq];
+    d.len = (n - 1) * kTile + tail[d.seq] + 1;
+    if (wide) {
+      d.len = min(p.context_lens[d.seq], p.bt_cols * p.block_size);
+      n = (d.len + kTile - 1) / kTile;
+    }
+    d.parts = split ? (n + cap - 1) / cap : 1;
+    d.t0 = split ? static_cast<int>(static_cast<long long>(part) * n / d.parts) : 0;
+    d.t1 = split ? static_cast<int>(static_cast<long long>(part + 1) * n / d.parts) : n;
+    d.slot = u;
+    d.part0 = u - part * p.Hkv;
+    return d;
   }
 };
 
-__device__ __forceinline__ DecPieces dec_pieces(long long T, int grid, int dyn_factor, int big_pct, int small_pct100,
-                                              int small_n) {
-  DecPieces pc;
-  pc.T = T;
-  pc.g = T < grid ? static_cast<int>(T) : grid;
-  if (T < static_cast<long long>(dyn_factor) * grid) {          // too little work to be worth a dynamic tail
-    pc.Ts = pc.Tb_end = T;
-    pc.nb = pc.ns = 0;
-    pc.Cb = pc.Cs = 1;
-    return pc;
-  }
-  const long long W = T / grid;   // tiles per CTA if all ran at the same speed
-  pc.Cs = static_cast<int>((W * small_pct100 + 5000) / 10000);   // small_pct100 / 100 % of W each, small_n per CTA
-  pc.Cb = static_cast<int>((W * big_pct + 50) / 100);            // big_pct % of W, one per CTA
-  if (pc.Cs < 1) pc.Cs = 1;
-  if (pc.Cb < 1) pc.Cb = 1;
-  pc.nb = grid;
-  pc.ns = small_n * grid;
-  pc.Ts = T - static_cast<long long>(pc.nb) * pc.Cb - static_cast<long long>(pc.ns) * pc.Cs;
-  pc.Tb_end = pc.Ts + static_cast<long long>(pc.nb) * pc.Cb;
-  return pc;
+__device__ __forceinline__ int ld_acquire_gpu(const int* ptr) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(ptr) : "memory");
+  return v;
 }
 
-// The segment that starts at flat position x inside a piece [.., r_end).
-__device__ __forceinline__ SegDesc dec_locate(const int* s_prefix, int batch, int Hkv, long long x, long long r_begin,
-                                              long long r_end, int piece) {
-  int lo = 0, hi = batch;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (static_cast<long long>(s_prefix[mid]) * Hkv <= x) lo = mid; else hi = mid;
+// Merges into r (query head gq) the partials of n of the pair's parts; `mine` >= 0: all but that slot's (the caller holds
+// it).  Eight partials a trip: their maxima and sums travel together with their rows.
+__device__ __forceinline__ void dec_merge_partials(const DecodeParams& p, int part0, int n, int mine, int gq, int lane, DecPart& r) {
+#pragma unroll 1
+  for (int first = 0; first < n; first += 8) {
+    // lane j (mod 8) looks after partial first + j
+    const int j = first + (lane & 7);
+    int slot = part0 + (j < n ? j : n - 1) * p.Hkv;
+    if (mine >= 0 && slot >= mine) slot += p.Hkv;
+    const int row = slot * p.G + gq;
+    float2 ml = __ldcg(reinterpret_cast<const float2*>(p.ws_ml + row * 2));
+    float4 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int ru = __shfl_sync(0xffffffffu, row, u);
+      if (first + u < n) v[u] = __ldcg(reinterpret_cast<const float4*>(p.ws_o + static_cast<long long>(ru) * 128 + lane * 4));
+    }
+    if (j >= n) ml = make_float2(-INFINITY, 0.f);
+    float M = ml.x;
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
+    M = fmaxf(M, r.M);
+    const float w = fast_exp2(ml.x - M), w0 = fast_exp2(r.M - M);
+    float L = ml.y * w;
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) L += __shfl_xor_sync(0xffffffffu, L, off);
+    r.M = M;
+    r.L = r.L * w0 + L;
+    r.v.x *= w0; r.v.y *= w0; r.v.z *= w0; r.v.w *= w0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const float wu = __shfl_sync(0xffffffffu, w, u);
+      if (first + u < n) {
+        r.v.x += v[u].x * wu; r.v.y += v[u].y * wu;
+        r.v.z += v[u].z * wu; r.v.w += v[u].w * wu;
+      }
+    }
   }
-  SegDesc d;
-  d.seq = lo;
-  d.nt = s_prefix[lo + 1] - s_prefix[lo];
-  const long long rem = x - static_cast<long long>(s_prefix[lo]) * Hkv;
-  d.h = static_cast<int>(rem / d.nt);
-  d.t0 = static_cast<int>(rem - static_cast<long long>(d.h) * d.nt);
-  d.seg_start = x - d.t0;
-  const long long seg_end = d.seg_start + d.nt;
-  const long long my_end = seg_end < r_end ? seg_end : r_end;
-  d.t1 = d.t0 + static_cast<int>(my_end - x);
-  d.slot = piece * 2 + (d.seg_start <= r_begin ? 0 : 1);
-  d.len = 0;
-  d.pad = 0;
-  return d;
 }
 
-// 1-D bulk copy global -> shared, completion counted on an mbarrier (addresses and size multiples of 16).
-__device__ __forceinline__ void bulk_load_1d(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
+// L2 prefetch of the full tiles among [t0, t1), which lie in the blocks of table columns col0 and col0 + 1.
+__device__ __forceinline__ void dec_prefetch_tiles(const DecodeParams& p, const CUtensorMap& map_k, const CUtensorMap& map_v, int h,
+                                                   int t0, int t1, int len, const int* bt, int col0, int blk0, int blk1) {
+  for (int t = t0; t < t1; ++t) {
+    const int tok0 = t * kTile, col = tok0 / p.block_size;
+    if (tok0 + kTile > len) return;
+    const int blk = col == col0 ? blk0 : col == col0 + 1 ? blk1 : -1;
+    if (blk < 0 || blk >= p.num_blocks) return;
+    const int slot0 = static_cast<int>(blk * static_cast<long long>(p.block_size)) + (tok0 - col * p.block_size);
+    tma_prefetch_l2_3d(&map_k, 0, h, slot0);
+    tma_prefetch_l2_3d(&map_k, 64, h, slot0);
+    tma_prefetch_l2_3d(&map_v, 0, h, slot0);
+    tma_prefetch_l2_3d(&map_v, 64, h, slot0);
+  }
+}
+
+__device__ __forceinline__ void dec_store_partial(const DecodeParams& p, int slot, int gq, int lane, const DecPart& r) {
+  *reinterpret_cast<float4*>(p.ws_o + (static_cast<long long>(slot) * p.G + gq) * 128 + lane * 4) = r.v;
+  if (lane == 0) *reinterpret_cast<float2*>(p.ws_ml + (slot * p.G + gq) * 2) = make_float2(r.M, r.L);
 }
 
 __global__ void __launch_bounds__(kDecThreads, 2)
 decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map_k,
                    const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_k16,
                    const __grid_constant__ CUtensorMap map_v16) {
-  extern __shared__ unsigned char smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) unsigned char smem[];
   const int G = p.G, Hkv = p.Hkv;
   unsigned char* stages = smem;
-  __nv_bfloat16* s_q = reinterpret_cast<__nv_bfloat16*>(smem + kDecStages * kStageBytes);          // [kSegRing][G][128]
-  float* merge_o = reinterpret_cast<float*>(s_q + kSegRing * G * 128);                            // [n_merge][4][G][128]
+  __nv_bfloat16* s_q = reinterpret_cast<__nv_bfloat16*>(smem + kDecStages * kStageBytes);          // [kUnitRing][G][128]
+  float* merge_o = reinterpret_cast<float*>(s_q + kUnitRing * G * 128);                           // [n_merge][4][G][128]
   float* merge_ml = merge_o + p.n_merge * kDecConsumerWarps * G * 128;                              // [n_merge][4][G][2]
-  int* s_prefix = reinterpret_cast<int*>(merge_ml + p.n_merge * kDecConsumerWarps * G * 2);       // [batch + 1]
+  unsigned short* s_order = reinterpret_cast<unsigned short*>(merge_ml + p.n_merge * kDecConsumerWarps * G * 2);
+  unsigned short* s_base = s_order + kDecMaxBatch;
+  unsigned short* s_nt = s_base + kDecMaxBatch;
+  unsigned char* s_tail = reinterpret_cast<unsigned char*>(s_nt + kDecMaxBatch);
   __shared__ __align__(8) uint64_t bar_full[kDecStages];
   __shared__ __align__(8) uint64_t bar_empty[kDecStages];
   __shared__ __align__(8) uint64_t bar_merge_full[2];
   __shared__ __align__(8) uint64_t bar_merge_empty[2];
-  __shared__ __align__(16) SegDesc s_desc[kSegRing];
-  __shared__ __align__(16) SegDesc s_merge_desc[2];
-  __shared__ __align__(16) SegDesc s_pending[kDecPending];
-  __shared__ int s_warp_sums[kDecThreads / 32];
-  __shared__ int s_abort;
+  __shared__ __align__(8) uint64_t bar_decide, bar_part, bar_final;
+  __shared__ __align__(16) UnitDesc s_desc[kUnitRing];
+  __shared__ __align__(16) UnitDesc s_merge_desc[2];
+  __shared__ __align__(16) UnitDesc s_pending[kDecPending];
+  __shared__ int s_warp_sums[kDecWarps], s_warp_max[kDecWarps], s_warp_live[kDecWarps];
+  __shared__ int s_abort, s_known, s_last, s_decision, s_merge_all;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int max_len = p.bt_cols * p.block_size;
 
   if (tid == 0) {
     s_abort = 0;
+    s_known = 0;
+    s_last = -1;
+    mbar_init(&bar_decide, 1);
+    mbar_init(&bar_part, kDecConsumerWarps);
+    mbar_init(&bar_final, 1);
     for (int s = 0; s < kDecStages; ++s) {
       mbar_init(&bar_full[s], 1);
       mbar_init(&bar_empty[s], kDecConsumerWarps);
@@ -200,18 +208,28 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
 
   // Launched with programmatic stream serialization: the kernel may start while the previous kernel
   // of the stream is still running, if that kernel allows it (griddepcontrol.launch_dependents; only
-  // this library's store and producer kernels do, any other kernel has completed before this one
-  // starts).  Those kernels write K/V rows of the cache and the query rows, never the metadata, so
-  // the scan over context_lens, the piece geometry and the first block-table reads below run ahead;
+  // this library's store, producer and decode kernels do, any other kernel has completed before this one
+  // starts).  Those kernels write K/V rows of the cache, query rows and outputs, never the metadata, so
+  // the scan over context_lens and the first block-table reads below run ahead;
   // every thread that goes on to touch q, the cache, the output or the workspace first executes
-  // griddepcontrol.wait (the consumer warps only ever read shared memory filled after it).
+  // griddepcontrol.wait (the consumer warps only touch them after data that was loaded behind it).
 
-  // ---- tile counts per sequence and their exclusive prefix (block scan) ----
+  // ---- the units of the launch: lengths -> parts -> order ----
+  DecUnits un;
+  un.order = s_order;
+  un.base = s_base;
+  un.nt = s_nt;
+  un.tail = s_tail;
+  int units;
   {
+    // scratch of the sort, in the stage memory that no load has been issued into yet: sequences per (round, warp) and class
+    uint32_t* const s_cnt = reinterpret_cast<uint32_t*>(stages);                    // [kSortRows][kDecClasses / 2], two a word
+    unsigned short* const cnt = reinterpret_cast<unsigned short*>(s_cnt);
+    for (int i = tid; i < kSortRows * kDecClasses / 2; i += kDecThreads) s_cnt[i] = 0;
     const int per = (p.batch + kDecThreads - 1) / kDecThreads;
     const int i0 = tid * per;
     int local[kDecPer];
-    int sum = 0;
+    int sum = 0, longest = 0, live = 0;
 #pragma unroll
     for (int k = 0; k < kDecPer; ++k) {
       int nt = 0;
@@ -220,29 +238,127 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
         int len = p.context_lens[i];
         len = len < 0 ? 0 : (len > max_len ? max_len : len);
         nt = (len + kTile - 1) / kTile;
+        s_nt[i] = static_cast<unsigned short>(nt < 65535 ? nt : 65535);
+        s_tail[i] = static_cast<unsigned char>((len - 1) & (kTile - 1));
       }
       local[k] = nt;
       sum += nt;
+      longest = max(longest, nt);
+      live += nt > 0;
     }
-    int incl = sum;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, incl, off);
-      if (lane >= off) incl += v;
-    }
-    if (lane == 31) s_warp_sums[warp] = incl;
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    live = __reduce_add_sync(0xffffffffu, live);
+    if (lane == 0) { s_warp_sums[warp] = sum; s_warp_max[warp] = longest; s_warp_live[warp] = live; }
     __syncthreads();
-    int excl = incl - sum;
-    for (int w = 0; w < warp; ++w) excl += s_warp_sums[w];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    long long total = 0;
+    longest = live = 0;
+#pragma unroll
+    for (int w = 0; w < kDecWarps; ++w) {
+      total += s_warp_sums[w];
+      longest = max(longest, s_warp_max[w]);
+      live += s_warp_live[w];
+    }
+    // Pairs are cut only if the longest one is well above a CTA's equal share of the tiles: whole pairs, longest first,
+    // level out well enough below that and leave nothing to merge.  The line is 1.25 shares, or 1.85 where
+    // every CTA has at most one pair (short and long ones share an SM then, and the long one gets the SM's bandwidth when
+    // the short one is done).  Above it, pairs longer than 2/3 of a share (and kDecMinPart tiles) are cut into
+    // equal parts: 1/2 and 1/3 leave parts of a size that do not add up to a share, and cost more merges (measured over
+    // batches of 16 .. 500 sequences of 1 .. 8192 tokens).  The parts come first in the order, so that their merging
+    // happens while the whole pairs stream.  A part is longer than a third of a share, so there are at most
+    // 3 x grid of them: the workspace's kPartialSlots x grid slots hold every partial.
+    const long long tiles = total * Hkv;
+    const int line = live * Hkv <= static_cast<int>(gridDim.x) ? 185 : 125;
+    un.cap = longest;
+    if (static_cast<long long>(longest) * gridDim.x * 100 > line * tiles) {
+      const long long part = 2 * tiles / (3 * static_cast<int>(gridDim.x)) + 1;
+      un.cap = static_cast<int>(part < kDecMinPart ? kDecMinPart : part < longest ? part : longest);
+    }
+    un.live = live;
+    un.split = longest > un.cap;
+    un.wide = longest >= 65535;
+    // size classes: without cuts all 64 for the whole pairs, else 32 for the parts and, behind them, 32 for the whole pairs
+    const int top = un.split ? un.cap : longest, classes = un.split ? kDecClasses / 2 : kDecClasses;
+    // Longest first: a stable counting sort by length class (longest -> class 0).  Every CTA must arrive at
+    // the same order, so places within a class follow from (round, warp, lane), not from who comes first.
+    int cls[kDecPer], pos[kDecPer];
 #pragma unroll
     for (int k = 0; k < kDecPer; ++k) {
-      const int i = i0 + k;
-      if (k < per && i < p.batch) {
-        s_prefix[i] = excl;
-        excl += local[k];
-        if (i == p.batch - 1) s_prefix[p.batch] = excl;
+      cls[k] = -1;
+      if (local[k] > 0) {
+        const int parts = (local[k] + un.cap - 1) / un.cap;
+        const int part = parts == 1 ? local[k] : (local[k] + parts - 1) / parts;
+        cls[k] = static_cast<int>(static_cast<unsigned>(top - part) * (classes - 1) / static_cast<unsigned>(top));
+        if (un.split && parts == 1) cls[k] += classes;
+      }
+      const unsigned same = __match_any_sync(0xffffffffu, cls[k]);
+      pos[k] = __popc(same & ((1u << lane) - 1));
+      if (pos[k] == 0 && cls[k] >= 0) cnt[(k * kDecWarps + warp) * kDecClasses + cls[k]] = static_cast<unsigned short>(__popc(same));
+    }
+    __syncthreads();
+    if (warp == 0) {
+      // lane owns classes 2 * lane and 2 * lane + 1 (the halves of a word; no sum exceeds kDecMaxBatch)
+      uint32_t v[kSortRows], sum2 = 0;
+#pragma unroll
+      for (int r = 0; r < kSortRows; ++r) v[r] = s_cnt[r * (kDecClasses / 2) + lane];
+#pragma unroll
+      for (int r = 0; r < kSortRows; ++r) sum2 += v[r];
+      const uint32_t both = (sum2 & 0xffff) + (sum2 >> 16);
+      uint32_t in = both;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, in, off);
+        if (lane >= off) in += x;
+      }
+      uint32_t at = (in - both) | ((in - (sum2 >> 16)) << 16);        // first place of either class
+#pragma unroll
+      for (int r = 0; r < kSortRows; ++r) {
+        s_cnt[r * (kDecClasses / 2) + lane] = at;
+        at += v[r];
       }
     }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kDecPer; ++k)
+      if (cls[k] >= 0) s_order[cnt[(k * kDecWarps + warp) * kDecClasses + cls[k]] + pos[k]] = static_cast<unsigned short>(i0 + k);
+    units = live * Hkv;
+    if (un.split) {
+      // first chunk of every sequence, in that order
+      __syncthreads();
+      int parts[kDecPer], mine = 0;
+#pragma unroll
+      for (int k = 0; k < kDecPer; ++k) {
+        parts[k] = 0;
+        if (k < per && i0 + k < live) {
+          int n = s_nt[s_order[i0 + k]];
+          if (un.wide) n = (min(p.context_lens[s_order[i0 + k]], max_len) + kTile - 1) / kTile;
+          parts[k] = (n + un.cap - 1) / un.cap;
+        }
+        mine += parts[k];
+      }
+      int incl = mine;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += v;
+      }
+      if (lane == 31) s_warp_live[warp] = incl;     // (its first use is two barriers back)
+      __syncthreads();
+      int at = incl - mine, chunks = 0;
+#pragma unroll
+      for (int w = 0; w < kDecWarps; ++w) {
+        if (w < warp) at += s_warp_live[w];
+        chunks += s_warp_live[w];
+      }
+#pragma unroll
+      for (int k = 0; k < kDecPer; ++k) {
+        if (k < per && i0 + k < live) s_base[i0 + k] = static_cast<unsigned short>(at);
+        at += parts[k];
+      }
+      units = chunks * Hkv;
+    }
+    fence_proxy_async_smem();                        // the loads write over the scratch
     __syncthreads();
   }
 
@@ -250,18 +366,17 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
   if (warp == kDecEpilogueWarp) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (int i = blockIdx.x; i < p.batch; i += gridDim.x) {
-      if (s_prefix[i + 1] == s_prefix[i]) {
+      if (s_nt[i] == 0) {
         uint4* o = reinterpret_cast<uint4*>(p.out + static_cast<long long>(i) * p.H * 128);
         for (int v = lane; v < p.H * 16; v += 32) o[v] = make_uint4(0, 0, 0, 0);
       }
     }
   }
 
-  const long long T = static_cast<long long>(s_prefix[p.batch]) * Hkv;  // tiles in this launch
-  const DecPieces pc = dec_pieces(T, static_cast<int>(gridDim.x), p.dyn_factor, p.big_pct, p.small_pct100, p.small_n);
   const int cta = blockIdx.x;
-  if (cta >= pc.g) return;
-
+  const int n_first = min(units, static_cast<int>(gridDim.x));     // units handed out statically, one per CTA
+  if (cta >= n_first) return;
+  const int n_drawn = units - n_first;                             // units handed out through tickets
   volatile int* abort_flag = &s_abort;
 
   if (warp == kDecProducerWarp) {
@@ -271,28 +386,28 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
     tma_prefetch_desc(&map_v);
     tma_prefetch_desc(&map_k16);
     tma_prefetch_desc(&map_v16);
-    int it = 0, segc = 0;
+    int it = 0, n_unit = 0;
     bool ok = true;
-    int piece = cta;   // the CTA's own static piece first, then tickets
-    long long r_begin = pc.start(piece), r_end = pc.start(piece + 1);
-    SegDesc cur = dec_locate(s_prefix, p.batch, Hkv, r_begin, r_begin, r_end, piece);
-    // metadata of a segment, fetched one segment ahead: its length and its first two block ids
-    int cur_len = p.context_lens[cur.seq];
+    // The SM's second CTA (ids from the SM count on) counts from the short end, so that long and short units share an SM.
+    const int half = gridDim.x / 2;
+    UnitDesc cur = un.get(p, cta < half ? cta : n_first - 1 - (cta - half));
+    // the unit's first two block ids, fetched one unit ahead
     const int* cur_bt = p.block_tables + cur.seq * p.bt_row_stride;
     int cur_col0 = (cur.t0 * kTile) / p.block_size;
     int cur_blk0 = cur_bt[cur_col0];
     int cur_blk1 = cur_col0 + 1 < p.bt_cols ? cur_bt[cur_col0 + 1] : -1;
+    // Bring the first tiles into L2 while the kernel in front still runs: nothing is read, so it does not matter
+    // that that kernel may be writing this step's rows.
+    dec_prefetch_tiles(p, map_k, map_v, cur.h, cur.t0, min(cur.t1, cur.t0 + kDecStages), cur.len, cur_bt, cur_col0, cur_blk0, cur_blk1);
     asm volatile("griddepcontrol.wait;" ::: "memory");   // from here on: query rows and the cache
     while (true) {
-      cur_len = cur_len > max_len ? max_len : cur_len;
-      cur.len = cur_len;
-      const int last_col = (cur_len - 1) / p.block_size;
+      const int last_col = (cur.len - 1) / p.block_size;
       int col_now = cur_col0;
       long long blk_now = cur_blk0;
       long long blk_next = cur_col0 < last_col ? cur_blk1 : -1;
-      SegDesc nxt;
-      nxt.seq = -1;
-      int nxt_len = 0, nxt_col0 = 0, nxt_blk0 = -1, nxt_blk1 = -1;
+      UnitDesc nxt;
+      bool more = false;
+      int nxt_col0 = 0, nxt_blk0 = -1, nxt_blk1 = -1;
       const int* nxt_bt = nullptr;
       for (int t = cur.t0; t < cur.t1; ++t, ++it) {
         const int stage = it % kDecStages;
@@ -308,59 +423,32 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
         int slot0 = -kTile;  // out-of-range block id: the box lies outside the tensor and reads zeros
         if (blk_now >= 0 && blk_now < p.num_blocks)
           slot0 = static_cast<int>(blk_now * p.block_size + (tok0 - col * p.block_size));
-        unsigned char* st = stages + stage * kStageBytes;
-        const int valid = cur_len - tok0;
-        const int nslab = valid >= kTile - 15 ? 4 : (valid + 15) >> 4;
-        uint32_t tx = nslab == 4 ? kStageBytes : nslab * 4 * 2048;
+        const int nslab = dec_tile_slabs(cur.len - tok0);
         const bool first = t == cur.t0;
-        if (first) {
-          // descriptor and query rows travel with the segment's first tile
-          s_desc[segc % kSegRing] = cur;
-          tx += G * 256;
-        }
-        mbar_expect_tx(&bar_full[stage], tx);
+        // descriptor and query rows travel with the unit's first tile
+        if (first) s_desc[n_unit % kUnitRing] = cur;
+        mbar_expect_tx(&bar_full[stage], dec_tile_bytes(nslab) + (first ? G * 256 : 0));
         if (first)
-          bulk_load_1d(s_q + (segc % kSegRing) * G * 128,
+          bulk_load_1d(s_q + (n_unit % kUnitRing) * G * 128,
                        p.q + cur.seq * p.q_row_stride + static_cast<long long>(cur.h) * G * 128, G * 256, &bar_full[stage]);
-        if (nslab == 4) {
-          tma_load_3d(st, &map_k, &bar_full[stage], 0, cur.h, slot0);
-          tma_load_3d(st + kSubTileBytes, &map_k, &bar_full[stage], 64, cur.h, slot0);
-          tma_load_3d(st + 2 * kSubTileBytes, &map_v, &bar_full[stage], 0, cur.h, slot0);
-          tma_load_3d(st + 3 * kSubTileBytes, &map_v, &bar_full[stage], 64, cur.h, slot0);
-        } else {
-          // ragged last tile of the sequence: fetch only the 16-token slabs that hold tokens
-          for (int sl = 0; sl < nslab; ++sl) {
-            unsigned char* d = st + sl * 2048;
-            tma_load_3d(d, &map_k16, &bar_full[stage], 0, cur.h, slot0 + sl * 16);
-            tma_load_3d(d + kSubTileBytes, &map_k16, &bar_full[stage], 64, cur.h, slot0 + sl * 16);
-            tma_load_3d(d + 2 * kSubTileBytes, &map_v16, &bar_full[stage], 0, cur.h, slot0 + sl * 16);
-            tma_load_3d(d + 3 * kSubTileBytes, &map_v16, &bar_full[stage], 64, cur.h, slot0 + sl * 16);
-          }
-        }
+        dec_load_tile(stages + stage * kStageBytes, &bar_full[stage], &map_k, &map_v, &map_k16, &map_v16, cur.h, slot0, nslab);
         if (first) {
-          // with this segment under way, find the next one and start fetching its metadata
-          long long x = cur.seg_start + cur.t1;   // flat position after this segment's part
-          if (x >= r_end) {
-            // next piece: a ticket.  Each of the g CTAs draws until it fails, so exactly
-            // dynamic() + g tickets are drawn per launch; whoever draws the last one resets the counter.
-            int np = -1;
-            if (pc.dynamic() > 0) {
-              const unsigned int tk = atomicAdd(p.ticket, 1u);
-              if (tk == static_cast<unsigned int>(pc.dynamic() + pc.g - 1)) atomicExch(p.ticket, 0u);
-              if (tk < static_cast<unsigned int>(pc.dynamic())) np = pc.g + static_cast<int>(tk);
-            }
-            if (np >= 0) {
-              piece = np;
-              r_begin = pc.start(np);
-              r_end = pc.start(np + 1);
-              x = r_begin;
-            } else {
-              x = -1;
-            }
+          // With this unit under way, find the next one and start fetching its metadata: a ticket.  Each CTA
+          // draws until it fails, so exactly n_drawn + n_first tickets are drawn per launch (none if n_drawn is 0); whoever
+          // draws the last one resets the counter.
+          unsigned int tk = 0;
+          if (n_drawn > 0) {
+            tk = atomicAdd(p.ticket, 1u);
+            if (tk == static_cast<unsigned int>(units - 1)) atomicExch(p.ticket, 0u);
+            more = tk < static_cast<unsigned int>(n_drawn);
           }
-          if (x >= 0) {
-            nxt = dec_locate(s_prefix, p.batch, Hkv, x, r_begin, r_end, piece);
-            nxt_len = p.context_lens[nxt.seq];
+          if (!more) {
+            *const_cast<volatile int*>(&s_last) = n_unit;
+            __threadfence_block();
+          }
+          *const_cast<volatile int*>(&s_known) = n_unit + 1;     // whether anything follows this unit is settled
+          if (more) {
+            nxt = un.get(p, n_first + static_cast<int>(tk));
             nxt_bt = p.block_tables + nxt.seq * p.bt_row_stride;
             nxt_col0 = (nxt.t0 * kTile) / p.block_size;
             nxt_blk0 = nxt_bt[nxt_col0];
@@ -369,32 +457,21 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
         }
       }
       if (!ok) break;
-      ++segc;
-      if (nxt.seq < 0) break;
+      ++n_unit;
+      if (!more) break;
       cur = nxt;
-      cur_len = nxt_len;
       cur_bt = nxt_bt;
       cur_col0 = nxt_col0;
       cur_blk0 = nxt_blk0;
       cur_blk1 = nxt_blk1;
     }
-    if (ok) {
-      // end marker: a descriptor with seq = -1 on the next full-barrier, no bytes attached
-      const int stage = it % kDecStages;
-      const uint32_t ph = (it / kDecStages) & 1;
-      if (mbar_wait(&bar_empty[stage], ph ^ 1, abort_flag)) {
-        s_desc[segc % kSegRing].seq = -1;
-        mbar_arrive(&bar_full[stage]);
-      }
-    } else {
-      atomicExch(&g_status_decode, 1);
-    }
+    if (!ok) atomicExch(&g_status_decode, 1);
     return;
   }
 
   if (warp == kDecEpilogueWarp) {
     // =========================== epilogue warp ===========================
-    // Lane owns 4 of the 128 output dims.  Step 1 for every segment: combine the four consumer
+    // Lane owns 4 of the 128 output dims.  Step 1 for every unit: combine the four consumer
     // warps' states and store the row (or the partial) -- no waiting on global memory, so the
     // consumers get their hand-off buffer back at once.  The slow part of a partial (fence, arrival
     // counter, merge: several dependent trips to L2) is queued and flushed when no hand-off is
@@ -404,110 +481,22 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
       if (n_pending == 0) return;
       __threadfence();
       __syncwarp();
-      int expected = 0, old = -1;
+      bool last = false;
       if (lane < n_pending) {
-        const SegDesc& d = s_pending[lane];
-        expected = pc.of(d.seg_start + d.nt - 1) - pc.of(d.seg_start);
-        old = atomicAdd(&p.counters[d.seq * Hkv + d.h], 1);
+        const UnitDesc& d = s_pending[lane];
+        last = atomicAdd(&p.counters[d.seq * Hkv + d.h], 1) == d.parts - 1;
       }
-      const unsigned last_mask = __ballot_sync(0xffffffffu, lane < n_pending && old == expected);
+      const unsigned last_mask = __ballot_sync(0xffffffffu, last);
       if (last_mask) __threadfence();
       for (int k = 0; k < n_pending; ++k) {
         if (!((last_mask >> k) & 1u)) continue;
-        // this CTA brought the last partial of (sequence, head) k: merge them all
-        const SegDesc d = s_pending[k];
-        const int i_first = pc.of(d.seg_start);
-        const int n = pc.of(d.seg_start + d.nt - 1) - i_first + 1;
-        if (n <= 4) {
-          // The common case (a few partials): all loads of a query head are issued before the first is used,
-          // one trip to L2 per head instead of two.
-          int sl[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int i = i_first + (u < n ? u : 0);
-            sl[u] = i * 2 + (d.seg_start <= pc.start(i) ? 0 : 1);
-          }
+        // this CTA brought the last partial of pair k: merge them all
+        const UnitDesc d = s_pending[k];
 #pragma unroll 1
-          for (int gq = 0; gq < G; ++gq) {
-            float4 v[4];
-            float2 ml[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              if (u < n) {
-                v[u] = __ldcg(reinterpret_cast<const float4*>(p.ws_o + (static_cast<long long>(sl[u]) * G + gq) * 128 + lane * 4));
-                ml[u] = __ldcg(reinterpret_cast<const float2*>(p.ws_ml + (sl[u] * G + gq) * 2));
-              }
-            }
-            float M = -INFINITY;
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-              if (u < n) M = fmaxf(M, ml[u].x);
-            float L = 0.f;
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              if (u < n) {
-                const float wu = fast_exp2(ml[u].x - M);
-                L += ml[u].y * wu;
-                acc.x += v[u].x * wu; acc.y += v[u].y * wu; acc.z += v[u].z * wu; acc.w += v[u].w * wu;
-              }
-            }
-            const float inv = 1.f / L;
-            uint2 o2;
-            o2.x = pack_bf16(acc.x * inv, acc.y * inv);
-            o2.y = pack_bf16(acc.z * inv, acc.w * inv);
-            *reinterpret_cast<uint2*>(p.out + (static_cast<long long>(d.seq) * p.H + d.h * G + gq) * 128 + lane * 4) = o2;
-          }
-        } else {
-          for (int gq = 0; gq < G; ++gq) {
-            float M = -INFINITY, L = 0.f;
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int base = 0; base < n; base += 32) {
-              const int cnt = n - base < 32 ? n - base : 32;
-              // lane j looks after partial base + j: its slot, its (max, sum)
-              int sl = 0;
-              float mj = -INFINITY, lj = 0.f;
-              if (lane < cnt) {
-                const int i = i_first + base + lane;
-                sl = i * 2 + (d.seg_start <= pc.start(i) ? 0 : 1);
-                const float2 v = __ldcg(reinterpret_cast<const float2*>(p.ws_ml + (sl * G + gq) * 2));
-                mj = v.x;
-                lj = v.y;
-              }
-              float Mr = mj;
-  #pragma unroll
-              for (int off = 16; off > 0; off >>= 1) Mr = fmaxf(Mr, __shfl_xor_sync(0xffffffffu, Mr, off));
-              const float Mn = fmaxf(M, Mr);
-              const float rescale = fast_exp2(M - Mn);
-              const float wj = fast_exp2(mj - Mn);
-              float Lr = lj * wj;
-  #pragma unroll
-              for (int off = 16; off > 0; off >>= 1) Lr += __shfl_xor_sync(0xffffffffu, Lr, off);
-              L = L * rescale + Lr;
-              acc.x *= rescale; acc.y *= rescale; acc.z *= rescale; acc.w *= rescale;
-              M = Mn;
-              // every lane accumulates its 4 dims over the partials, 8 independent loads at a time
-              for (int u0 = 0; u0 < cnt; u0 += 8) {
-                float4 v[8];
-  #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                  const int slu = __shfl_sync(0xffffffffu, sl, (u0 + u) & 31);
-                  if (u0 + u < cnt)
-                    v[u] = __ldcg(reinterpret_cast<const float4*>(p.ws_o + (static_cast<long long>(slu) * G + gq) * 128 + lane * 4));
-                }
-  #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                  const float wu = __shfl_sync(0xffffffffu, wj, (u0 + u) & 31);
-                  if (u0 + u < cnt) { acc.x += v[u].x * wu; acc.y += v[u].y * wu; acc.z += v[u].z * wu; acc.w += v[u].w * wu; }
-                }
-              }
-            }
-            const float inv = 1.f / L;
-            uint2 o2;
-            o2.x = pack_bf16(acc.x * inv, acc.y * inv);
-            o2.y = pack_bf16(acc.z * inv, acc.w * inv);
-            *reinterpret_cast<uint2*>(p.out + (static_cast<long long>(d.seq) * p.H + d.h * G + gq) * 128 + lane * 4) = o2;
-          }
+        for (int gq = 0; gq < G; ++gq) {
+          DecPart r = dec_nothing();
+          dec_merge_partials(p, d.part0, d.parts, -1, gq, lane, r);
+          dec_store_row(p.out + (static_cast<long long>(d.seq) * p.H + d.h * G + gq) * 128, r, lane);
         }
         if (lane == 0) p.counters[d.seq * Hkv + d.h] = 0;
       }
@@ -519,46 +508,63 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
     for (int n = 0;;) {
       const int e = n % p.n_merge;
       const uint32_t ph = (n / p.n_merge) & 1;
-      const bool ready = !finished && !flush_now && mbar_try_wait(&bar_merge_full[e], ph);
+      bool is_last = __shfl_sync(0xffffffffu, *const_cast<volatile int*>(&s_last), 0) == n;
+      const bool ready = __all_sync(0xffffffffu, !finished && !flush_now && !is_last && mbar_try_wait(&bar_merge_full[e], ph));
       flush_now = false;
       if (!ready) {
         flush();                                     // nothing to combine right now: do the slow part
         if (finished) break;
-        if (!mbar_wait(&bar_merge_full[e], ph, abort_flag)) break;
+        if (!is_last && !mbar_wait(&bar_merge_full[e], ph, abort_flag)) break;
       }
-      const SegDesc d = s_merge_desc[e];
-      if (d.seq < 0) { finished = true; continue; }
+      // (settled by now: the consumers hand a unit over only when it is known what follows it)
+      is_last = is_last || __shfl_sync(0xffffffffu, *const_cast<volatile int*>(&s_last), 0) == n;
+      if (is_last) {
+        const UnitDesc d = s_desc[n % kUnitRing];
+        // The CTA's last unit: nothing is left to hide the trips to L2 behind, so all warps finish it together.
+        // If it is a part and the pair's other parts have all arrived (looked up while the consumers still stream), the
+        // row is finished from this CTA's own state and their partials, without a partial of its own.
+        const bool whole = d.parts == 1;
+        int* counter = &p.counters[d.seq * Hkv + d.h];
+        bool arrived = whole, handed = false;
+        const long long c0 = clock64();
+        for (int look = 0; !arrived && !handed; ++look) {
+          if ((look & 31) == 0) arrived = ld_acquire_gpu(counter) == d.parts - 1;
+          handed = mbar_test_wait(&bar_merge_full[e], ph);
+          if (*abort_flag || clock64() - c0 > kSpinLimitCycles) break;
+        }
+        arrived = __shfl_sync(0xffffffffu, arrived, 0);
+        if (lane == 0) {
+          s_decision = whole ? 0 : arrived ? 1 : 2;
+          mbar_arrive(&bar_decide);
+          if (arrived && !whole) *counter = 0;
+        }
+        if (!arrived) {
+          if (!mbar_wait(&bar_part, 0, abort_flag)) break;
+          if (lane == 0) {
+            __threadfence();
+            const bool merge = atomicAdd(counter, 1) == d.parts - 1;
+            if (merge) { __threadfence(); *counter = 0; }
+            s_merge_all = merge;
+            mbar_arrive(&bar_final);
+          }
+        }
+        finished = true;
+        continue;
+      }
+      const UnitDesc d = s_merge_desc[e];
       const float* mo = merge_o + e * kDecConsumerWarps * G * 128;
       const float* ml = merge_ml + e * kDecConsumerWarps * G * 2;
-      const bool full = d.t0 == 0 && d.t1 == d.nt;
       for (int gq = 0; gq < G; ++gq) {
-        float M = -INFINITY;
-#pragma unroll
-        for (int w = 0; w < kDecConsumerWarps; ++w) M = fmaxf(M, ml[(w * G + gq) * 2]);
-        float L = 0.f;
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int w = 0; w < kDecConsumerWarps; ++w) {
-          const float wgt = fast_exp2(ml[(w * G + gq) * 2] - M);
-          L += ml[(w * G + gq) * 2 + 1] * wgt;
-          const float4 v = *reinterpret_cast<const float4*>(mo + (w * G + gq) * 128 + lane * 4);
-          acc.x += v.x * wgt; acc.y += v.y * wgt; acc.z += v.z * wgt; acc.w += v.w * wgt;
-        }
-        if (full) {
-          const float inv = 1.f / L;
-          uint2 o2;
-          o2.x = pack_bf16(acc.x * inv, acc.y * inv);
-          o2.y = pack_bf16(acc.z * inv, acc.w * inv);
-          *reinterpret_cast<uint2*>(p.out + (static_cast<long long>(d.seq) * p.H + d.h * G + gq) * 128 + lane * 4) = o2;
-        } else {
-          *reinterpret_cast<float4*>(p.ws_o + (static_cast<long long>(d.slot) * G + gq) * 128 + lane * 4) = acc;
-          if (lane == 0) *reinterpret_cast<float2*>(p.ws_ml + (d.slot * G + gq) * 2) = make_float2(M, L);
-        }
+        const DecPart r = dec_combine_warps(mo, ml, G, gq, lane);
+        if (d.parts == 1)
+          dec_store_row(p.out + (static_cast<long long>(d.seq) * p.H + d.h * G + gq) * 128, r, lane);
+        else
+          dec_store_partial(p, d.slot, gq, lane, r);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar_merge_empty[e]);   // the consumers may refill the hand-off buffer
       ++n;
-      if (!full) {
+      if (d.parts > 1) {
         if (lane == 0) s_pending[n_pending] = d;
         __syncwarp();
         if (++n_pending == kDecPending) flush_now = true;   // a full queue is flushed at the top of the loop
@@ -568,173 +574,81 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
   }
 
   // ============================= consumer warps =============================
-  const int row = lane >> 2;        // A/C fragment row (query head within the kv group)
-  const int quad = lane & 3;
-  const bool row0_ok = row < G, row1_ok = row + 8 < G;
-  int it = 0, segc = 0;
+  int it = 0;
   bool ok = true;
-  while (ok) {
-    // ---- a new segment: its descriptor and query rows arrive with its first tile ----
-    {
-      const int stage = it % kDecStages;
-      const uint32_t ph = (it / kDecStages) & 1;
-      if (!mbar_wait(&bar_full[stage], ph, abort_flag)) { ok = false; break; }
-    }
-    const SegDesc d = s_desc[segc % kSegRing];
-    if (d.seq < 0) break;
+  for (int n_unit = 0; ok; ++n_unit) {
+    // ---- a new unit: its descriptor and query rows arrive with its first tile ----
+    if (!mbar_wait(&bar_full[it % kDecStages], (it / kDecStages) & 1, abort_flag)) { ok = false; break; }
+    const UnitDesc d = s_desc[n_unit % kUnitRing];
     uint32_t qa[8][4];   // query fragments: rows = the G heads sharing the kv head
-    {
-      const uint32_t* q0 = reinterpret_cast<const uint32_t*>(s_q + (segc % kSegRing) * G * 128 + row * 128);
-      const uint32_t* q1 = q0 + 8 * 64;
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        qa[ks][0] = row0_ok ? q0[ks * 8 + quad] : 0u;
-        qa[ks][1] = row1_ok ? q1[ks * 8 + quad] : 0u;
-        qa[ks][2] = row0_ok ? q0[ks * 8 + 4 + quad] : 0u;
-        qa[ks][3] = row1_ok ? q1[ks * 8 + 4 + quad] : 0u;
-      }
-    }
-    float o[16][4];
-#pragma unroll
-    for (int n = 0; n < 16; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
-    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
-
+    dec_query_fragments(s_q + (n_unit % kUnitRing) * G * 128, G, lane, qa);
+    DecAcc acc;
+    acc.reset();
     for (int t = d.t0; t < d.t1; ++t, ++it) {
       const int stage = it % kDecStages;
       const uint32_t ph = (it / kDecStages) & 1;
       if (t != d.t0 && !mbar_wait(&bar_full[stage], ph, abort_flag)) { ok = false; break; }
       const int valid = d.len - (t * kTile + warp * 16);  // valid tokens in this warp's 16-token slab
-      if (valid > 0) {
-        const uint32_t st = smem_u32(stages + stage * kStageBytes);
-        const uint32_t k_base = st, v_base = st + 2 * kSubTileBytes;
-        if (valid < 16) {
-          // rows past the sequence end hold whatever the cache block holds: zero the V rows so
-          // that 0 * garbage cannot produce NaN (K garbage is masked by select below)
-          unsigned char* vb = stages + stage * kStageBytes + 2 * kSubTileBytes;
-          for (int e = lane; e < 16 * 16; e += 32) {
-            const int r = warp * 16 + (e >> 4), c = e & 15;
-            if ((e >> 4) >= valid)
-              *reinterpret_cast<uint4*>(vb + (c >> 3) * kSubTileBytes + r * 128 + (((c & 7) ^ (r & 7)) << 4)) =
-                  make_uint4(0, 0, 0, 0);
-          }
-          fence_proxy_async_smem();
-          __syncwarp();
-        }
-        // ---- S = Q K^T (16 x 16 tokens) ----
-        float s[2][4];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
-        {
-          const int tok = warp * 16 + ((lane >> 4) << 3) + (lane & 7);
-          const int dsel = ((lane >> 3) & 1) << 3;
-#pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            uint32_t b0, b1, b2, b3;
-            ldmatrix_x4(k_base + tile_offset(tok, ks * 16 + dsel, kTile), b0, b1, b2, b3);
-            mma_bf16_16816(s[0], qa[ks], b0, b1);
-            mma_bf16_16816(s[1], qa[ks], b2, b3);
-          }
-        }
-        // ---- online softmax (log2 domain) ----
-        float mx0 = -INFINITY, mx1 = -INFINITY;
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const bool in = (j * 8 + quad * 2 + e) < valid;
-            s[j][e] = in ? s[j][e] * p.scale_log2 : -INFINITY;
-            s[j][2 + e] = in ? s[j][2 + e] * p.scale_log2 : -INFINITY;
-            mx0 = fmaxf(mx0, s[j][e]);
-            mx1 = fmaxf(mx1, s[j][2 + e]);
-          }
-        }
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1));
-        mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1));
-        mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-        const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);
-        const float a0 = fast_exp2(m0 - mn0), a1 = fast_exp2(m1 - mn1);
-        m0 = mn0; m1 = mn1;
-        float ps0 = 0.f, ps1 = 0.f;
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            s[j][e] = fast_exp2(s[j][e] - mn0);
-            s[j][2 + e] = fast_exp2(s[j][2 + e] - mn1);
-            ps0 += s[j][e];
-            ps1 += s[j][2 + e];
-          }
-        }
-        l0 = l0 * a0 + ps0;
-        l1 = l1 * a1 + ps1;
-        if (a0 != 1.f || a1 != 1.f) {
-#pragma unroll
-          for (int n = 0; n < 16; ++n) { o[n][0] *= a0; o[n][1] *= a0; o[n][2] *= a1; o[n][3] *= a1; }
-        }
-        // ---- O += P V ----
-        uint32_t pa[4];
-        pa[0] = pack_bf16(s[0][0], s[0][1]);
-        pa[1] = pack_bf16(s[0][2], s[0][3]);
-        pa[2] = pack_bf16(s[1][0], s[1][1]);
-        pa[3] = pack_bf16(s[1][2], s[1][3]);
-        {
-          const int tok = warp * 16 + (((lane >> 3) & 1) << 3) + (lane & 7);
-          const int dsel = (lane >> 4) << 3;
-#pragma unroll
-          for (int n2 = 0; n2 < 8; ++n2) {
-            uint32_t b0, b1, b2, b3;
-            ldmatrix_x4_trans(v_base + tile_offset(tok, n2 * 16 + dsel, kTile), b0, b1, b2, b3);
-            mma_bf16_16816(o[2 * n2], pa, b0, b1);
-            mma_bf16_16816(o[2 * n2 + 1], pa, b2, b3);
-          }
-        }
-      }
+      if (valid > 0) dec_tile(stages + stage * kStageBytes, warp, lane, valid, p.scale_log2, qa, acc);
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar_empty[stage]);
     }
     if (!ok) break;
 
     // ---- hand the warp's running state to the epilogue warp and move on ----
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
-    l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, 1);
-    l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+    const int e = n_unit % p.n_merge;
+    const uint32_t ph = (n_unit / p.n_merge) & 1;
+    if (!mbar_wait(&bar_merge_empty[e], ph ^ 1, abort_flag)) { ok = false; break; }
+    dec_hand_off(acc, merge_o + (e * kDecConsumerWarps + warp) * G * 128, merge_ml + (e * kDecConsumerWarps + warp) * G * 2, G, lane);
     {
-      const int e = segc % p.n_merge;
-      const uint32_t ph = (segc / p.n_merge) & 1;
-      if (!mbar_wait(&bar_merge_empty[e], ph ^ 1, abort_flag)) { ok = false; break; }
-      float* mo = merge_o + (e * kDecConsumerWarps + warp) * G * 128;
-#pragma unroll
-      for (int n = 0; n < 16; ++n) {
-        if (row0_ok) *reinterpret_cast<float2*>(mo + row * 128 + n * 8 + quad * 2) = make_float2(o[n][0], o[n][1]);
-        if (row1_ok) *reinterpret_cast<float2*>(mo + (row + 8) * 128 + n * 8 + quad * 2) = make_float2(o[n][2], o[n][3]);
+      const long long c0 = clock64();
+      while (*const_cast<volatile int*>(&s_known) <= n_unit) {
+        if (*abort_flag || clock64() - c0 > kSpinLimitCycles) { *abort_flag = 1; ok = false; break; }
       }
-      if (quad == 0) {
-        float* ml = merge_ml + (e * kDecConsumerWarps + warp) * G * 2;
-        if (row0_ok) { ml[row * 2] = m0; ml[row * 2 + 1] = l0; }
-        if (row1_ok) { ml[(row + 8) * 2] = m1; ml[(row + 8) * 2 + 1] = l1; }
+      __threadfence_block();
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) break;
+    const bool is_last = *const_cast<volatile int*>(&s_last) == n_unit;
+    if (tid == 0) s_merge_desc[e] = d;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&bar_merge_full[e]);
+    if (is_last) {
+      // finished by all warps together: warp w takes query heads w, w + 4, ..
+      if (!mbar_wait(&bar_merge_full[e], ph, abort_flag) || !mbar_wait(&bar_decide, 0, abort_flag)) { ok = false; break; }
+      const int decision = *const_cast<volatile int*>(&s_decision);
+      const float* mo = merge_o + e * kDecConsumerWarps * G * 128;
+      const float* ml = merge_ml + e * kDecConsumerWarps * G * 2;
+      __nv_bfloat16* out_row = p.out + (static_cast<long long>(d.seq) * p.H + d.h * G) * 128;
+#pragma unroll 1
+      for (int gq = warp; gq < G; gq += kDecConsumerWarps) {
+        DecPart r = dec_combine_warps(mo, ml, G, gq, lane);
+        if (decision == 2) {
+          dec_store_partial(p, d.slot, gq, lane, r);
+        } else {
+          if (decision == 1) dec_merge_partials(p, d.part0, d.parts - 1, d.slot, gq, lane, r);
+          dec_store_row(out_row + gq * 128, r, lane);
+        }
       }
-      if (tid == 0) s_merge_desc[e] = d;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bar_merge_full[e]);
+      if (decision == 2) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar_part);
+        if (!mbar_wait(&bar_final, 0, abort_flag)) { ok = false; break; }
+        if (*const_cast<volatile int*>(&s_merge_all)) {
+          // this CTA brought the last partial
+#pragma unroll 1
+          for (int gq = warp; gq < G; gq += kDecConsumerWarps) {
+            DecPart r = dec_nothing();
+            dec_merge_partials(p, d.part0, d.parts, -1, gq, lane, r);
+            dec_store_row(out_row + gq * 128, r, lane);
+          }
+        }
+      }
+      return;
     }
-    ++segc;
   }
-  // tell the epilogue warp that nothing more will come
-  if (ok) {
-    const int e = segc % p.n_merge;
-    const uint32_t ph = (segc / p.n_merge) & 1;
-    if (mbar_wait(&bar_merge_empty[e], ph ^ 1, abort_flag)) {
-      if (tid == 0) s_merge_desc[e].seq = -1;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bar_merge_full[e]);
-    }
-  } else if (lane == 0) {
-    atomicExch(&g_status_decode, 1);
-  }
+  if (lane == 0) atomicExch(&g_status_decode, 1);
 }
-
 
 int read_status_decode() {
   int v = 0;
@@ -753,14 +667,13 @@ int reset_state_decode() {
 static int decode_merge_buffers(int G) { return G <= 2 ? 2 : 1; }
 
 static size_t decode_smem_bytes(int G) {
-  return 1024 + static_cast<size_t>(kDecStages) * kStageBytes + static_cast<size_t>(kSegRing) * G * 256 +
-         static_cast<size_t>(decode_merge_buffers(G)) * kDecConsumerWarps * G * 130 * 4 + (kDecMaxBatch + 1) * 4 + 64;
+  return static_cast<size_t>(kDecStages) * kStageBytes + static_cast<size_t>(kUnitRing) * G * 256 +
+         static_cast<size_t>(decode_merge_buffers(G)) * kDecConsumerWarps * G * 130 * 4 + kDecMaxBatch * 7;
 }
 
 static int decode_grid() { return 2 * sm_count(); }
 
-// Two partial slots per piece; at most grid static + grid big + 4 * grid small pieces.
-static long long decode_partial_slots(int grid) { return 12LL * grid; }
+static long long decode_partial_slots(int grid) { return static_cast<long long>(kPartialSlots) * grid; }
 static long long decode_partial_bytes(int grid, int G) { return decode_partial_slots(grid) * G * 130 * 4; }
 static long long decode_ws_bytes(int grid, int G) {
   return kWsStatusBytes + static_cast<long long>(kWsCounterInts) * 4 + decode_partial_bytes(grid, G);
@@ -848,10 +761,6 @@ extern "C" int b200_decode_attn(const void* q, int64_t q_row_stride, const void*
   p.num_blocks = num_blocks;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.n_merge = decode_merge_buffers(G);
-  p.dyn_factor = kDynFactor;
-  p.big_pct = kDynBigPct;
-  p.small_pct100 = kDynSmallPct100;
-  p.small_n = kDynSmallN;
   p.ticket = reinterpret_cast<unsigned int*>(ws);
   p.counters = reinterpret_cast<int*>(ws + kWsStatusBytes);
   p.ws_o = reinterpret_cast<float*>(ws + kWsStatusBytes + static_cast<long long>(kWsCounterInts) * 4);
@@ -863,17 +772,13 @@ extern "C" int b200_decode_attn(const void* q, int64_t q_row_stride, const void*
     p.out = static_cast<__nv_bfloat16*>(out) + static_cast<long long>(b0) * num_heads * 128;
     p.context_lens = context_lens + b0;
     p.block_tables = block_tables + b0 * bt_row_stride;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kDecThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = static_cast<cudaStream_t>(stream);
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t le = cudaLaunchKernelEx(&cfg, decode_attn_kernel, p, map_k, map_v, map_k16, map_v16);
+    const int ctas = decode_cluster_ctas(p.batch, num_kv_heads, G, static_cast<int>(static_cast<long long>(bt_cols) * block_size / kTile));
+    if (ctas) {
+      rc = launch_decode_cluster(p, map_k, map_v, map_k16, map_v16, ctas, static_cast<cudaStream_t>(stream));
+      if (rc) return rc;
+      continue;
+    }
+    const cudaError_t le = launch_early(decode_attn_kernel, grid, kDecThreads, smem, static_cast<cudaStream_t>(stream), p, map_k, map_v, map_k16, map_v16);
     g_launches.fetch_add(1);
     rc = check_cuda(le != cudaSuccess ? le : cudaGetLastError(), "decode_attn launch");
     if (rc) return rc;
@@ -895,7 +800,7 @@ namespace b200 {
 
 constexpr int kStaticMaxGridTimesG = 320 * 4;   // persistent CTAs x query heads per kv head the scratch has room for
 constexpr long long kStaticScratchBytes =
-    kWsStatusBytes + static_cast<long long>(kWsCounterInts) * 4 + 12LL * kStaticMaxGridTimesG * 130 * 4;
+    kWsStatusBytes + static_cast<long long>(kWsCounterInts) * 4 + static_cast<long long>(kPartialSlots) * kStaticMaxGridTimesG * 130 * 4;
 
 static __device__ __align__(256) unsigned char g_decode_static_scratch[kStaticScratchBytes];
 

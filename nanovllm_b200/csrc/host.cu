@@ -121,11 +121,12 @@ int b200_device_status(void) {
     cudaError_t e = cudaGetLastError();
     return b200::check_cuda(e == cudaSuccess ? cudaErrorUnknown : e, "device_status: cudaDeviceSynchronize");
   }
-  const int sd = b200::read_status_decode(), sm = b200::read_status_prefill_mma(), st = b200::read_status_prefill_tc2();
+  const int sd = b200::read_status_decode() | b200::read_status_decode_cluster(), sm = b200::read_status_prefill_mma(), st = b200::read_status_prefill_tc2();
   if (sd || sm || st) {
     // Report once and recover: clear the status words and the library's own launch-to-launch state, so that the
     // next call of this function speaks about later launches only and the next prefill starts from ticket 0.
     int rc = b200::reset_state_decode();
+    if (!rc) rc = b200::reset_state_decode_cluster();
     if (!rc) rc = b200::reset_state_prefill_mma();
     if (!rc) rc = b200::reset_state_prefill_tc2();
     if (rc) return rc;

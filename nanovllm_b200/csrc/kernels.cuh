@@ -42,9 +42,11 @@ int launch_prefill_tc2(PrefillParams p, const CUtensorMap& map_q, const CUtensor
 // The reset functions clear the flag and whatever launch-to-launch state of the unit an abandoned
 // launch may have left behind (the tcgen05 kernel's ticket counter).
 int read_status_decode();
+int read_status_decode_cluster();
 int read_status_prefill_mma();
 int read_status_prefill_tc2();
 int reset_state_decode();
+int reset_state_decode_cluster();
 int reset_state_prefill_mma();
 int reset_state_prefill_tc2();
 int inject_timeout_prefill_tc2();   // test hook: leaves the unit as an abandoned launch would
