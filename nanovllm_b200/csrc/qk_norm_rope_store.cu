@@ -146,7 +146,10 @@ qk_norm_rope_store_kernel(const QkNormRopeParams p) {
   const long long n_units = static_cast<long long>(p.n_tokens) * groups;
   const long long stride = static_cast<long long>(gridDim.x) * (kQkThreads / 16);
   const unsigned half_mask = 0xffffu << (threadIdx.x & 16);
+  // Launched with programmatic stream serialization (a decode kernel in front lets it start early): nothing is read
+  // or written before the wait.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   unsigned long long wq[4], wk[4];
   if (GROUP > 1) {
     qk_weight_pairs(p.q_weight, sub, wq);
@@ -242,10 +245,8 @@ extern "C" int b200_qk_norm_rope_store(const void* qkv, int64_t qkv_row_stride, 
   const long long want = (n_units + kQkThreads / 16 - 1) / (kQkThreads / 16);
   const long long cap = static_cast<long long>(sms) * (small ? 8 : 6);
   const int grid = static_cast<int>(want < cap ? want : cap);
-  if (small)
-    qk_norm_rope_store_kernel<1><<<grid, kQkThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
-  else
-    qk_norm_rope_store_kernel<kQkGroup><<<grid, kQkThreads, 0, static_cast<cudaStream_t>(stream)>>>(p);
+  const cudaError_t le = launch_early(small ? qk_norm_rope_store_kernel<1> : qk_norm_rope_store_kernel<kQkGroup>, grid, kQkThreads,
+                                      0, static_cast<cudaStream_t>(stream), p);
   g_launches.fetch_add(1);
-  return check_cuda(cudaGetLastError(), "qk_norm_rope_store launch");
+  return check_cuda(le != cudaSuccess ? le : cudaGetLastError(), "qk_norm_rope_store launch");
 }

@@ -22,6 +22,7 @@ store_kvcache_kernel(const char* __restrict__ key, const char* __restrict__ valu
   // Let a dependent launch (the decode kernel that follows in the stream) start its prologue
   // now; it still waits for this grid to finish before it reads the cache.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const long long row_bytes = static_cast<long long>(row_vecs) * 16;
   const long long step = static_cast<long long>(gridDim.x) * kStoreThreads * kStoreUnroll;
   for (long long base = static_cast<long long>(blockIdx.x) * kStoreThreads * kStoreUnroll + threadIdx.x;
@@ -82,9 +83,10 @@ extern "C" int b200_store_kvcache(const void* key, const void* value, int64_t ke
   if (sms <= 0) return set_error(kErrNoDriver, "store_kvcache: no CUDA device");
   const long long cap = static_cast<long long>(sms) * 16;
   if (blocks > cap) blocks = cap;
-  store_kvcache_kernel<<<static_cast<unsigned>(blocks), kStoreThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const char*>(key), static_cast<const char*>(value), ks, vs, static_cast<char*>(k_cache),
-      static_cast<char*>(v_cache), slot_mapping, total, row_vecs, n_slots);
+  const cudaError_t le = launch_early(store_kvcache_kernel, static_cast<unsigned>(blocks), kStoreThreads, 0, static_cast<cudaStream_t>(stream),
+                                      static_cast<const char*>(key), static_cast<const char*>(value), ks, vs,
+                                      static_cast<char*>(k_cache), static_cast<char*>(v_cache), slot_mapping, total, row_vecs,
+                                      static_cast<long long>(n_slots));
   g_launches.fetch_add(1);
-  return check_cuda(cudaGetLastError(), "store_kvcache launch");
+  return check_cuda(le != cudaSuccess ? le : cudaGetLastError(), "store_kvcache launch");
 }
