@@ -137,6 +137,18 @@ int b200_prefill_attn(const void* q, int64_t q_row_stride, const void* k, const 
                       int32_t total_q, int32_t max_seqlen_q, int32_t max_seqlen_k, void* out, int32_t num_heads,
                       int32_t num_kv_heads, int32_t head_dim, float scale, int32_t kernel_variant, void* stream);
 
+/* b200_store_kvcache(k, v, ..) and dense b200_prefill_attn(q, k, v, ..) as one call, the layer's prefill step without a
+ * cached prefix (nanovllm/layers/attention.py:59-70): token i's k and v rows also go to flat cache row slot_mapping[i]
+ * (total_k entries; -1 and slots >= n_slots are skipped).  Attention does not read the cache here, so the tcgen05 kernel
+ * does the copy on the side in the same launch; head ratios that it does not take run the two kernels one after the
+ * other. */
+int b200_store_prefill_attn(const void* q, int64_t q_row_stride, const void* k, const void* v, int64_t k_row_stride,
+                            int64_t v_row_stride, int64_t total_k, void* k_cache, void* v_cache,
+                            const int32_t* slot_mapping, int64_t n_slots, const int32_t* cu_seqlens_q,
+                            const int32_t* cu_seqlens_k, int32_t batch, int32_t total_q, int32_t max_seqlen_q,
+                            int32_t max_seqlen_k, void* out, int32_t num_heads, int32_t num_kv_heads,
+                            int32_t head_dim, float scale, void* stream);
+
 /* ---- producer side of the layer: QK-norm + rotary embedding + cache store in one launch -------------------
  * Replaces, for one decoder layer and one step, what the reference runs between its fused qkv projection
  * and its attention call (nanovllm/models/qwen3.py:75-79 and nanovllm/layers/attention.py:62-63):

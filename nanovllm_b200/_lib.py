@@ -32,6 +32,9 @@ SIGNATURES = {
                                     c_void_p, c_int64, c_int32, c_void_p, c_int64, c_int32, c_void_p, c_void_p,
                                     c_int32, c_int32, c_int32, c_int32, c_void_p, c_int32, c_int32, c_int32,
                                     c_float, c_int32, c_void_p]),
+    "b200_store_prefill_attn": (c_int32, [c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_void_p,
+                                          c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_int32, c_int32, c_int32,
+                                          c_int32, c_void_p, c_int32, c_int32, c_int32, c_float, c_void_p]),
     "b200_qk_norm_rope_store": (c_int32, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int32, c_float,
                                           c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int32, c_int32,
                                           c_int32, c_int32, c_void_p]),

@@ -28,15 +28,22 @@ struct PrefillParams {
   int n_slots;  // upper bound on query tiles: total_q / QT + batch
   int total_q, max_seqlen_q, max_seqlen_k;
   float scale_log2;
+  // cache store done on the side (tc2): the step's K and V rows to their slots; st_slots == nullptr: none
+  const char *st_k, *st_v;
+  char *st_k_cache, *st_v_cache;
+  const int* st_slots;
+  long long st_k_stride, st_v_stride, st_n_slots;   // bytes; slots of the cache
+  int st_tokens;
   int out_tma;  // tc2: the output map (boxes of 32 tile rows) is usable: 32 % G == 0
 };
 
 // mma.sync variant: K/V maps with 64-token boxes.
 int launch_prefill_mma(const PrefillParams& p, const CUtensorMap& map_k, const CUtensorMap& map_v, cudaStream_t stream);
 // tcgen05 variant, persistent with two query tiles per CTA sharing each K/V tile: Q map with a
-// {64, G, 128 / G} box, K/V maps with 128-token boxes; needs 128 % G == 0.
+// {64, G, 128 / G} box, K/V maps with 128-token boxes; needs 128 % G == 0.  map_kc / map_vc: the caches with 32-token boxes,
+// used where p.st_slots asks for the cache store.
 int launch_prefill_tc2(PrefillParams p, const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v,
-                       const CUtensorMap& map_o, cudaStream_t stream);
+                       const CUtensorMap& map_o, const CUtensorMap& map_kc, const CUtensorMap& map_vc, cudaStream_t stream);
 
 // Device-side "a bounded wait gave up" flags, one per translation unit, read by b200_device_status().
 // The reset functions clear the flag and whatever launch-to-launch state of the unit an abandoned

@@ -170,8 +170,11 @@ PyObject* do_decode(const Tensor& q, const Tensor& kc, const Tensor& vc, const T
 }
 
 // ---- prefill (nanovllm/layers/attention.py:64-70) ------------------------------------------------------------
+// `slots` given (dense K/V): k and v also go to the caches kc and vc.
 PyObject* do_prefill(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu_q, const Tensor& cu_k, int max_q,
-                     int max_k, double scale, int hkv, const Tensor* bt, int variant, Tensor* result) {
+                     int max_k, double scale, int hkv, const Tensor* bt, int variant, const Tensor* kc, const Tensor* vc,
+                     const Tensor* slots, Tensor* result) {
+  if (slots && !check_store(k, v, *kc, *vc, *slots)) return nullptr;
   if (q.dim() != 3) {
     PyErr_SetString(PyExc_ValueError, "prefill_attention: q must be (tokens, heads, head_dim)");
     return nullptr;
@@ -184,7 +187,9 @@ PyObject* do_prefill(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   REQUIRE(cu_q.scalar_type() == at::kInt && cu_k.scalar_type() == at::kInt, "cu_seqlens must be int32");
   Tensor out = empty_like_rows({tq, h, d}, q);
   const int64_t batch = cu_q.numel() - 1;
-  if (tq > 0 && batch > 0) {
+  if (slots && (tq == 0 || batch <= 0)) {
+    if (!do_store(k, v, *kc, *vc, *slots)) return nullptr;
+  } else if (tq > 0 && batch > 0) {
     const int32_t* cq = static_cast<const int32_t*>(cu_q.data_ptr());
     const int32_t* ck = static_cast<const int32_t*>(cu_k.data_ptr());
     if (bt) {
@@ -198,6 +203,15 @@ PyObject* do_prefill(const Tensor& q, const Tensor& k, const Tensor& v, const Te
     } else {
       REQUIRE(k.dim() == 3 && v.dim() == 3 && k.stride(2) == 1 && v.stride(2) == 1 && k.stride(1) == d && v.stride(1) == d,
               "key and value heads must be contiguous");
+      if (slots) {
+        const int64_t row = k.size(1) * d;
+        LAUNCH(b200_store_prefill_attn(q.data_ptr(), q.stride(0), k.data_ptr(), v.data_ptr(), k.stride(0), v.stride(0), k.size(0),
+                                       kc->data_ptr(), vc->data_ptr(), static_cast<const int32_t*>(slots->data_ptr()), kc->numel() / row,
+                                       cq, ck, static_cast<int32_t>(batch), static_cast<int32_t>(tq), max_q, max_k, out.data_ptr(),
+                                       static_cast<int32_t>(h), hkv, static_cast<int32_t>(d), static_cast<float>(scale), stream_ptr()));
+        *result = std::move(out);
+        return kFine;
+      }
       LAUNCH(b200_prefill_attn(q.data_ptr(), q.stride(0), k.data_ptr(), v.data_ptr(), k.stride(0), v.stride(0), k.size(0),
                                nullptr, nullptr, 0, 0, nullptr, 0, 0, cq, ck, static_cast<int32_t>(batch),
                                static_cast<int32_t>(tq), max_q, max_k, out.data_ptr(), static_cast<int32_t>(h), hkv,
@@ -272,7 +286,7 @@ PyObject* py_prefill_attention(PyObject*, PyObject* const* a, Py_ssize_t nargs) 
   if (a[9] != Py_None && !(bt = tensor_of(a[9], "block_tables"))) return nullptr;
   if (!as_int(a[10], &variant)) return nullptr;
   Tensor out;
-  if (!do_prefill(*t[0], *t[1], *t[2], *t[3], *t[4], max_q, max_k, scale, hkv, bt, variant, &out)) return nullptr;
+  if (!do_prefill(*t[0], *t[1], *t[2], *t[3], *t[4], max_q, max_k, scale, hkv, bt, variant, nullptr, nullptr, nullptr, &out)) return nullptr;
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
 }
@@ -307,11 +321,18 @@ PyObject* py_attention_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) 
   if (!is_prefill.o || !bt_o.o) return nullptr;
   const int prefill = PyObject_IsTrue(is_prefill.o);
   if (prefill < 0) return nullptr;
-  if (!stored && t[3]->numel() && t[4]->numel()) {
-    Ref slots_o(PyObject_GetAttr(ctx, s_slots));
-    if (!slots_o.o) return nullptr;
-    const Tensor* slots = tensor_of(slots_o.o, "slot_mapping");
-    if (!slots || !do_store(*t[1], *t[2], *t[3], *t[4], *slots)) return nullptr;
+  const bool store = !stored && t[3]->numel() && t[4]->numel();
+  Ref slots_o(store ? PyObject_GetAttr(ctx, s_slots) : nullptr);
+  const Tensor* slots = nullptr;
+  if (store) {
+    if (!slots_o.o || !(slots = tensor_of(slots_o.o, "slot_mapping"))) return nullptr;
+    // (dense prefill of bf16 with the layer's own head count stores and attends in one launch)
+    const bool together = prefill && bt_o.o == Py_None && t[1]->dim() == 3 && t[1]->size(1) == hkv && t[0]->dim() == 3 &&
+                          t[0]->size(2) == t[1]->size(2) && t[1]->scalar_type() == at::kBFloat16 && t[0]->scalar_type() == at::kBFloat16;
+    if (!together) {
+      if (!do_store(*t[1], *t[2], *t[3], *t[4], *slots)) return nullptr;
+      slots = nullptr;
+    }
   }
   Tensor out;
   if (prefill) {
@@ -324,7 +345,8 @@ PyObject* py_attention_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) 
     const Tensor* bt = nullptr;
     if (bt_o.o != Py_None && !(bt = tensor_of(bt_o.o, "block_tables"))) return nullptr;
     // prefix cache: keys and values come from the cache
-    if (!do_prefill(*t[0], bt ? *t[3] : *t[1], bt ? *t[4] : *t[2], *cu_q, *cu_k, max_q, max_k, scale, hkv, bt, 0, &out))
+    if (!do_prefill(*t[0], bt ? *t[3] : *t[1], bt ? *t[4] : *t[2], *cu_q, *cu_k, max_q, max_k, scale, hkv, bt, 0, t[3], t[4], slots,
+                    &out))
       return nullptr;
   } else {
     Ref lens_o(PyObject_GetAttr(ctx, s_lens));

@@ -1,16 +1,24 @@
-// C-ABI entry point of prefill attention: argument checks, tensor maps, kernel selection.
+// C-ABI entry points of prefill attention: argument checks, tensor maps, kernel selection.
 #include "../../include/b200_attn.h"
 #include "kernels.cuh"
 
-extern "C" int b200_prefill_attn(const void* q, int64_t q_row_stride, const void* k, const void* v,
+namespace b200 {
+
+struct StoreArgs {
+  const int* slots;
+  void *k_cache, *v_cache;
+  long long n_slots;
+};
+
+// `store` != nullptr (dense K/V only): k and v also go to the cache rows store->slots names.
+static int prefill(const void* q, int64_t q_row_stride, const void* k, const void* v,
                                  int64_t k_row_stride, int64_t v_row_stride, int64_t total_k, const void* k_cache,
                                  const void* v_cache, int64_t num_blocks, int32_t block_size,
                                  const int32_t* block_tables, int64_t bt_row_stride, int32_t bt_cols,
                                  const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, int32_t batch,
                                  int32_t total_q, int32_t max_seqlen_q, int32_t max_seqlen_k, void* out,
                                  int32_t num_heads, int32_t num_kv_heads, int32_t head_dim, float scale,
-                                 int32_t kernel_variant, void* stream) {
-  using namespace b200;
+                                 int32_t kernel_variant, void* stream, const StoreArgs* store) {
   if (batch < 0 || total_q < 0) return set_error(kErrBadShape, "prefill_attn: negative batch or total_q");
   if (batch == 0 || total_q == 0) return kOk;
   if (!q || !out || !cu_seqlens_q || !cu_seqlens_k) return set_error(kErrNullPointer, "prefill_attn: null pointer argument");
@@ -88,6 +96,22 @@ extern "C" int b200_prefill_attn(const void* q, int64_t q_row_stride, const void
   p.max_seqlen_q = max_seqlen_q;
   p.max_seqlen_k = max_seqlen_k;
   p.out_tma = 0;
+  p.st_slots = nullptr;
+  if (store && !use_tc) {
+    rc = b200_store_kvcache(k, v, k_row_stride, v_row_stride, store->k_cache, store->v_cache, store->slots,
+                            static_cast<int32_t>(total_k), num_kv_heads * 128, 2, store->n_slots, stream);
+    if (rc) return rc;
+  } else if (store) {
+    p.st_k = static_cast<const char*>(k);
+    p.st_v = static_cast<const char*>(v);
+    p.st_k_cache = static_cast<char*>(store->k_cache);
+    p.st_v_cache = static_cast<char*>(store->v_cache);
+    p.st_slots = store->slots;
+    p.st_k_stride = k_row_stride * 2;
+    p.st_v_stride = v_row_stride * 2;
+    p.st_n_slots = store->n_slots;
+    p.st_tokens = static_cast<int>(total_k);
+  }
   if (use_tc) {
     CUtensorMap map_q;
     rc = make_tokens_heads_map(&map_q, q, static_cast<uint64_t>(total_q), num_heads, static_cast<uint64_t>(q_row_stride),
@@ -102,7 +126,53 @@ extern "C" int b200_prefill_attn(const void* q, int64_t q_row_stride, const void
                                         static_cast<uint32_t>(G));
       if (rc) return rc;
     }
-    return launch_prefill_tc2(p, map_q, map_k, map_v, map_o, static_cast<cudaStream_t>(stream));
+    CUtensorMap map_kc = map_k, map_vc = map_v;
+    if (p.st_slots) {
+      rc = make_tokens_heads_map(&map_kc, store->k_cache, static_cast<uint64_t>(store->n_slots), num_kv_heads,
+                                 static_cast<uint64_t>(num_kv_heads) * 128, 32);
+      if (rc) return rc;
+      rc = make_tokens_heads_map(&map_vc, store->v_cache, static_cast<uint64_t>(store->n_slots), num_kv_heads,
+                                 static_cast<uint64_t>(num_kv_heads) * 128, 32);
+      if (rc) return rc;
+    }
+    return launch_prefill_tc2(p, map_q, map_k, map_v, map_o, map_kc, map_vc, static_cast<cudaStream_t>(stream));
   }
   return launch_prefill_mma(p, map_k, map_v, static_cast<cudaStream_t>(stream));
+}
+
+}  // namespace b200
+
+extern "C" int b200_prefill_attn(const void* q, int64_t q_row_stride, const void* k, const void* v,
+                                 int64_t k_row_stride, int64_t v_row_stride, int64_t total_k, const void* k_cache,
+                                 const void* v_cache, int64_t num_blocks, int32_t block_size,
+                                 const int32_t* block_tables, int64_t bt_row_stride, int32_t bt_cols,
+                                 const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, int32_t batch,
+                                 int32_t total_q, int32_t max_seqlen_q, int32_t max_seqlen_k, void* out,
+                                 int32_t num_heads, int32_t num_kv_heads, int32_t head_dim, float scale,
+                                 int32_t kernel_variant, void* stream) {
+  return b200::prefill(q, q_row_stride, k, v, k_row_stride, v_row_stride, total_k, k_cache, v_cache, num_blocks, block_size,
+                       block_tables, bt_row_stride, bt_cols, cu_seqlens_q, cu_seqlens_k, batch, total_q, max_seqlen_q,
+                       max_seqlen_k, out, num_heads, num_kv_heads, head_dim, scale, kernel_variant, stream, nullptr);
+}
+
+extern "C" int b200_store_prefill_attn(const void* q, int64_t q_row_stride, const void* k, const void* v,
+                                       int64_t k_row_stride, int64_t v_row_stride, int64_t total_k, void* k_cache,
+                                       void* v_cache, const int32_t* slot_mapping, int64_t n_slots,
+                                       const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, int32_t batch,
+                                       int32_t total_q, int32_t max_seqlen_q, int32_t max_seqlen_k, void* out,
+                                       int32_t num_heads, int32_t num_kv_heads, int32_t head_dim, float scale,
+                                       void* stream) {
+  using namespace b200;
+  if (!k_cache || !v_cache || !slot_mapping)
+    return set_error(kErrNullPointer, "store_prefill_attn: null cache or slot_mapping");
+  if (n_slots < 0 || n_slots >= (1LL << 31)) return set_error(kErrBadShape, "store_prefill_attn: n_slots must be in [0, 2^31)");
+  if ((reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache)) & 15)
+    return set_error(kErrMisaligned, "store_prefill_attn: caches must be 16-byte aligned");
+  if (batch == 0 || total_q == 0)     // nothing to attend: the store alone
+    return b200_store_kvcache(k, v, k_row_stride, v_row_stride, k_cache, v_cache, slot_mapping, static_cast<int32_t>(total_k),
+                              num_kv_heads * head_dim, 2, n_slots, stream);
+  const StoreArgs store = {slot_mapping, k_cache, v_cache, n_slots};
+  return prefill(q, q_row_stride, k, v, k_row_stride, v_row_stride, total_k, nullptr, nullptr, 0, 0, nullptr, 0, 0, cu_seqlens_q,
+                 cu_seqlens_k, batch, total_q, max_seqlen_q, max_seqlen_k, out, num_heads, num_kv_heads, head_dim, scale, 0, stream,
+                 &store);
 }

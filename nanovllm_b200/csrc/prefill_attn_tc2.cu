@@ -19,7 +19,8 @@
 //   warps 12-15   output warpgroup: takes a finished O out of TMEM, scales it by 1 / row sum and
 //                 sends it out as bf16 through TMA stores (plain stores where a box would overhang
 //                 the sequence), so the softmax warpgroups never stop for output.
-//   (Warps 2-3 idle; setmaxnreg: warpgroup 0 -> 80, softmax -> 184, output -> 64 registers.)
+//   warps 2-3     send the step's K and V tiles on to the paged cache where the call asks for it (t2_store_tile);
+//   (setmaxnreg: warpgroup 0 -> 80, softmax -> 184, output -> 64 registers.)
 // TMEM: S_A [0,128)  S_B [128,256)  O_A [256,384)  O_B [384,512).  Every mbarrier wait is bounded.
 #include "../../include/b200_attn.h"
 #include "kernels.cuh"
@@ -144,10 +145,65 @@ __device__ __forceinline__ void t2_output_tma(const CUtensorMap* map_o, uint32_t
   }
 }
 
+// The layer's cache store (nanovllm/layers/attention.py:10-40) on the side.  Attention over dense K and V does not read
+// the cache, so the copy needs no launch of its own in front of it (193 us on 143872 tokens at 16/8 heads), and every
+// K and V tile passes through shared memory anyway: the item whose query block is the first to need a tile sends it on,
+// warp 2 the K tiles and warp 3 the V tiles, as TMA stores of 32 rows where the slots run on (they do inside a block),
+// else row by row.  Nothing is read from memory for it but the slots.
+// t2_store_slots() looks the slots up before the tile has arrived: the slot of its first row if they run on, else -1.
+__device__ __forceinline__ int t2_store_slots(const PrefillParams& p, int row0, int rows, int lane) {
+  int s[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) s[u] = u * 32 + lane < rows ? __ldg(p.st_slots + row0 + u * 32 + lane) : 0;
+  const int s0 = __shfl_sync(0xffffffffu, s[0], 0);
+  bool run = s0 >= 0 && s0 + static_cast<long long>(rows) <= p.st_n_slots;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) run = run && (u * 32 + lane >= rows || s[u] == s0 + u * 32 + lane);
+  return __all_sync(0xffffffffu, run) ? s0 : -1;
+}
+__device__ __forceinline__ void t2_store_tile(const PrefillParams& p, const CUtensorMap* map, char* cache, const unsigned char* tile,
+                                              int h, int row0, int rows, int s0, int lane) {
+  const int boxes = s0 >= 0 ? rows >> 5 : 0;
+  if (lane == 0 && boxes > 0) {
+    for (int b = 0; b < boxes; ++b) {
+      tma_store_3d(map, tile + b * 4096, 0, h, s0 + b * 32);
+      tma_store_3d(map, tile + kT2Sub + b * 4096, 64, h, s0 + b * 32);
+    }
+    tma_store_commit();
+  }
+  const long long row_bytes = static_cast<long long>(p.Hkv) * 256;
+#pragma unroll 1      // (short code: unrolled four times it costs the kernel 5 %, the hot loops fetch from the same cache)
+  for (int e = boxes * 512 + lane; e < rows * 16; e += 32) {
+    const int r = e >> 4, c = e & 15;
+    const long long slot = s0 >= 0 ? s0 + r : __ldg(p.st_slots + row0 + r);
+    if (slot < 0 || slot >= p.st_n_slots) continue;
+    *reinterpret_cast<uint4*>(cache + slot * row_bytes + h * 256 + c * 16) =
+        *reinterpret_cast<const uint4*>(tile + (c >> 3) * kT2Sub + r * 128 + (((c & 7) ^ (r & 7)) << 4));
+  }
+  __syncwarp();
+  if (lane == 0 && boxes > 0) tma_store_wait_read();
+}
+
+// Rows [row0, row1) that no query block loads (sequences without queries, rows outside cu_seqlens_k), all heads.
+__device__ __forceinline__ void t2_store_rows(const PrefillParams& p, const char* src, long long stride, char* cache, int row0,
+                                              int row1, int lane) {
+  const int vecs = p.Hkv * 16;
+  for (int r = row0; r < row1; ++r) {
+    const long long slot = __ldg(p.st_slots + r);
+    if (slot < 0 || slot >= p.st_n_slots) continue;
+    for (int v = lane; v < vecs; v += 32)
+      reinterpret_cast<uint4*>(cache)[slot * vecs + v] = __ldg(reinterpret_cast<const uint4*>(src + r * stride) + v);
+  }
+}
+
+// (kStore in the type, not in the arguments: the code of the store warps moves the hot loops of the others, worth 5 % to a
+// launch that stores nothing.)
+template <bool kStore>
 __global__ void __launch_bounds__(kT2Threads, 1)
 prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap map_q,
                         const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                        const __grid_constant__ CUtensorMap map_o) {
+                        const __grid_constant__ CUtensorMap map_o, const __grid_constant__ CUtensorMap map_kc,
+                        const __grid_constant__ CUtensorMap map_vc) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* sQ = smem;                              // [2][32 KiB]
@@ -171,7 +227,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
 
   if (tid == 0) {
     s_abort = 0;
-    for (int i = 0; i < kT2Items; ++i) { mbar_init(&bar_item_full[i], 1); mbar_init(&bar_item_empty[i], 13); }
+    for (int i = 0; i < kT2Items; ++i) { mbar_init(&bar_item_full[i], 1); mbar_init(&bar_item_empty[i], kStore ? 15 : 13); }
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bar_q_full[i], 1);
       mbar_init(&bar_q_empty[i], 1);
@@ -184,18 +240,21 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
     }
     for (int i = 0; i < kT2Ring; ++i) {
       mbar_init(&bar_k_full[i], 1);
-      mbar_init(&bar_k_empty[i], 1);
+      mbar_init(&bar_k_empty[i], kStore ? 2 : 1);
       mbar_init(&bar_v_full[i], 1);
-      mbar_init(&bar_v_empty[i], 1);
+      mbar_init(&bar_v_empty[i], kStore ? 2 : 1);
     }
     mbar_fence_init();
   }
-  if (slot_in_smem)
-    for (int i = tid; i <= p.batch; i += kT2Threads) s_slot[i] = __ldg(p.cu_q + i) / QB + i;
   if (warp == 1) {
     tc::tmem_alloc(&s_tmem_base, 512);
     tc::tmem_relinquish();
   }
+  // Launched with programmatic stream serialization: everything above overlaps the end of the kernel in front.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (slot_in_smem)
+    for (int i = tid; i <= p.batch; i += kT2Threads) s_slot[i] = __ldg(p.cu_q + i) / QB + i;
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
@@ -385,6 +444,50 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
           if (j + 1 < n) { tc::commit(&bar_k_empty[kt % kT2Ring]); ++kt; }
         }
         ++n_item;
+      }
+    }
+  } else if (kStore) {
+    // ================================ cache store ================================
+    const bool is_v = warp == 3;
+    uint64_t* const full = is_v ? bar_v_full : bar_k_full;
+    uint64_t* const empty = is_v ? bar_v_empty : bar_k_empty;     // (a tile's slot is free when this warp is through, too)
+    const unsigned char* const ring = is_v ? sV : sK;
+    const CUtensorMap* const map = is_v ? &map_vc : &map_kc;
+    char* const cache = is_v ? p.st_v_cache : p.st_k_cache;
+    int n_item = 0, kt = 0;
+    bool ok = true;
+    while (ok) {
+      const int is = n_item % kT2Items;
+      if (!mbar_wait(&bar_item_full[is], (n_item / kT2Items) & 1, abort_flag)) break;
+      const int seq = s_item[is].seq, h = s_item[is].h, tq0 = s_item[is].tq0, Lq = s_item[is].Lq, Lk = s_item[is].Lk;
+      const int k_begin = s_item[is].k_begin, n = max(s_item[is].n[0], s_item[is].n[1]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bar_item_empty[is]);
+      if (seq < 0) break;
+      ++n_item;
+      // The tiles this item stores: those whose first row lies in its query block; where queries and keys do not
+      // start together, the sequence's last item, which loads all tiles, stores them all.
+      const int j0 = Lq == Lk ? (tq0 + kT2Kv - 1) / kT2Kv : tq0 + QB >= Lq ? 0 : n;
+      const int j1 = Lq == Lk ? min(n, (tq0 + QB + kT2Kv - 1) / kT2Kv) : n;
+      for (int j = 0; j < n; ++j, ++kt) {
+        const int slot = kt % kT2Ring;
+        const bool mine = j >= j0 && j < j1;
+        const int row0 = k_begin + j * kT2Kv, rows = min(min(kT2Kv, Lk - j * kT2Kv), p.st_tokens - row0);
+        const int s0 = mine ? t2_store_slots(p, row0, rows, lane) : -1;
+        if (!mbar_wait(&full[slot], (kt / kT2Ring) & 1, abort_flag)) { ok = false; break; }
+        if (mine) t2_store_tile(p, map, cache, ring + slot * kT2Tile, h, row0, rows, s0, lane);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[slot]);
+      }
+    }
+    if (ok) {
+      const char* src = is_v ? p.st_v : p.st_k;
+      const long long stride = is_v ? p.st_v_stride : p.st_k_stride;
+      for (int i = blockIdx.x; i < p.batch; i += gridDim.x)
+        if (__ldg(p.cu_q + i) == __ldg(p.cu_q + i + 1)) t2_store_rows(p, src, stride, cache, __ldg(p.cu_k + i), __ldg(p.cu_k + i + 1), lane);
+      if (blockIdx.x == 0) {
+        t2_store_rows(p, src, stride, cache, 0, __ldg(p.cu_k), lane);
+        t2_store_rows(p, src, stride, cache, __ldg(p.cu_k + p.batch), p.st_tokens, lane);
       }
     }
   }
@@ -628,20 +731,21 @@ int inject_timeout_prefill_tc2() {
 
 // Needs whole query heads groups in a 128-row tile.  The query-block slots are laid out for 2 * QT tokens.
 int launch_prefill_tc2(PrefillParams p, const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v,
-                       const CUtensorMap& map_o, cudaStream_t stream) {
+                       const CUtensorMap& map_o, const CUtensorMap& map_kc, const CUtensorMap& map_vc, cudaStream_t stream) {
   p.n_slots = p.total_q / (2 * p.QT) + p.batch;
   const size_t smem = 1024 + static_cast<size_t>(2 + 2 * kT2Ring) * kT2Tile + 8 * 2048 +
                       (p.batch <= kT2MaxSeqSmem ? (p.batch + 1) * 4 : 4) + 64;
-  static std::atomic<size_t> configured[kMaxDevices];
-  const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(prefill_attn_tc2_kernel), smem, configured,
+  static std::atomic<size_t> configured[2][kMaxDevices];
+  auto* const kernel = p.st_slots ? prefill_attn_tc2_kernel<true> : prefill_attn_tc2_kernel<false>;
+  const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem, configured[p.st_slots != nullptr],
                                      "prefill_attn(tcgen05): cudaFuncSetAttribute");
   if (rc) return rc;
   const int grid = sm_count();
   if (grid <= 0) return set_error(kErrNoDriver, "prefill_attn: no CUDA device");
   if (static_cast<long long>(p.n_slots) * p.Hkv > 0x7fffffffLL) return set_error(kErrBadShape, "prefill_attn: too many query blocks");
-  prefill_attn_tc2_kernel<<<grid, kT2Threads, smem, stream>>>(p, map_q, map_k, map_v, map_o);
+  const cudaError_t le = launch_early(kernel, grid, kT2Threads, smem, stream, p, map_q, map_k, map_v, map_o, map_kc, map_vc);
   g_launches.fetch_add(1);
-  return check_cuda(cudaGetLastError(), "prefill_attn(tc2) launch");
+  return check_cuda(le != cudaSuccess ? le : cudaGetLastError(), "prefill_attn(tc2) launch");
 }
 
 }  // namespace b200
