@@ -125,7 +125,8 @@ int b200_decode_attn_static(const void* q, int64_t q_row_stride, const void* k_c
  * Sequences with Lq_i == 0 produce no rows.  out is (total_q, num_heads, 128) contiguous bf16.
  * max_seqlen_q / max_seqlen_k are the host-side bounds the caller already has
  * (nanovllm/utils/context.py:9-10).  kernel_variant: 0 = default (the persistent tcgen05 kernel
- * when 128 % (num_heads / num_kv_heads) == 0, else the mma.sync kernel), 1 = force the mma.sync
+ * when 128 % (num_heads / num_kv_heads) == 0 and the batch is not so short that the mma.sync kernel is through it sooner,
+ * else the mma.sync kernel), 1 = force the mma.sync
  * kernel, 2 = force the tcgen05 kernel (B200_ERR_BAD_SHAPE if it cannot take the shape).  Launches
  * of the tcgen05 kernel share one device-side ticket counter: do not overlap two of them on one
  * GPU.  The persistent kernel
@@ -139,9 +140,8 @@ int b200_prefill_attn(const void* q, int64_t q_row_stride, const void* k, const 
 
 /* b200_store_kvcache(k, v, ..) and dense b200_prefill_attn(q, k, v, ..) as one call, the layer's prefill step without a
  * cached prefix (nanovllm/layers/attention.py:59-70): token i's k and v rows also go to flat cache row slot_mapping[i]
- * (total_k entries; -1 and slots >= n_slots are skipped).  Attention does not read the cache here, so the tcgen05 kernel
- * does the copy on the side in the same launch; head ratios that it does not take run the two kernels one after the
- * other. */
+ * (total_k entries; -1 and slots >= n_slots are skipped).  Attention does not read the cache here and does
+ * not wait for it: both kernels do the copy on the side, in the same launch. */
 int b200_store_prefill_attn(const void* q, int64_t q_row_stride, const void* k, const void* v, int64_t k_row_stride,
                             int64_t v_row_stride, int64_t total_k, void* k_cache, void* v_cache,
                             const int32_t* slot_mapping, int64_t n_slots, const int32_t* cu_seqlens_q,

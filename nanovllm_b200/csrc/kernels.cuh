@@ -28,7 +28,7 @@ struct PrefillParams {
   int n_slots;  // upper bound on query tiles: total_q / QT + batch
   int total_q, max_seqlen_q, max_seqlen_k;
   float scale_log2;
-  // cache store done on the side (tc2): the step's K and V rows to their slots; st_slots == nullptr: none
+  // cache store done on the side: the step's K and V rows to their slots; st_slots == nullptr: none
   const char *st_k, *st_v;
   char *st_k_cache, *st_v_cache;
   const int* st_slots;
@@ -37,8 +37,8 @@ struct PrefillParams {
   int out_tma;  // tc2: the output map (boxes of 32 tile rows) is usable: 32 % G == 0
 };
 
-// mma.sync variant: K/V maps with 64-token boxes.
-int launch_prefill_mma(const PrefillParams& p, const CUtensorMap& map_k, const CUtensorMap& map_v, cudaStream_t stream);
+// mma.sync variant: K/V maps with 64-token boxes.  `small`: 64 rows per CTA instead of 128 (G <= 64).
+int launch_prefill_mma(PrefillParams p, const CUtensorMap& map_k, const CUtensorMap& map_v, bool small, cudaStream_t stream);
 // tcgen05 variant, persistent with two query tiles per CTA sharing each K/V tile: Q map with a
 // {64, G, 128 / G} box, K/V maps with 128-token boxes; needs 128 % G == 0.  map_kc / map_vc: the caches with 32-token boxes,
 // used where p.st_slots asks for the cache store.

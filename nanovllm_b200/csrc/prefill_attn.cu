@@ -2,7 +2,32 @@
 #include "../../include/b200_attn.h"
 #include "kernels.cuh"
 
+#include <cmath>
+
 namespace b200 {
+
+// Which kernel a batch goes to, from what the host knows of it.  A tcgen05 item is a chain of some 8 us however short the
+// prompt; the mma.sync kernel with 64-row CTAs is through a short one in 4 to 6, but pays 1.05 us per 64 keys where
+// tcgen05 pays half, and its CTAs come in waves of one per SM.  The lines below are fits, in us, to both kernels'
+// times over 29 batches of 1 .. 128 prompts of 1 .. 1000 tokens at 1 .. 8 kv heads (within 20 % of all of them; one prompt
+// of 137 tokens 12.8 -> 6.0 us, 16 of up to 100: 14.9 -> 10.9, 2 of 1000: stays at 27 instead of 43).
+struct PrefillChoice {
+  bool tc;           // tcgen05 (where it takes the head ratio)
+  bool small_ctas;   // mma.sync: 64 rows per CTA, not 128
+};
+static PrefillChoice prefill_choice(int total_q, int batch, int Hkv, int G, int max_k) {
+  PrefillChoice c = {true, false};
+  if (G > 64) return c;
+  const double sms = sm_count() > 0 ? sm_count() : 1;
+  const double tiles = (max_k + 63) / 64;                                                          // of 64 keys
+  const double small_waves = (static_cast<double>(total_q) / (64 / G) + batch) * Hkv / sms;        // CTAs per SM
+  const double tc_items = (static_cast<double>(total_q) / (256 / G) + batch) * Hkv / sms;          // items per SM
+  const double t_small = 1.5 + fmax(2 + 1.05 * tiles, small_waves * (3 + 0.6 * tiles));
+  const double t_tc = fmax(10 + 0.95 * tiles, 4 + tc_items * (5.2 + 0.5 * tiles));
+  c.tc = t_small > t_tc;
+  c.small_ctas = !c.tc || small_waves <= 2;
+  return c;
+}
 
 struct StoreArgs {
   const int* slots;
@@ -40,7 +65,8 @@ static int prefill(const void* q, int64_t q_row_stride, const void* k, const voi
   const bool tc_ok = 128 % G == 0;
   if (kernel_variant == 2 && !tc_ok)
     return set_error(kErrBadShape, "prefill_attn: the tcgen05 kernel needs 128 %% (num_heads / num_kv_heads) == 0 (got %d)", G);
-  const bool use_tc = kernel_variant == 2 || (kernel_variant == 0 && tc_ok);
+  const PrefillChoice choice = prefill_choice(total_q, batch, num_kv_heads, G, max_seqlen_k);
+  const bool use_tc = kernel_variant == 2 || (kernel_variant == 0 && tc_ok && choice.tc);
   const uint32_t kv_box = use_tc ? 128 : 64;
   CUtensorMap map_k, map_v;
   const bool paged = block_tables != nullptr;
@@ -97,11 +123,7 @@ static int prefill(const void* q, int64_t q_row_stride, const void* k, const voi
   p.max_seqlen_k = max_seqlen_k;
   p.out_tma = 0;
   p.st_slots = nullptr;
-  if (store && !use_tc) {
-    rc = b200_store_kvcache(k, v, k_row_stride, v_row_stride, store->k_cache, store->v_cache, store->slots,
-                            static_cast<int32_t>(total_k), num_kv_heads * 128, 2, store->n_slots, stream);
-    if (rc) return rc;
-  } else if (store) {
+  if (store) {
     p.st_k = static_cast<const char*>(k);
     p.st_v = static_cast<const char*>(v);
     p.st_k_cache = static_cast<char*>(store->k_cache);
@@ -137,7 +159,7 @@ static int prefill(const void* q, int64_t q_row_stride, const void* k, const voi
     }
     return launch_prefill_tc2(p, map_q, map_k, map_v, map_o, map_kc, map_vc, static_cast<cudaStream_t>(stream));
   }
-  return launch_prefill_mma(p, map_k, map_v, static_cast<cudaStream_t>(stream));
+  return launch_prefill_mma(p, map_k, map_v, choice.small_ctas, static_cast<cudaStream_t>(stream));
 }
 
 }  // namespace b200

@@ -1,12 +1,14 @@
-// Varlen causal prefill attention on warp-level mma.sync (the portable variant; the tcgen05
-// kernel in prefill_attn_tc.cu is the fast path).  Replaces flash_attn_varlen_func as called at
+// Varlen causal prefill attention on warp-level mma.sync: head ratios that the tcgen05 kernel
+// (prefill_attn_tc2.cu) does not take, and prompts too short for it.  Replaces flash_attn_varlen_func as called at
 // nanovllm/layers/attention.py:64-70, for dense K/V and for K/V read from the paged cache.
 //
-// One CTA owns `QT = 128 / G` consecutive query tokens of one sequence for one kv head: its
+// One CTA owns `QT = 16 * WARPS / G` consecutive query tokens of one sequence for one kv head: its
 // 16-row-per-warp M dimension is the (token, query-head-of-the-group) product, so each K/V tile
 // is loaded once for all G query heads that share it.  K/V arrive as 64-token TMA tiles through
-// a 4-stage mbarrier ring fed by a producer warp; 8 consumer warps run QK^T, online softmax and
-// PV in registers.
+// a 4-stage mbarrier ring fed by a producer warp; the consumer warps run QK^T, online softmax and
+// PV in registers.  A tile costs a scheduler 1.05 us per warp that it holds (the mma.sync rate), so short prompts, where
+// CTAs are few and latency is all there is, take 4 warps per CTA, one per scheduler, and large batches 8.  Two more
+// warps do the layer's cache store where the call asks for it.
 #include <atomic>
 
 #include "../../include/b200_attn.h"
@@ -19,23 +21,71 @@ constexpr int kPfTile = 64;
 constexpr int kPfSub = kPfTile * 128;
 constexpr int kPfStageBytes = 4 * kPfSub;
 constexpr int kPfStages = 4;
-constexpr int kPfConsumerWarps = 8;
-constexpr int kPfConsumers = kPfConsumerWarps * 32;
-constexpr int kPfThreads = kPfConsumers + 32;
+constexpr int kPfStoreThreads = 64;      // one warp for K, one for V
 
 static __device__ int g_status_prefill_mma = 0;
 
-__global__ void __launch_bounds__(kPfThreads, 1)
+// The layer's cache store (nanovllm/layers/attention.py:10-40) on the side: attention over dense K and V does not read the
+// cache.  A CTA sends on the rows of its own query tokens (they are keys of its last tiles) from shared memory.
+__device__ __forceinline__ void pf_store_tile(const PrefillParams& p, char* cache, const unsigned char* tile, int h, int r0,
+                                              int r1, const int (&slots)[2], int lane) {
+  const long long row_bytes = static_cast<long long>(p.Hkv) * 256;
+  for (int r2 = r0; r2 < r1; r2 += 2) {               // two rows per pass, half a warp each
+    const int r = r2 + (lane >> 4), c = lane & 15;
+    const int s_lo = __shfl_sync(0xffffffffu, slots[0], r & 31), s_hi = __shfl_sync(0xffffffffu, slots[1], r & 31);
+    const int slot = r < 32 ? s_lo : s_hi;
+    if (r < r1 && slot >= 0 && slot < p.st_n_slots)
+      *reinterpret_cast<uint4*>(cache + slot * row_bytes + h * 256 + c * 16) =
+          *reinterpret_cast<const uint4*>(tile + (c >> 3) * kPfSub + r * 128 + (((c & 7) ^ (r & 7)) << 4));
+  }
+}
+// Rows [row0, row1) from memory, kv heads [h0, h1): what no CTA has as its own query tokens.
+__device__ __forceinline__ void pf_store_rows(const PrefillParams& p, const char* src, long long stride, char* cache, int row0, int row1,
+                                              int h0, int h1, int lane) {
+  const int vecs = p.Hkv * 16;
+  for (int r = row0; r < row1; ++r) {
+    const long long slot = __ldg(p.st_slots + r);
+    if (slot < 0 || slot >= p.st_n_slots) continue;
+    for (int v = h0 * 16 + lane; v < h1 * 16; v += 32)
+      reinterpret_cast<uint4*>(cache)[slot * vecs + v] = __ldg(reinterpret_cast<const uint4*>(src + r * stride) + v);
+  }
+}
+
+template <int kPfConsumerWarps>
+__global__ void __launch_bounds__(kPfConsumerWarps * 32 + 32 + kPfStoreThreads, 1)
 prefill_attn_mma_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap map_k,
                         const __grid_constant__ CUtensorMap map_v) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* stages = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ __align__(8) uint64_t bar_full[kPfStages];
   __shared__ __align__(8) uint64_t bar_empty[kPfStages];
+  __shared__ __align__(8) uint64_t bar_last;     // the last tile's load is under way
   __shared__ int s_abort;
 
+  constexpr int kPfConsumers = kPfConsumerWarps * 32;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = p.G, QT = p.QT;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (tid == kPfConsumers) {
+    tma_prefetch_desc(&map_k);
+    tma_prefetch_desc(&map_v);
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const bool storing = warp > kPfConsumerWarps, st_v = warp == kPfConsumerWarps + 2;
+  char* const st_cache = st_v ? p.st_v_cache : p.st_k_cache;
+  const char* const st_src = st_v ? p.st_v : p.st_k;
+  const long long st_stride = st_v ? p.st_v_stride : p.st_k_stride;
+  if (storing) {
+    if (!p.st_slots) return;
+    // rows that belong to no query block: sequences without queries, rows outside cu_seqlens_k
+    for (int i = blockIdx.x; i < p.batch; i += gridDim.x)
+      if (__ldg(p.cu_q + i) == __ldg(p.cu_q + i + 1))
+        pf_store_rows(p, st_src, st_stride, st_cache, __ldg(p.cu_k + i), min(__ldg(p.cu_k + i + 1), p.st_tokens), 0, p.Hkv, lane);
+    if (blockIdx.x == 0) {
+      pf_store_rows(p, st_src, st_stride, st_cache, 0, min(__ldg(p.cu_k), p.st_tokens), 0, p.Hkv, lane);
+      pf_store_rows(p, st_src, st_stride, st_cache, __ldg(p.cu_k + p.batch), p.st_tokens, 0, p.Hkv, lane);
+    }
+  }
   const int h = blockIdx.x % p.Hkv;
   const int x = p.n_slots - 1 - static_cast<int>(blockIdx.x / p.Hkv);  // later (heavier) tiles first
 
@@ -57,9 +107,15 @@ prefill_attn_mma_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
   const int shift = Lk - Lq;                     // bottom-right causal alignment
   const int kv_end = min(Lk, shift + tq1);       // keys [0, kv_end) are visible to at least one row
   const int n_tiles = (kv_end + kPfTile - 1) / kPfTile;
+  if (storing && shift != 0) {
+    // queries and keys do not start together: the CTA of the last query block stores the sequence's rows of its head
+    if (tq1 == Lq) pf_store_rows(p, st_src, st_stride, st_cache, k_begin, min(k_begin + Lk, p.st_tokens), h, h + 1, lane);
+    return;
+  }
   if (n_tiles <= 0) {
+    if (storing) return;
     // no visible key (Lk < Lq rows): zeros, as the reference's attention library does
-    for (int e = tid; e < (tq1 - tq0) * G * 128; e += kPfThreads) {
+    for (int e = tid; e < (tq1 - tq0) * G * 128; e += kPfConsumers + 32) {
       const int r = e >> 7, d = e & 127;
       p.out[(static_cast<long long>(q_begin + tq0 + r / G) * p.H + h * G + r % G) * 128 + d] = __float2bfloat16(0.f);
     }
@@ -72,15 +128,30 @@ prefill_attn_mma_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       mbar_init(&bar_full[s], 1);
       mbar_init(&bar_empty[s], kPfConsumerWarps);
     }
+    mbar_init(&bar_last, 1);
     mbar_fence_init();
   }
-  __syncthreads();
+  // (the store warps take part only where they get this far)
+  named_bar_sync(2, kPfConsumers + 32 + (p.st_slots && shift == 0 ? kPfStoreThreads : 0));
   volatile int* abort_flag = &s_abort;
+
+  if (storing) {
+    for (int t = tq0 / kPfTile; t <= (tq1 - 1) / kPfTile; ++t) {
+      const int key0 = t * kPfTile, row0 = k_begin + key0;
+      const int r0 = max(tq0 - key0, 0), r1 = min(min(tq1 - key0, kPfTile), p.st_tokens - row0);
+      int slots[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) slots[u] = u * 32 + lane >= r0 && u * 32 + lane < r1 ? __ldg(p.st_slots + row0 + u * 32 + lane) : -1;
+      // These are among the CTA's last tiles: once the very last is under way their stages are not loaded again, and each
+      // full-barrier is in its tile's phase.
+      if (!mbar_wait(&bar_last, 0, abort_flag) || !mbar_wait(&bar_full[t % kPfStages], (t / kPfStages) & 1, abort_flag)) return;
+      pf_store_tile(p, st_cache, stages + (t % kPfStages) * kPfStageBytes + (st_v ? 2 * kPfSub : 0), h, r0, r1, slots, lane);
+    }
+    return;
+  }
 
   if (warp == kPfConsumerWarps) {
     if (lane == 0) {
-      tma_prefetch_desc(&map_k);
-      tma_prefetch_desc(&map_v);
       const int* bt_row = p.block_tables ? p.block_tables + seq * p.bt_row_stride : nullptr;
       for (int t = 0; t < n_tiles; ++t) {
         const int stage = t % kPfStages;
@@ -102,6 +173,7 @@ prefill_attn_mma_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         tma_load_3d(st + kPfSub, &map_k, &bar_full[stage], 64, h, row0);
         tma_load_3d(st + 2 * kPfSub, &map_v, &bar_full[stage], 0, h, row0);
         tma_load_3d(st + 3 * kPfSub, &map_v, &bar_full[stage], 64, h, row0);
+        if (t + 1 == n_tiles) mbar_arrive(&bar_last);
       }
     }
     return;
@@ -260,18 +332,22 @@ prefill_attn_mma_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
   }
 }
 
-int launch_prefill_mma(const PrefillParams& p, const CUtensorMap& map_k, const CUtensorMap& map_v, cudaStream_t stream) {
+int launch_prefill_mma(PrefillParams p, const CUtensorMap& map_k, const CUtensorMap& map_v, bool small, cudaStream_t stream) {
   const size_t smem = 1024 + static_cast<size_t>(kPfStages) * kPfStageBytes;
-  static std::atomic<size_t> configured[kMaxDevices];
-  const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(prefill_attn_mma_kernel), smem, configured,
+  static std::atomic<size_t> configured[2][kMaxDevices];
+  const int warps = small ? 4 : 8;
+  auto* const kernel = small ? prefill_attn_mma_kernel<4> : prefill_attn_mma_kernel<8>;
+  const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem, configured[small],
                                      "prefill_attn(mma.sync): cudaFuncSetAttribute");
   if (rc) return rc;
+  p.QT = 16 * warps / p.G;
+  p.n_slots = p.total_q / p.QT + p.batch;
   const long long blocks = static_cast<long long>(p.n_slots) * p.Hkv;
   if (blocks <= 0) return kOk;
   if (blocks > 0x7fffffffLL) return set_error(kErrBadShape, "prefill_attn: too many query tiles");
-  prefill_attn_mma_kernel<<<static_cast<unsigned>(blocks), kPfThreads, smem, stream>>>(p, map_k, map_v);
+  const cudaError_t le = launch_early(kernel, static_cast<unsigned>(blocks), warps * 32 + 32 + kPfStoreThreads, smem, stream, p, map_k, map_v);
   g_launches.fetch_add(1);
-  return check_cuda(cudaGetLastError(), "prefill_attn launch");
+  return check_cuda(le != cudaSuccess ? le : cudaGetLastError(), "prefill_attn launch");
 }
 
 int read_status_prefill_mma() {

@@ -13,11 +13,11 @@ DEV = "cuda:0"
 
 @pytest.mark.parametrize("slots", ["blocks", "scattered", "holes"])
 @pytest.mark.parametrize("h,hkv,lq,lk", [
-    (16, 8, [1, 127, 128, 129, 31, 32, 33, 700], None),
+    (16, 8, [1, 127, 128, 129, 31, 32, 33, 700, 2000], None), (16, 8, [1, 63, 64, 65, 33], None), (2, 1, [70], None),
     (2, 2, [255, 256, 257, 600], None),                      # one query head per kv head: two key tiles per query block
     (32, 8, [63, 64, 65, 500], None), (8, 1, [300, 17], None),
-    (5, 1, [100, 200], None),                                # not a tcgen05 head ratio: two launches
-    (4, 2, [100, 0, 300, 64], [150, 90, 300, 400]),
+    (5, 1, [100, 200], None), (3, 1, [2000, 7], None),       # not tcgen05 head ratios
+    (4, 2, [100, 0, 300, 64], [150, 90, 300, 400]), (8, 8, [900, 0, 1300, 64, 2000], [950, 90, 1300, 400, 2000]),
 ])
 def test_layer_prefill_with_store(slots, h, hkv, lq, lk):
     import nanovllm_b200
