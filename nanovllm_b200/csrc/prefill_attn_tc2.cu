@@ -246,15 +246,16 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
     }
     mbar_fence_init();
   }
+  // Launched with programmatic stream serialization: what is above overlaps the end of the kernel in front.  This kernel does
+  // not let its successor start early (its waiting CTAs cost a prefill step 5 %: 166 against 175 us on 16298 tokens), and
+  // TMEM is allocated behind the wait (in front of it: 2 % slower on every size, 786 against 769 us on cached prefixes).
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (slot_in_smem)
+    for (int i = tid; i <= p.batch; i += kT2Threads) s_slot[i] = __ldg(p.cu_q + i) / QB + i;
   if (warp == 1) {
     tc::tmem_alloc(&s_tmem_base, 512);
     tc::tmem_relinquish();
   }
-  // Launched with programmatic stream serialization: everything above overlaps the end of the kernel in front.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (slot_in_smem)
-    for (int i = tid; i <= p.batch; i += kT2Threads) s_slot[i] = __ldg(p.cu_q + i) / QB + i;
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
