@@ -86,6 +86,17 @@ int b200_decode_attn(const void* q, int64_t q_row_stride, const void* k_cache, c
                      int64_t workspace_bytes, int32_t batch, int32_t num_heads, int32_t num_kv_heads,
                      int32_t head_dim, float scale, void* stream);
 
+/* b200_store_kvcache(k, v, ..) of one row per sequence and b200_decode_attn as one call, the layer's decode step
+ * (nanovllm/layers/attention.py:59-74): row i of k and v goes to flat cache row slot_mapping[i] (-1 and slots outside the
+ * cache are skipped), and attention sees the cache with all of the step's rows in place.  A batch with few (sequence,
+ * kv head) pairs is one launch, any other the two kernels one after the other. */
+int b200_store_decode_attn(const void* q, int64_t q_row_stride, const void* k, const void* v, int64_t k_row_stride,
+                           int64_t v_row_stride, const int32_t* slot_mapping, void* k_cache, void* v_cache,
+                           int64_t num_blocks, int32_t block_size, const int32_t* block_tables, int64_t bt_row_stride,
+                           int32_t bt_cols, const int32_t* context_lens, void* out, void* workspace,
+                           int64_t workspace_bytes, int32_t batch, int32_t num_heads, int32_t num_kv_heads,
+                           int32_t head_dim, float scale, void* stream);
+
 /* No counterpart in the reference: decode attention for callers that cannot allocate.
  *
  * b200_decode_attn needs a caller-owned workspace.  Some callers have no way to provide one: an

@@ -694,12 +694,20 @@ extern "C" int64_t b200_decode_workspace_bytes(int32_t max_batch, int32_t num_he
   return decode_ws_bytes(grid, num_heads / num_kv_heads);
 }
 
-extern "C" int b200_decode_attn(const void* q, int64_t q_row_stride, const void* k_cache, const void* v_cache,
+namespace b200 {
+
+struct DecodeStore {
+  const int* slots;
+  const void *k, *v;
+  long long k_stride, v_stride;   // elements
+};
+
+// `store` != nullptr: row i of k and v also goes to slot store->slots[i] of the caches first.
+static int decode(const void* q, int64_t q_row_stride, const void* k_cache, const void* v_cache,
                                 int64_t num_blocks, int32_t block_size, const int32_t* block_tables,
                                 int64_t bt_row_stride, int32_t bt_cols, const int32_t* context_lens, void* out,
                                 void* workspace, int64_t workspace_bytes, int32_t batch, int32_t num_heads,
-                                int32_t num_kv_heads, int32_t head_dim, float scale, void* stream) {
-  using namespace b200;
+                                int32_t num_kv_heads, int32_t head_dim, float scale, void* stream, const DecodeStore* store) {
   if (batch < 0) return set_error(kErrBadShape, "decode_attn: negative batch");
   if (batch == 0) return kOk;
   if (!q || !k_cache || !v_cache || !block_tables || !context_lens || !out)
@@ -772,7 +780,22 @@ extern "C" int b200_decode_attn(const void* q, int64_t q_row_stride, const void*
     p.out = static_cast<__nv_bfloat16*>(out) + static_cast<long long>(b0) * num_heads * 128;
     p.context_lens = context_lens + b0;
     p.block_tables = block_tables + b0 * bt_row_stride;
+    p.st_slots = nullptr;
     const int ctas = decode_cluster_ctas(p.batch, num_kv_heads, G, static_cast<int>(static_cast<long long>(bt_cols) * block_size / kTile));
+    if (store && ctas && p.batch == batch) {
+      p.st_slots = store->slots;
+      p.st_k = static_cast<const __nv_bfloat16*>(store->k);
+      p.st_v = static_cast<const __nv_bfloat16*>(store->v);
+      p.st_k_stride = store->k_stride;
+      p.st_v_stride = store->v_stride;
+      p.st_n_slots = num_blocks * block_size;
+      p.st_k_cache = static_cast<__nv_bfloat16*>(const_cast<void*>(k_cache));
+      p.st_v_cache = static_cast<__nv_bfloat16*>(const_cast<void*>(v_cache));
+    } else if (store && b0 == 0) {
+      rc = b200_store_kvcache(store->k, store->v, store->k_stride, store->v_stride, const_cast<void*>(k_cache),
+                              const_cast<void*>(v_cache), store->slots, batch, num_kv_heads * 128, 2, num_blocks * block_size, stream);
+      if (rc) return rc;
+    }
     if (ctas) {
       rc = launch_decode_cluster(p, map_k, map_v, map_k16, map_v16, ctas, static_cast<cudaStream_t>(stream));
       if (rc) return rc;
@@ -784,6 +807,36 @@ extern "C" int b200_decode_attn(const void* q, int64_t q_row_stride, const void*
     if (rc) return rc;
   }
   return kOk;
+}
+
+}  // namespace b200
+
+extern "C" int b200_decode_attn(const void* q, int64_t q_row_stride, const void* k_cache, const void* v_cache,
+                                int64_t num_blocks, int32_t block_size, const int32_t* block_tables,
+                                int64_t bt_row_stride, int32_t bt_cols, const int32_t* context_lens, void* out,
+                                void* workspace, int64_t workspace_bytes, int32_t batch, int32_t num_heads,
+                                int32_t num_kv_heads, int32_t head_dim, float scale, void* stream) {
+  return b200::decode(q, q_row_stride, k_cache, v_cache, num_blocks, block_size, block_tables, bt_row_stride, bt_cols, context_lens, out,
+                      workspace, workspace_bytes, batch, num_heads, num_kv_heads, head_dim, scale, stream, nullptr);
+}
+
+extern "C" int b200_store_decode_attn(const void* q, int64_t q_row_stride, const void* k, const void* v, int64_t k_row_stride,
+                                      int64_t v_row_stride, const int32_t* slot_mapping, void* k_cache, void* v_cache,
+                                      int64_t num_blocks, int32_t block_size, const int32_t* block_tables,
+                                      int64_t bt_row_stride, int32_t bt_cols, const int32_t* context_lens, void* out,
+                                      void* workspace, int64_t workspace_bytes, int32_t batch, int32_t num_heads,
+                                      int32_t num_kv_heads, int32_t head_dim, float scale, void* stream) {
+  using namespace b200;
+  if (batch > 0) {
+    if (!k || !v || !slot_mapping) return set_error(kErrNullPointer, "store_decode_attn: null k, v or slot_mapping");
+    const int64_t row = static_cast<int64_t>(num_kv_heads) * head_dim;
+    if (k_row_stride < row || v_row_stride < row || k_row_stride % 8 || v_row_stride % 8 ||
+        ((reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15))
+      return set_error(kErrMisaligned, "store_decode_attn: k and v must be 16-byte aligned, their row strides >= Hkv*128 and multiples of 8 elements");
+  }
+  const DecodeStore store = {slot_mapping, k, v, k_row_stride, v_row_stride};
+  return decode(q, q_row_stride, k_cache, v_cache, num_blocks, block_size, block_tables, bt_row_stride, bt_cols, context_lens, out,
+                workspace, workspace_bytes, batch, num_heads, num_kv_heads, head_dim, scale, stream, &store);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -16,6 +16,7 @@ extern std::atomic<long long> g_launches;
 constexpr int kCluStages = 4;          // even: a stage belongs to one of the two groups of consumer warps
 constexpr int kCluWarps = 8;           // consumer warps: two groups of four that take the CTA's tiles in turn
 constexpr int kCluThreads = kCluWarps * 32 + 32;
+constexpr int kCluSlots = 5;           // slots per lane: a batch with a store has at most 32 * kCluSlots sequences
 constexpr int kCluMaxG = 8;            // query heads per kv head that the hand-off buffers have room for
 static __device__ int g_status_decode_cluster = 0;
 
@@ -56,6 +57,17 @@ __device__ __forceinline__ bool cluster_mbar_wait(uint64_t* bar, uint32_t parity
   }
 }
 
+// One 16-byte chunk per lane of head h of the step's row `tok`: lanes 0 .. 15 K, 16 .. 31 V.
+__device__ __forceinline__ uint4 step_chunk(const DecodeParams& p, int tok, int h, int lane) {
+  const __nv_bfloat16* src = lane < 16 ? p.st_k + tok * p.st_k_stride : p.st_v + tok * p.st_v_stride;
+  return __ldg(reinterpret_cast<const uint4*>(src + h * 128 + (lane & 15) * 8));
+}
+
+// kStore: the step's cache store (nanovllm/layers/attention.py:62-63) in the same launch; as one of its own it is half of what
+// an eager step of a small batch costs the host.  Nothing orders this launch's CTAs, so none of them relies on finding
+// another's row in the cache: rank 0 of (sequence i, head h) writes row i of head h to its slot, and whoever loads a tile
+// that covers ANY slot of the step puts the new row into its copy of the tile.
+template <bool kStore>
 __global__ void __launch_bounds__(kCluThreads, 1)
 decode_cluster_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map_k,
                       const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_k16,
@@ -72,7 +84,7 @@ decode_cluster_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap 
   __shared__ __align__(8) uint64_t bar_full[kCluStages];
   __shared__ __align__(8) uint64_t bar_empty[kCluStages];
   __shared__ __align__(8) uint64_t bar_q, bar_merge, bar_inbox;
-  __shared__ int s_abort;
+  __shared__ int s_abort, s_slot0[kCluStages];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int rank = static_cast<int>(cluster_rank());
@@ -102,6 +114,22 @@ decode_cluster_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap 
   __syncthreads();
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   len = len < 0 ? 0 : (len > max_len ? max_len : len);
+  int slots[kCluSlots];                    // consumer warps: the step's slots, lane l those of sequences l, l + 32, ..
+  uint4 own = make_uint4(0, 0, 0, 0);      // and this sequence's new row: lanes 0 .. 15 a K chunk each, 16 .. 31 a V chunk
+  if (kStore && warp < kCluWarps) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    own = step_chunk(p, seq, h, lane);
+#pragma unroll
+    for (int u = 0; u < kCluSlots; ++u) {
+      slots[u] = u * 32 + lane < p.batch ? p.st_slots[u * 32 + lane] : -1;
+      if (slots[u] >= p.st_n_slots) slots[u] = -1;
+    }
+    if (rank == 0 && warp == 0) {
+      const long long slot = p.st_slots[seq];
+      if (slot >= 0 && slot < p.st_n_slots)
+        *reinterpret_cast<uint4*>((lane < 16 ? p.st_k_cache : p.st_v_cache) + (slot * p.Hkv + h) * 128 + (lane & 15) * 8) = own;
+    }
+  }
   if (len == 0) {
     // no context: zeros (the whole cluster agrees, nobody waits for anybody)
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -151,6 +179,7 @@ decode_cluster_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap 
         int slot0 = -kTile;  // out-of-range block id: the box lies outside the tensor and reads zeros
         if (blk >= 0 && blk < p.num_blocks) slot0 = blk * p.block_size + (tok0 - col * p.block_size);
         const int nslab = dec_tile_slabs(len - tok0);
+        if (kStore) s_slot0[stage] = slot0;
         mbar_expect_tx(&bar_full[stage], dec_tile_bytes(nslab));
         dec_load_tile(stages + stage * kStageBytes, &bar_full[stage], &map_k, &map_v, &map_k16, &map_v16, h, slot0, nslab);
       }
@@ -174,6 +203,25 @@ decode_cluster_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap 
       dec_query_fragments(s_q, G, lane, qa);
     }
     const int valid = len - ((t0 + it) * kTile + slab * 16);
+    if (kStore && valid > 0) {
+      // rows of this slab that the step replaces
+      const int first = s_slot0[stage] + slab * 16;
+#pragma unroll
+      for (int u = 0; u < kCluSlots; ++u) {
+        const int row = slots[u] - first;
+        unsigned hits = __ballot_sync(0xffffffffu, slots[u] >= 0 && row >= 0 && row < 16 && row < valid);
+        while (hits) {
+          const int l = __ffs(hits) - 1;
+          hits &= hits - 1;
+          const int r = slab * 16 + __shfl_sync(0xffffffffu, row, l), tok = u * 32 + l, c = lane & 15;
+          const uint4 w = tok == seq ? own : step_chunk(p, tok, h, lane);
+          *reinterpret_cast<uint4*>(stages + stage * kStageBytes + (lane < 16 ? 0 : 2 * kSubTileBytes) + (c >> 3) * kSubTileBytes +
+                                    r * 128 + (((c & 7) ^ (r & 7)) << 4)) = w;
+          fence_proxy_async_smem();          // (a later load writes over it)
+        }
+      }
+      __syncwarp();
+    }
     if (valid > 0) dec_tile(stages + stage * kStageBytes, slab, lane, valid, p.scale_log2, qa, acc);
     __syncwarp();
     if (lane == 0) mbar_arrive(&bar_empty[stage]);
@@ -267,8 +315,9 @@ int decode_cluster_ctas(int batch, int Hkv, int G, int max_tiles) {
 int launch_decode_cluster(const DecodeParams& p, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_k16,
                           const CUtensorMap& map_v16, int ctas_per_pair, cudaStream_t stream) {
   const size_t smem = cluster_smem_bytes(p.G, ctas_per_pair);
-  static std::atomic<size_t> configured[kMaxDevices];
-  int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(decode_cluster_kernel), smem, configured,
+  static std::atomic<size_t> configured[2][kMaxDevices];
+  auto* const kernel = p.st_slots ? decode_cluster_kernel<true> : decode_cluster_kernel<false>;
+  int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem, configured[p.st_slots != nullptr],
                                "decode_attn(cluster): cudaFuncSetAttribute");
   if (rc) return rc;
   cudaLaunchConfig_t cfg = {};
@@ -284,7 +333,7 @@ int launch_decode_cluster(const DecodeParams& p, const CUtensorMap& map_k, const
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  const cudaError_t le = cudaLaunchKernelEx(&cfg, decode_cluster_kernel, p, map_k, map_v, map_k16, map_v16, ctas_per_pair);
+  const cudaError_t le = cudaLaunchKernelEx(&cfg, kernel, p, map_k, map_v, map_k16, map_v16, ctas_per_pair);
   g_launches.fetch_add(1);
   return check_cuda(le != cudaSuccess ? le : cudaGetLastError(), "decode_attn(cluster) launch");
 }

@@ -29,6 +29,11 @@ struct DecodeParams {
   float* ws_ml;   // [slots][G][2]   running max (log2 domain) and sum
   int* counters;  // [batch * Hkv], zero between launches
   unsigned int* ticket;  // unit scheduler, zero between launches
+  // the step's cache store in the same launch (cluster kernel): row i of st_k / st_v to slot st_slots[i]; nullptr: none
+  const int* st_slots;
+  const __nv_bfloat16 *st_k, *st_v;
+  long long st_k_stride, st_v_stride, st_n_slots;   // elements; slots of the cache
+  __nv_bfloat16 *st_k_cache, *st_v_cache;
 };
 
 // 1-D bulk copy global -> shared, completion counted on an mbarrier (addresses and size multiples of 16).

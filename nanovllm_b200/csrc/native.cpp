@@ -141,8 +141,10 @@ const Tensor* decode_workspace(const Tensor& q, int h, int hkv, int d) {
   return &it->second;
 }
 
+// `slots` given: the step's rows k and v (one per sequence) go to the caches first.
 PyObject* do_decode(const Tensor& q, const Tensor& kc, const Tensor& vc, const Tensor& lens, const Tensor& bt, double scale,
-                    int hkv, Tensor* result) {
+                    int hkv, const Tensor* k, const Tensor* v, const Tensor* slots, Tensor* result) {
+  if (slots && !check_store(*k, *v, kc, vc, *slots)) return nullptr;
   if (q.dim() != 3) {
     PyErr_SetString(PyExc_ValueError, "decode_attention: q must be (batch, heads, head_dim)");
     return nullptr;
@@ -159,6 +161,16 @@ PyObject* do_decode(const Tensor& q, const Tensor& kc, const Tensor& vc, const T
   if (b > 0) {
     const Tensor* ws = decode_workspace(q, static_cast<int>(h), hkv, static_cast<int>(d));
     if (!ws) return nullptr;
+    if (slots) {
+      LAUNCH(b200_store_decode_attn(q.data_ptr(), q.stride(0), k->data_ptr(), v->data_ptr(), k->stride(0), v->stride(0),
+                                    static_cast<const int32_t*>(slots->data_ptr()), kc.data_ptr(), vc.data_ptr(), kc.size(0),
+                                    static_cast<int32_t>(kc.size(1)), static_cast<const int32_t*>(bt.data_ptr()), bt.stride(0),
+                                    static_cast<int32_t>(bt.size(1)), static_cast<const int32_t*>(lens.data_ptr()), out.data_ptr(),
+                                    ws->data_ptr(), ws->numel(), static_cast<int32_t>(b), static_cast<int32_t>(h), hkv,
+                                    static_cast<int32_t>(d), static_cast<float>(scale), stream_ptr()));
+      *result = std::move(out);
+      return kFine;
+    }
     LAUNCH(b200_decode_attn(q.data_ptr(), q.stride(0), kc.data_ptr(), vc.data_ptr(), kc.size(0), static_cast<int32_t>(kc.size(1)),
                             static_cast<const int32_t*>(bt.data_ptr()), bt.stride(0), static_cast<int32_t>(bt.size(1)),
                             static_cast<const int32_t*>(lens.data_ptr()), out.data_ptr(), ws->data_ptr(), ws->numel(),
@@ -267,7 +279,7 @@ PyObject* py_decode_attention(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   int hkv;
   if (!as_double(a[5], &scale) || !as_int(a[6], &hkv)) return nullptr;
   Tensor out;
-  if (!do_decode(*t[0], *t[1], *t[2], *t[3], *t[4], scale, hkv, &out)) return nullptr;
+  if (!do_decode(*t[0], *t[1], *t[2], *t[3], *t[4], scale, hkv, nullptr, nullptr, nullptr, &out)) return nullptr;
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
 }
@@ -326,9 +338,10 @@ PyObject* py_attention_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) 
   const Tensor* slots = nullptr;
   if (store) {
     if (!slots_o.o || !(slots = tensor_of(slots_o.o, "slot_mapping"))) return nullptr;
-    // (dense prefill of bf16 with the layer's own head count stores and attends in one launch)
-    const bool together = prefill && bt_o.o == Py_None && t[1]->dim() == 3 && t[1]->size(1) == hkv && t[0]->dim() == 3 &&
-                          t[0]->size(2) == t[1]->size(2) && t[1]->scalar_type() == at::kBFloat16 && t[0]->scalar_type() == at::kBFloat16;
+    // (bf16 with the layer's own head count stores and attends in one call: dense prefill, and decode with a row per sequence)
+    const bool together = (prefill ? bt_o.o == Py_None : t[1]->dim() == 3 && t[0]->dim() == 3 && t[1]->size(0) == t[0]->size(0) && t[1]->size(0) > 0 && t[3]->dim() == 4 && t[3]->size(2) == hkv) &&
+                          t[1]->dim() == 3 && t[1]->size(1) == hkv && t[0]->dim() == 3 && t[0]->size(2) == t[1]->size(2) &&
+                          t[1]->scalar_type() == at::kBFloat16 && t[0]->scalar_type() == at::kBFloat16;
     if (!together) {
       if (!do_store(*t[1], *t[2], *t[3], *t[4], *slots)) return nullptr;
       slots = nullptr;
@@ -352,7 +365,7 @@ PyObject* py_attention_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) 
     Ref lens_o(PyObject_GetAttr(ctx, s_lens));
     if (!lens_o.o) return nullptr;
     const Tensor *lens = tensor_of(lens_o.o, "context_lens"), *bt = lens ? tensor_of(bt_o.o, "block_tables") : nullptr;
-    if (!bt || !do_decode(*t[0], *t[3], *t[4], *lens, *bt, scale, hkv, &out)) return nullptr;
+    if (!bt || !do_decode(*t[0], *t[3], *t[4], *lens, *bt, scale, hkv, t[1], t[2], slots, &out)) return nullptr;
   }
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS

@@ -45,3 +45,45 @@ def test_decode_shares(kind, n, h, hkv):
         out = nanovllm_b200.decode_attention(*d, default_scale(128), hkv)
         torch.testing.assert_close(out.float().cpu(), want.float(), atol=2e-2, rtol=1e-2)
     _lib.check(_lib.load().b200_device_status())
+
+
+@pytest.mark.parametrize("slots", ["own", "anywhere", "holes"])
+@pytest.mark.parametrize("n,h,hkv", [(1, 16, 8), (3, 8, 8), (9, 2, 1), (70, 4, 2), (140, 2, 1), (20, 16, 8)])
+def test_layer_decode_with_store(slots, n, h, hkv):
+    """The step's rows stored in the attention launch: at the sequences' ends, in other sequences' blocks (whoever reads such
+    a row must see the new one), skipped and outside the cache; a row without context is stored all the same."""
+    import nanovllm_b200
+    from nanovllm_b200.utils.context import reset_context, set_context
+    from oracle.attention_oracle import AttentionRef, Context
+    from workloads import decode_slots
+    g = torch.Generator().manual_seed(n * 7 + h)
+    lens = torch.randint(1, 700, (n,), generator=g).tolist()
+    bt, nb = make_block_tables(lens, 256, g)
+    if slots == "own":
+        sm = decode_slots(lens, bt, 256)
+    else:
+        sm = torch.randperm(nb * 256, generator=g)[:n].to(torch.int32)
+        if slots == "holes":
+            sm[::3] = -1
+            sm[n // 2] = nb * 256 + 7
+            lens[0] = 0
+            sm[0] = 5 if not (sm == 5).any() else sm[0]
+    kc = (torch.randn(nb, 256, hkv, 128, generator=g) * 0.5).to(torch.bfloat16)
+    vc = (torch.randn(nb, 256, hkv, 128, generator=g) * 0.5).to(torch.bfloat16)
+    q = torch.randn(n, h, 128, generator=g).to(torch.bfloat16)
+    fused = torch.randn(n, 2 * hkv * 128, generator=g).to(torch.bfloat16)
+    k, v = fused[:, :hkv * 128].reshape(n, hkv, 128).contiguous(), fused[:, hkv * 128:].view(n, hkv, 128)
+    cl = torch.tensor(lens, dtype=torch.int32)
+    att = nanovllm_b200.Attention(h, 128, default_scale(128), hkv)
+    att.k_cache, att.v_cache = kc.to(DEV), vc.to(DEV)
+    set_context(False, slot_mapping=sm.to(DEV), context_lens=cl.to(DEV), block_tables=bt.to(DEV))
+    out = att(q.to(DEV), k.to(DEV), fused.to(DEV)[:, hkv * 128:].view(n, hkv, 128))
+    torch.cuda.synchronize()
+    reset_context()
+    ref = AttentionRef(h, 128, default_scale(128), hkv)
+    ref.k_cache, ref.v_cache = kc, vc
+    inside = torch.where(sm < nb * 256, sm, torch.full_like(sm, -1))
+    want = ref.forward(q, k, v, Context(False, slot_mapping=inside, context_lens=cl, block_tables=bt.clamp_min(0)))
+    torch.testing.assert_close(out.float().cpu(), want.float(), atol=2e-2, rtol=1e-2)
+    assert torch.equal(att.k_cache.cpu().view(torch.int16), kc.view(torch.int16))
+    assert torch.equal(att.v_cache.cpu().view(torch.int16), vc.view(torch.int16))
