@@ -32,7 +32,7 @@ extern std::atomic<long long> g_launches;
 constexpr int kT2Kv = 128;
 constexpr int kT2Sub = 128 * 128;            // one 64-column sub-tile of a 128-row tile (bytes)
 constexpr int kT2Tile = 2 * kT2Sub;          // 128 rows x 128 dims bf16 = 32 KiB
-constexpr int kT2Threads = 512;   // warpgroup 0: TMA producer, MMA issuer, two idle warps; 1, 2: softmax; 3: output
+constexpr int kT2Threads = 512;   // warpgroup 0: TMA producer, MMA issuer, two store warps (idle without the store); 1, 2: softmax; 3: output
 constexpr int kT2Ring = 2;                   // K ring depth and V ring depth
 constexpr int kT2Items = 4;                  // item descriptors in flight
 constexpr int kT2MaxSeqSmem = 1024;          // sequences whose slot table fits in shared memory
@@ -209,7 +209,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
   unsigned char* sQ = smem;                              // [2][32 KiB]
   unsigned char* sK = smem + 2 * kT2Tile;                // [kT2Ring][32 KiB]
   unsigned char* sV = sK + kT2Ring * kT2Tile;            // [kT2Ring][32 KiB]
-  unsigned char* sStage = sV + kT2Ring * kT2Tile;       // [8 softmax warps][32 rows x 64 B] output staging
+  unsigned char* sStage = sV + kT2Ring * kT2Tile;       // [4 output warps][32 rows x 128 B] output staging
   int* s_slot = reinterpret_cast<int*>(sStage + 8 * 2048);       // [batch + 1] first slot of every sequence
   __shared__ __align__(8) uint64_t bar_item_full[kT2Items], bar_item_empty[kT2Items];
   __shared__ __align__(8) uint64_t bar_q_full[2], bar_q_empty[2];
