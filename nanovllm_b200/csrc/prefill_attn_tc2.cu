@@ -36,6 +36,7 @@ constexpr int kT2Threads = 512;   // warpgroup 0: TMA producer, MMA issuer, two 
 constexpr int kT2Ring = 2;                   // K ring depth and V ring depth
 constexpr int kT2Items = 4;                  // item descriptors in flight
 constexpr int kT2MaxSeqSmem = 1024;          // sequences whose slot table fits in shared memory
+constexpr int kT2MaxSort = kT2Threads / 2;   // sequences that are put in order of length
 constexpr float kT2Rescale = 8.0f;
 
 static __device__ int g_status_prefill_tc2 = 0;
@@ -196,6 +197,38 @@ __device__ __forceinline__ void t2_store_rows(const PrefillParams& p, const char
   }
 }
 
+// Order of the query blocks: s_order has the batch's sequences by ascending number of keys, s_slot the first block of each in
+// that order (and, at the end, the number of blocks).  Items are drawn from the back: longest sequence first and in it
+// the last, longest block, so that the launch ends with short items whatever order the batch came in.  Two threads per
+// sequence count what lies before it.  `scratch`: 8 bytes per sequence.
+__device__ __forceinline__ void t2_order(const PrefillParams& p, int QB, int* s_slot, unsigned short* s_order, int2* scratch) {
+  const int tid = threadIdx.x;
+  if (tid < p.batch) {
+    const int Lq = __ldg(p.cu_q + tid + 1) - __ldg(p.cu_q + tid);
+    scratch[tid] = make_int2(Lq > 0 ? __ldg(p.cu_k + tid + 1) - __ldg(p.cu_k + tid) : 0, Lq > 0 ? (Lq + QB - 1) / QB : 0);
+  }
+  __syncthreads();
+  const int i = tid >> 1;
+  int rank = 0, first = 0;
+  if (i < p.batch) {
+    const int mine = scratch[i].x;
+#pragma unroll 4
+    for (int j = tid & 1; j < p.batch; j += 2) {
+      const int2 o = scratch[j];
+      const bool before = o.x < mine || (o.x == mine && j < i);
+      rank += before;
+      first += before ? o.y : 0;
+    }
+  }
+  rank += __shfl_xor_sync(0xffffffffu, rank, 1);
+  first += __shfl_xor_sync(0xffffffffu, first, 1);
+  if (i < p.batch && !(tid & 1)) {
+    s_order[rank] = static_cast<unsigned short>(i);
+    s_slot[rank] = first;
+    if (rank == p.batch - 1) s_slot[p.batch] = min(first + scratch[i].y, p.n_slots);
+  }
+}
+
 // (kStore in the type, not in the arguments: the code of the store warps moves the hot loops of the others, worth 5 % to a
 // launch that stores nothing.)
 template <bool kStore>
@@ -210,7 +243,8 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
   unsigned char* sK = smem + 2 * kT2Tile;                // [kT2Ring][32 KiB]
   unsigned char* sV = sK + kT2Ring * kT2Tile;            // [kT2Ring][32 KiB]
   unsigned char* sStage = sV + kT2Ring * kT2Tile;       // [4 output warps][32 rows x 128 B] output staging
-  int* s_slot = reinterpret_cast<int*>(sStage + 8 * 2048);       // [batch + 1] first slot of every sequence
+  int* s_slot = reinterpret_cast<int*>(sStage + 8 * 2048);       // [batch + 1] first slot of every sequence, in the order of
+  unsigned short* s_order = reinterpret_cast<unsigned short*>(s_slot + p.batch + 1);             // [batch]
   __shared__ __align__(8) uint64_t bar_item_full[kT2Items], bar_item_empty[kT2Items];
   __shared__ __align__(8) uint64_t bar_q_full[2], bar_q_empty[2];
   __shared__ __align__(8) uint64_t bar_k_full[kT2Ring], bar_k_empty[kT2Ring], bar_v_full[kT2Ring], bar_v_empty[kT2Ring];
@@ -246,12 +280,18 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
     }
     mbar_fence_init();
   }
+  // (cu_seqlens ahead of the wait below: no kernel that lets this one start early writes them)
+  const bool sorted = p.batch <= kT2MaxSort;
+  if (sorted) t2_order(p, QB, s_slot, s_order, reinterpret_cast<int2*>(sStage));
   // Launched with programmatic stream serialization: what is above overlaps the end of the kernel in front.  This kernel does
   // not let its successor start early (its waiting CTAs cost a prefill step 5 %: 166 against 175 us on 16298 tokens), and
   // TMEM is allocated behind the wait (in front of it: 2 % slower on every size, 786 against 769 us on cached prefixes).
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (slot_in_smem)
-    for (int i = tid; i <= p.batch; i += kT2Threads) s_slot[i] = __ldg(p.cu_q + i) / QB + i;
+  if (slot_in_smem && !sorted)
+    for (int i = tid; i <= p.batch; i += kT2Threads) {
+      s_slot[i] = __ldg(p.cu_q + i) / QB + i;
+      if (i < p.batch) s_order[i] = static_cast<unsigned short>(i);
+    }
   if (warp == 1) {
     tc::tmem_alloc(&s_tmem_base, 512);
     tc::tmem_relinquish();
@@ -272,7 +312,8 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       tma_prefetch_desc(&map_q);
       tma_prefetch_desc(&map_k);
       tma_prefetch_desc(&map_v);
-      const unsigned int n_items = static_cast<unsigned int>(p.n_slots) * p.Hkv;
+      const int n_slots = sorted ? s_slot[p.batch] : p.n_slots;
+      const unsigned int n_items = static_cast<unsigned int>(n_slots) * p.Hkv;
       int n_pub = 0;            // items published
       int kt = 0, vt = 0;       // K / V tiles issued so far (ring positions)
       bool ok = true;
@@ -287,16 +328,17 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         bool b_rows = false;                                            // half B holds query rows
         if (tk < n_items) {
           h = tk % p.Hkv;
-          const int x = p.n_slots - 1 - static_cast<int>(tk / p.Hkv);   // reverse slot order: within a sequence the later, longer blocks come first
+          const int x = n_slots - 1 - static_cast<int>(tk / p.Hkv);     // reverse slot order: within a sequence the later, longer blocks come first
           int lo = 0, hi = p.batch;
           while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
             const int f = slot_in_smem ? s_slot[mid] : __ldg(p.cu_q + mid) / QB + mid;
             if (f <= x) lo = mid; else hi = mid;
           }
+          const int qb = x - (slot_in_smem ? s_slot[lo] : __ldg(p.cu_q + lo) / QB + lo);
+          if (slot_in_smem) lo = s_order[lo];
           const int q_begin = __ldg(p.cu_q + lo);
           const int Lq = __ldg(p.cu_q + lo + 1) - q_begin;
-          const int qb = x - (q_begin / QB + lo);
           if (qb < 0 || qb * QB >= Lq) continue;                        // slot owns no query block
           k_begin = __ldg(p.cu_k + lo);
           const int Lk = __ldg(p.cu_k + lo + 1) - k_begin;
@@ -735,7 +777,7 @@ int launch_prefill_tc2(PrefillParams p, const CUtensorMap& map_q, const CUtensor
                        const CUtensorMap& map_o, const CUtensorMap& map_kc, const CUtensorMap& map_vc, cudaStream_t stream) {
   p.n_slots = p.total_q / (2 * p.QT) + p.batch;
   const size_t smem = 1024 + static_cast<size_t>(2 + 2 * kT2Ring) * kT2Tile + 8 * 2048 +
-                      (p.batch <= kT2MaxSeqSmem ? (p.batch + 1) * 4 : 4) + 64;
+                      (p.batch <= kT2MaxSeqSmem ? (p.batch + 1) * 6 : 4) + 64;
   static std::atomic<size_t> configured[2][kMaxDevices];
   auto* const kernel = p.st_slots ? prefill_attn_tc2_kernel<true> : prefill_attn_tc2_kernel<false>;
   const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem, configured[p.st_slots != nullptr],
