@@ -42,7 +42,7 @@ int launch_prefill_mma(PrefillParams p, const CUtensorMap& map_k, const CUtensor
 // tcgen05 variant, persistent with two query tiles per CTA sharing each K/V tile: Q map with a
 // {64, G, 128 / G} box, K/V maps with 128-token boxes; needs 128 % G == 0.  map_kc / map_vc: the caches with 32-token boxes,
 // used where p.st_slots asks for the cache store.
-int launch_prefill_tc2(PrefillParams p, const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v,
+int launch_prefill_tc2(PrefillParams p, bool split, const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v,
                        const CUtensorMap& map_o, const CUtensorMap& map_kc, const CUtensorMap& map_vc, cudaStream_t stream);
 
 // Device-side "a bounded wait gave up" flags, one per translation unit, read by b200_device_status().

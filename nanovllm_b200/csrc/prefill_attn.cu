@@ -11,21 +11,30 @@ namespace b200 {
 // tcgen05 pays half, and its CTAs come in waves of one per SM.  The lines below are fits, in us, to both kernels'
 // times over 29 batches of 1 .. 128 prompts of 1 .. 1000 tokens at 1 .. 8 kv heads (within 20 % of all of them; one prompt
 // of 137 tokens 12.8 -> 6.0 us, 16 of up to 100: 14.9 -> 10.9, 2 of 1000: stays at 27 instead of 43).
+// Where the tcgen05 launch has few items its length is that of one item's chain, 0.9 us per 64 keys.  With the keys shared
+// between the halves (`split`) it is half of that, for twice as many items of half the rows, each with the same start and
+// end to pay: worth it up to some 1.2 whole items per SM, by the same kind of fit over 85 batches of 1 .. 64 prompts of
+// 50 .. 8192 tokens (one of 2048 at 8/4 heads 36.8 -> 24.2 us, of 8192 at 4/2 heads 124 -> 67, 4 of 200 .. 2000 at
+// 16/8 heads, 2.1 items per SM, stay at 42 instead of 44).
 struct PrefillChoice {
   bool tc;           // tcgen05 (where it takes the head ratio)
+  bool split;        // tcgen05: items of one tile of rows, the keys shared between the halves
   bool small_ctas;   // mma.sync: 64 rows per CTA, not 128
 };
 static PrefillChoice prefill_choice(int total_q, int batch, int Hkv, int G, int max_k) {
-  PrefillChoice c = {true, false};
-  if (G > 64) return c;
+  PrefillChoice c = {true, false, false};
+  if (G > 64) return c;   // (no room for a group in 64 rows)
   const double sms = sm_count() > 0 ? sm_count() : 1;
   const double tiles = (max_k + 63) / 64;                                                          // of 64 keys
   const double small_waves = (static_cast<double>(total_q) / (64 / G) + batch) * Hkv / sms;        // CTAs per SM
   const double tc_items = (static_cast<double>(total_q) / (256 / G) + batch) * Hkv / sms;          // items per SM
   const double t_small = 1.5 + fmax(2 + 1.05 * tiles, small_waves * (3 + 0.6 * tiles));
-  const double t_tc = fmax(10 + 0.95 * tiles, 4 + tc_items * (5.2 + 0.5 * tiles));
-  c.tc = t_small > t_tc;
-  c.small_ctas = !c.tc || small_waves <= 2;
+  const double split_items = (static_cast<double>(total_q) / (128 / G) + batch) * Hkv / sms;
+  const double t_full = fmax(8 + 0.9 * tiles, 4 + tc_items * (5.2 + 0.5 * tiles));
+  const double t_split = fmax(8.6 + 0.47 * tiles, 4 + split_items * (5.2 + 0.235 * tiles));
+  c.split = t_split < t_full;
+  c.tc = t_small > fmin(t_split, t_full);
+  c.small_ctas = t_small <= t_full || small_waves <= 2;   // (!c.tc, and the head ratios that tcgen05 does not take)
   return c;
 }
 
@@ -157,7 +166,7 @@ static int prefill(const void* q, int64_t q_row_stride, const void* k, const voi
                                  static_cast<uint64_t>(num_kv_heads) * 128, 32);
       if (rc) return rc;
     }
-    return launch_prefill_tc2(p, map_q, map_k, map_v, map_o, map_kc, map_vc, static_cast<cudaStream_t>(stream));
+    return launch_prefill_tc2(p, choice.split, map_q, map_k, map_v, map_o, map_kc, map_vc, static_cast<cudaStream_t>(stream));
   }
   return launch_prefill_mma(p, map_k, map_v, choice.small_ctas, static_cast<cudaStream_t>(stream));
 }

@@ -3,11 +3,11 @@
 // and for K/V read from the paged cache.
 //
 // One persistent CTA per SM.  A work item is (sequence, kv head, block of 2 * QT query tokens),
-// QT = 128 / G, handed out through an atomic ticket counter in reverse slot order (the last sequence first, and
-// within a sequence its last, longest query block first; not sorted by work across sequences).  The two
+// QT = 128 / G, handed out through an atomic ticket counter from the longest sequence down (t2_order), and
+// within a sequence from its last, longest query block.  The two
 // halves of the block ("A" = first QT tokens, "B" = next QT) are two independent 128-row tiles that
 // share every K/V tile, so K/V traffic per query row is halved and, more to the point, the tensor
-// core always has the other half's MMA to run while one half is in its softmax:
+// core always has the other half's MMA to run while one half is in its softmax (launches with few items: kSplit below):
 //   warp 0        TMA producer: draws tickets, publishes item descriptors, loads Q_A / Q_B and
 //                 feeds two-deep rings of 128-token K tiles and V tiles;
 //   warp 1        one elected thread issues tcgen05.mma:  S_X = Q_X K^T  (M128 N128 K16 x 8) and
@@ -25,6 +25,8 @@
 #include "../../include/b200_attn.h"
 #include "kernels.cuh"
 #include "tcgen05.cuh"
+
+#include <type_traits>
 
 namespace b200 {
 extern std::atomic<long long> g_launches;
@@ -53,6 +55,35 @@ struct T2Item {
   int n[2];       // K/V tiles each half needs (n[1] == 0: half B is empty)
 };
 
+// One 16-column chunk of a warp's 32 rows, scaled, to memory through the staging tile.
+__device__ __forceinline__ void t2_plain_chunk(const PrefillParams& p, const uint32_t (&ov)[16], unsigned char* stage, int lane,
+                                               int quarter, int hx, int cch, float inv, int q_row, int h, int tq0, int Lq) {
+  const int G = p.G, QT = p.QT;
+  const int srow = lane >> 1, sq = lane & 1;             // read-back role: 16 rows x 2 chunks per instruction
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    uint4 w;
+    w.x = pack_bf16(__uint_as_float(ov[8 * i]) * inv, __uint_as_float(ov[8 * i + 1]) * inv);
+    w.y = pack_bf16(__uint_as_float(ov[8 * i + 2]) * inv, __uint_as_float(ov[8 * i + 3]) * inv);
+    w.z = pack_bf16(__uint_as_float(ov[8 * i + 4]) * inv, __uint_as_float(ov[8 * i + 5]) * inv);
+    w.w = pack_bf16(__uint_as_float(ov[8 * i + 6]) * inv, __uint_as_float(ov[8 * i + 7]) * inv);
+    *reinterpret_cast<uint4*>(stage + lane * 32 + ((i ^ ((lane >> 2) & 1)) << 4)) = w;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int lr = 16 * k + srow;                         // row within the warp's 32
+    const uint4 w = *reinterpret_cast<const uint4*>(stage + lr * 32 + ((sq ^ ((lr >> 2) & 1)) << 4));
+    const int rr = quarter * 32 + lr;                     // row of the 128-row tile
+    const int tk = tq0 + hx * QT + rr / G;
+    if (rr < QT * G && tk < Lq)
+      *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(
+          p.out + (static_cast<long long>(q_row + hx * QT + rr / G) * p.H + h * G + rr % G) * 128) +
+          cch * 32 + sq * 16) = w;
+  }
+  __syncwarp();
+}
+
 // Output of one half of an item, run by the output warpgroup: read the finished O row out of TMEM
 // in 32-column chunks, scale by 1 / row sum and store bf16 rows through a per-warp staging tile so
 // that every store instruction writes 64-byte row segments (a thread owns a whole row: stored
@@ -61,8 +92,6 @@ struct T2Item {
 __device__ __forceinline__ void t2_output(const PrefillParams& p, uint32_t tmem_o_lane, uint64_t* bar_o_free,
                                           unsigned char* stage, int lane, int quarter, int hx,
                                           float inv, int q_row, int h, int tq0, int Lq) {
-  const int G = p.G, QT = p.QT;
-  const int srow = lane >> 1, sq = lane & 1;             // read-back role: 16 rows x 2 chunks per instruction
 #pragma unroll 1
   for (int cch = 0; cch < 8; ++cch) {
     uint32_t ov[16];
@@ -73,28 +102,7 @@ __device__ __forceinline__ void t2_output(const PrefillParams& p, uint32_t tmem_
       __syncwarp();
       if (lane == 0) mbar_arrive(bar_o_free);
     }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      uint4 w;
-      w.x = pack_bf16(__uint_as_float(ov[8 * i]) * inv, __uint_as_float(ov[8 * i + 1]) * inv);
-      w.y = pack_bf16(__uint_as_float(ov[8 * i + 2]) * inv, __uint_as_float(ov[8 * i + 3]) * inv);
-      w.z = pack_bf16(__uint_as_float(ov[8 * i + 4]) * inv, __uint_as_float(ov[8 * i + 5]) * inv);
-      w.w = pack_bf16(__uint_as_float(ov[8 * i + 6]) * inv, __uint_as_float(ov[8 * i + 7]) * inv);
-      *reinterpret_cast<uint4*>(stage + lane * 32 + ((i ^ ((lane >> 2) & 1)) << 4)) = w;
-    }
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int lr = 16 * k + srow;                         // row within the warp's 32
-      const uint4 w = *reinterpret_cast<const uint4*>(stage + lr * 32 + ((sq ^ ((lr >> 2) & 1)) << 4));
-      const int rr = quarter * 32 + lr;                     // row of the 128-row tile
-      const int tk = tq0 + hx * QT + rr / G;
-      if (rr < QT * G && tk < Lq)
-        *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(
-            p.out + (static_cast<long long>(q_row + hx * QT + rr / G) * p.H + h * G + rr % G) * 128) +
-            cch * 32 + sq * 16) = w;
-    }
-    __syncwarp();
+    t2_plain_chunk(p, ov, stage, lane, quarter, hx, cch, inv, q_row, h, tq0, Lq);
   }
 }
 
@@ -142,6 +150,51 @@ __device__ __forceinline__ void t2_output_tma(const CUtensorMap* map_o, uint32_t
     if (lane == 0) {
       tma_store_3d(map_o, box, bx * 32, head0, tok0);
       tma_store_commit();
+    }
+  }
+}
+
+// Output of an item whose keys the halves shared: the same rows lie in both accumulators, each relative to its own half's
+// maximum; `wa` and `wb` bring them together (has_b false: there was one tile, half B has nothing).
+__device__ __forceinline__ void t2_output_split(const PrefillParams& p, const CUtensorMap* map_o, uint32_t tmem_a, uint32_t tmem_b,
+                                                bool has_b, uint64_t* bar_o_free, unsigned char* stage, int lane, int quarter,
+                                                float wa, float wb, bool tma, int q_row, int h, int tq0, int Lq) {
+#pragma unroll 1
+  for (int cch = 0; cch < 8; ++cch) {
+    unsigned char* box = stage + ((cch >> 1) & 1) * 2048;
+    if (tma && !(cch & 1)) {
+      if (lane == 0) tma_store_wait_read_but_one();
+      __syncwarp();
+    }
+    uint32_t a[16], b[16];
+    tc::ld_32x32b_x16(tmem_a + cch * 16, a);
+    if (has_b) tc::ld_32x32b_x16(tmem_b + cch * 16, b);
+    tc::wait_ld();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float o = __uint_as_float(a[i]) * wa;
+      a[i] = __float_as_uint(has_b ? fmaf(__uint_as_float(b[i]), wb, o) : o);
+    }
+    if (cch == 7) {
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) {
+        mbar_arrive(&bar_o_free[0]);
+        if (has_b) mbar_arrive(&bar_o_free[1]);
+      }
+    }
+    if (tma) {
+      t2_stage_chunk(a, box, lane, cch & 1, 1.f);
+      if (cch & 1) {
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_3d(map_o, box, (cch >> 1) * 32, h * p.G, q_row + quarter * 32 / p.G);
+          tma_store_commit();
+        }
+      }
+    } else {
+      t2_plain_chunk(p, a, stage, lane, quarter, 0, cch, 1.f, q_row, h, tq0, Lq);
     }
   }
 }
@@ -231,32 +284,36 @@ __device__ __forceinline__ void t2_order(const PrefillParams& p, int QB, int* s_
 
 // (kStore in the type, not in the arguments: the code of the store warps moves the hot loops of the others, worth 5 % to a
 // launch that stores nothing.)
-template <bool kStore>
+// kSplit: for launches with few items.  An item is one 128-row tile of queries, and its halves take the key tiles in turn
+// (A the even, B the odd ones): the two chains S -> softmax -> PV that a CTA can keep going then work on the same rows, so
+// a lone long item takes half as long.  The output warpgroup joins them.  The room of the second Q tile is a third K slot.
+template <bool kStore, bool kSplit>
 __global__ void __launch_bounds__(kT2Threads, 1)
 prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap map_q,
                         const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                         const __grid_constant__ CUtensorMap map_o, const __grid_constant__ CUtensorMap map_kc,
                         const __grid_constant__ CUtensorMap map_vc) {
-  extern __shared__ unsigned char smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char* sQ = smem;                              // [2][32 KiB]
-  unsigned char* sK = smem + 2 * kT2Tile;                // [kT2Ring][32 KiB]
-  unsigned char* sV = sK + kT2Ring * kT2Tile;            // [kT2Ring][32 KiB]
+  extern __shared__ __align__(1024) unsigned char smem[];
+  constexpr int kRingK = kSplit ? kT2Ring + 1 : kT2Ring;
+  unsigned char* sQ = smem;                              // [2 (kSplit: 1)][32 KiB]
+  unsigned char* sK = smem + (kSplit ? 1 : 2) * kT2Tile; // [kRingK][32 KiB]
+  unsigned char* sV = sK + kRingK * kT2Tile;             // [kT2Ring][32 KiB]
   unsigned char* sStage = sV + kT2Ring * kT2Tile;       // [4 output warps][32 rows x 128 B] output staging
   int* s_slot = reinterpret_cast<int*>(sStage + 8 * 2048);       // [batch + 1] first slot of every sequence, in the order of
   unsigned short* s_order = reinterpret_cast<unsigned short*>(s_slot + p.batch + 1);             // [batch]
   __shared__ __align__(8) uint64_t bar_item_full[kT2Items], bar_item_empty[kT2Items];
   __shared__ __align__(8) uint64_t bar_q_full[2], bar_q_empty[2];
-  __shared__ __align__(8) uint64_t bar_k_full[kT2Ring], bar_k_empty[kT2Ring], bar_v_full[kT2Ring], bar_v_empty[kT2Ring];
+  __shared__ __align__(8) uint64_t bar_k_full[kRingK], bar_k_empty[kRingK], bar_v_full[kT2Ring], bar_v_empty[kT2Ring];
   __shared__ __align__(8) uint64_t bar_s_full[2], bar_p_full[2], bar_o_final[2], bar_o_free[2];
   __shared__ __align__(8) uint64_t bar_l_full[2], bar_l_empty[2];
   __shared__ float s_inv[2][128];                        // 1 / row sum of a finished half, softmax -> output warpgroup
+  __shared__ float s_max[kSplit ? 2 : 1][128];           // kSplit: a half's row maximum (log2 units), its sum in s_inv
   __shared__ __align__(16) T2Item s_item[kT2Items];
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int G = p.G, QT = p.QT, QB = 2 * p.QT;
+  const int G = p.G, QT = p.QT, QB = (kSplit ? 1 : 2) * p.QT;
   const bool slot_in_smem = p.batch <= kT2MaxSeqSmem;
 
   if (tid == 0) {
@@ -272,9 +329,11 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       mbar_init(&bar_l_full[i], 4);
       mbar_init(&bar_l_empty[i], 4);
     }
-    for (int i = 0; i < kT2Ring; ++i) {
+    for (int i = 0; i < kRingK; ++i) {
       mbar_init(&bar_k_full[i], 1);
       mbar_init(&bar_k_empty[i], kStore ? 2 : 1);
+    }
+    for (int i = 0; i < kT2Ring; ++i) {
       mbar_init(&bar_v_full[i], 1);
       mbar_init(&bar_v_empty[i], kStore ? 2 : 1);
     }
@@ -345,7 +404,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
           const int shift = Lk - Lq;
           const int tq0 = qb * QB;
           const int nA = max(0, (min(Lk, shift + min(tq0 + QT, Lq)) + kT2Kv - 1) / kT2Kv);
-          b_rows = tq0 + QT < Lq;
+          b_rows = !kSplit && tq0 + QT < Lq;
           const int nB = b_rows ? max(0, (min(Lk, shift + min(tq0 + QB, Lq)) + kT2Kv - 1) / kT2Kv) : 0;
           seq = lo;
           q_row = q_begin + tq0;
@@ -356,8 +415,8 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
           s_item[is].Lq = Lq;
           s_item[is].Lk = Lk;
           s_item[is].k_begin = k_begin;
-          s_item[is].n[0] = nA;
-          s_item[is].n[1] = nB;
+          s_item[is].n[0] = kSplit ? (n + 1) >> 1 : nA;
+          s_item[is].n[1] = kSplit ? n >> 1 : nB;
         }
         s_item[is].seq = seq;
         mbar_arrive(&bar_item_full[is]);                                // an item, or the end marker
@@ -383,29 +442,42 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         ++n_pub;
         // K and V tiles
         const int* bt_row = p.block_tables ? p.block_tables + seq * p.bt_row_stride : nullptr;
-        for (int j = 0; j < n; ++j) {
-          int row0;
-          if (bt_row) {
-            const int tok0 = j * kT2Kv;
-            const int col = tok0 / p.block_size;
-            const long long blk = col < p.bt_cols ? bt_row[col] : -1;
-            row0 = (blk >= 0 && blk < p.num_blocks) ? static_cast<int>(blk * p.block_size + (tok0 - col * p.block_size))
-                                                    : -kT2Kv;
-          } else {
-            row0 = k_begin + j * kT2Kv;
-          }
-          const int ks = kt % kT2Ring;
-          if (!mbar_wait(&bar_k_empty[ks], ((kt / kT2Ring) & 1) ^ 1, abort_flag)) { ok = false; break; }
+        auto tile_row = [&](int j) -> int {
+          if (!bt_row) return k_begin + j * kT2Kv;
+          const int tok0 = j * kT2Kv;
+          const int col = tok0 / p.block_size;
+          const long long blk = col < p.bt_cols ? bt_row[col] : -1;
+          return (blk >= 0 && blk < p.num_blocks) ? static_cast<int>(blk * p.block_size + (tok0 - col * p.block_size)) : -kT2Kv;
+        };
+        auto load_k = [&](int row0) -> bool {
+          const int ks = kt % kRingK;
+          if (!mbar_wait(&bar_k_empty[ks], ((kt / kRingK) & 1) ^ 1, abort_flag)) return false;
           mbar_expect_tx(&bar_k_full[ks], kT2Tile);
           tma_load_3d(sK + ks * kT2Tile, &map_k, &bar_k_full[ks], 0, h, row0);
           tma_load_3d(sK + ks * kT2Tile + kT2Sub, &map_k, &bar_k_full[ks], 64, h, row0);
           ++kt;
+          return true;
+        };
+        auto load_v = [&](int row0) -> bool {
           const int vs = vt % kT2Ring;
-          if (!mbar_wait(&bar_v_empty[vs], ((vt / kT2Ring) & 1) ^ 1, abort_flag)) { ok = false; break; }
+          if (!mbar_wait(&bar_v_empty[vs], ((vt / kT2Ring) & 1) ^ 1, abort_flag)) return false;
           mbar_expect_tx(&bar_v_full[vs], kT2Tile);
           tma_load_3d(sV + vs * kT2Tile, &map_v, &bar_v_full[vs], 0, h, row0);
           tma_load_3d(sV + vs * kT2Tile + kT2Sub, &map_v, &bar_v_full[vs], 64, h, row0);
           ++vt;
+          return true;
+        };
+        if constexpr (kSplit) {
+          // K two tiles ahead of V: the issuer needs K of step j + 2 in step j
+          for (int j = 0; j < n + 2 && ok; ++j) {
+            if (j < n) ok = load_k(tile_row(j));
+            if (ok && j >= 2) ok = load_v(tile_row(j - 2));
+          }
+        } else {
+          for (int j = 0; j < n && ok; ++j) {
+            const int row0 = tile_row(j);
+            ok = load_k(row0) && load_v(row0);
+          }
         }
       }
     }
@@ -418,6 +490,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       const uint32_t q_lo = tc::smem_desc_sw128_lo(smem_u32(sQ), 16), k_lo = tc::smem_desc_sw128_lo(smem_u32(sK), 16);
       const uint32_t v_lo = tc::smem_desc_sw128_lo(smem_u32(sV), kT2Sub);
       int n_item = 0, kt = 0, vt = 0;
+      int k_at = 0, k_ph = 0; // kSplit: place and phase in the K ring
       int np[2] = {0, 0};     // P tiles consumed per half (phase of bar_p_full)
       int no[2] = {0, 0};     // items whose O was read out per half (phase of bar_o_free)
       bool ok = true;
@@ -425,7 +498,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) {
           const uint32_t off = ((ks >> 2) * kT2Sub + (ks & 3) * 32) >> 4;
-          tc::mma_ss_lo(tmem + hx * 128, q_lo + hx * (kT2Tile >> 4) + off, k_lo + kslot * (kT2Tile >> 4) + off, desc_hi,
+          tc::mma_ss_lo(tmem + hx * 128, q_lo + (kSplit ? 0 : hx) * (kT2Tile >> 4) + off, k_lo + kslot * (kT2Tile >> 4) + off, desc_hi,
                         idesc_qk, ks > 0);
         }
         tc::commit(&bar_s_full[hx]);
@@ -439,11 +512,54 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       while (ok) {
         const int is = n_item % kT2Items;
         if (!mbar_wait(&bar_item_full[is], (n_item / kT2Items) & 1, abort_flag)) break;
-        const int seq = s_item[is].seq, nA = s_item[is].n[0], nB = s_item[is].n[1], n = max(nA, nB);
+        const int seq = s_item[is].seq, nA = s_item[is].n[0], nB = s_item[is].n[1], n = kSplit ? nA + nB : max(nA, nB);
         mbar_arrive(&bar_item_empty[is]);
         if (seq < 0) break;
         const uint32_t qph = n_item & 1;
         if (!mbar_wait(&bar_q_full[0], qph, abort_flag) || !mbar_wait(&bar_q_full[1], qph, abort_flag)) break;
+        if constexpr (kSplit) {
+          // the first S of either half, then PV of step j (half j & 1) and that half's next S; ring places and phases are
+          // counted along, the half is a constant of the code: what this thread computes is tensor-core idle time
+          auto next_k = [&]() { if (++k_at == kRingK) { k_at = 0; k_ph ^= 1; } };
+          for (int j = 0; j < 2 && j < n && ok; ++j) {
+            if (!mbar_wait(&bar_k_full[k_at], k_ph, abort_flag)) { ok = false; break; }
+            tc::fence_after_sync();
+            issue_s(j, k_at);
+            tc::commit(&bar_k_empty[k_at]);
+            next_k();
+          }
+          if (n <= 2) { tc::commit(&bar_q_empty[0]); tc::commit(&bar_q_empty[1]); }
+          auto step = [&](auto half, int j) -> bool {
+            constexpr int hx = decltype(half)::value;
+            const int vslot = vt & 1;
+            if (!mbar_wait(&bar_v_full[vslot], (vt >> 1) & 1, abort_flag)) return false;
+            if (j + 2 < n && !mbar_wait(&bar_k_full[k_at], k_ph, abort_flag)) return false;
+            if (j < 2 && !mbar_wait(&bar_o_free[hx], (no[hx] & 1) ^ 1, abort_flag)) return false;
+            if (!mbar_wait(&bar_p_full[hx], np[hx] & 1, abort_flag)) return false;
+            ++np[hx];
+            tc::fence_after_sync();
+            issue_pv(hx, vslot, j >= 2);
+            tc::commit(&bar_v_empty[vslot]);
+            ++vt;
+            if (j + 2 >= n) {
+              tc::commit(&bar_o_final[hx]);
+              ++no[hx];
+            } else {
+              issue_s(hx, k_at);
+              tc::commit(&bar_k_empty[k_at]);
+              next_k();
+              if (j + 3 >= n) { tc::commit(&bar_q_empty[0]); tc::commit(&bar_q_empty[1]); }   // the item's last S
+            }
+            return true;
+          };
+          static_assert(kT2Ring == 2, "V ring");
+          for (int j = 0; j < n && ok; j += 2) {
+            ok = step(std::integral_constant<int, 0>{}, j);
+            if (ok && j + 1 < n) ok = step(std::integral_constant<int, 1>{}, j + 1);
+          }
+          ++n_item;
+          continue;
+        }
         // first K tile: S for both halves
         if (n > 0) {
           if (!mbar_wait(&bar_k_full[kt % kT2Ring], (kt / kT2Ring) & 1, abort_flag)) break;
@@ -495,6 +611,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
     uint64_t* const full = is_v ? bar_v_full : bar_k_full;
     uint64_t* const empty = is_v ? bar_v_empty : bar_k_empty;     // (a tile's slot is free when this warp is through, too)
     const unsigned char* const ring = is_v ? sV : sK;
+    const int depth = !kSplit || is_v ? kT2Ring : kRingK;
     const CUtensorMap* const map = is_v ? &map_vc : &map_kc;
     char* const cache = is_v ? p.st_v_cache : p.st_k_cache;
     int n_item = 0, kt = 0;
@@ -503,7 +620,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       const int is = n_item % kT2Items;
       if (!mbar_wait(&bar_item_full[is], (n_item / kT2Items) & 1, abort_flag)) break;
       const int seq = s_item[is].seq, h = s_item[is].h, tq0 = s_item[is].tq0, Lq = s_item[is].Lq, Lk = s_item[is].Lk;
-      const int k_begin = s_item[is].k_begin, n = max(s_item[is].n[0], s_item[is].n[1]);
+      const int k_begin = s_item[is].k_begin, n = kSplit ? s_item[is].n[0] + s_item[is].n[1] : max(s_item[is].n[0], s_item[is].n[1]);
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar_item_empty[is]);
       if (seq < 0) break;
@@ -513,11 +630,11 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       const int j0 = Lq == Lk ? (tq0 + kT2Kv - 1) / kT2Kv : tq0 + QB >= Lq ? 0 : n;
       const int j1 = Lq == Lk ? min(n, (tq0 + QB + kT2Kv - 1) / kT2Kv) : n;
       for (int j = 0; j < n; ++j, ++kt) {
-        const int slot = kt % kT2Ring;
+        const int slot = kt % depth;
         const bool mine = j >= j0 && j < j1;
         const int row0 = k_begin + j * kT2Kv, rows = min(min(kT2Kv, Lk - j * kT2Kv), p.st_tokens - row0);
         const int s0 = mine ? t2_store_slots(p, row0, rows, lane) : -1;
-        if (!mbar_wait(&full[slot], (kt / kT2Ring) & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait(&full[slot], (kt / depth) & 1, abort_flag)) { ok = false; break; }
         if (mine) t2_store_tile(p, map, cache, ring + slot * kT2Tile, h, row0, rows, s0, lane);
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[slot]);
@@ -556,18 +673,20 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       if (it.seq < 0) break;
       ++n_item;
       const int nx = hx ? it.n[1] : it.n[0];
-      const int n_all = max(it.n[0], it.n[1]);
+      const int n_all = kSplit ? it.n[0] + it.n[1] : max(it.n[0], it.n[1]);
+      const int row_half = kSplit ? 0 : hx;               // which rows and ...
       const int shift = it.Lk - it.Lq;
-      const int tok = it.tq0 + hx * QT + r / G;
+      const int tok = it.tq0 + row_half * QT + r / G;
       const bool row_ok = r < QT * G && tok < it.Lq;
       const int kmax = row_ok ? shift + tok : -1;          // last visible key (inclusive)
-      const int first_row_kmax = shift + it.tq0 + hx * QT;
+      const int first_row_kmax = shift + it.tq0 + row_half * QT;
       float m_used = -INFINITY, l = 0.f;
       for (int j = 0; j < nx; ++j) {
         if (!mbar_wait(&bar_s_full[hx], ns & 1, abort_flag)) { ok = false; break; }
         ++ns;
         tc::fence_after_sync();
-        const int key0 = j * kT2Kv;
+        const int tile = kSplit ? 2 * j + hx : j;        // ... which key tiles this half works on
+        const int key0 = tile * kT2Kv;
         const bool need_mask = key0 + kT2Kv - 1 > first_row_kmax;
         // the whole S row in registers: four TMEM loads in flight, one wait
         uint32_t sv[4][32];
@@ -661,7 +780,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         if (key0 + kT2Kv > it.Lk) {
           // ragged last tile of the sequence: V rows past its end are foreign data; zero them so
           // that 0 * garbage cannot turn into NaN inside the tensor core
-          const int vt = vt_base + j;
+          const int vt = vt_base + tile;
           if (!mbar_wait(&bar_v_full[vt % kT2Ring], (vt / kT2Ring) & 1, abort_flag)) { ok = false; break; }
           // (Rows are 128 bytes and follow each other, so they are zeroed as one range, thread after thread: a row per
           // thread hits the same banks with every lane and took 2000 cycles.)
@@ -682,13 +801,14 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       if (nx > 0) {
         // the row's 1 / sum goes to the output warpgroup, which drains O while this one moves on
         if (!mbar_wait(&bar_l_empty[hx], (n_fin & 1) ^ 1, abort_flag)) { ok = false; break; }
-        s_inv[hx][r] = l > 0.f ? 1.f / l : 0.f;
+        if constexpr (kSplit) s_max[hx][r] = m_used == -INFINITY ? -INFINITY : m_used * c;
+        s_inv[hx][r] = kSplit ? l : l > 0.f ? 1.f / l : 0.f;
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar_l_full[hx]);
         ++n_fin;
-      } else if (row_ok) {
+      } else if (row_ok && (!kSplit || n_all == 0) && !(kSplit && hx)) {
         // no visible key at all (Lk < Lq rows): zeros, as the reference's attention library does
-        uint4* dst = reinterpret_cast<uint4*>(p.out + (static_cast<long long>(it.q_row + hx * QT + r / G) * p.H + it.h * G + r % G) * 128);
+        uint4* dst = reinterpret_cast<uint4*>(p.out + (static_cast<long long>(it.q_row + row_half * QT + r / G) * p.H + it.h * G + r % G) * 128);
 #pragma unroll
         for (int i = 0; i < 16; ++i) dst[i] = make_uint4(0, 0, 0, 0);
       }
@@ -711,6 +831,35 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       if (lane == 0) mbar_arrive(&bar_item_empty[is]);
       if (seq < 0) break;
       ++n_item;
+      if constexpr (kSplit) {
+        if (nA <= 0) continue;
+        const bool has_b = nB > 0;
+        float m[2] = {0.f, -INFINITY}, l[2] = {0.f, 0.f};
+#pragma unroll
+        for (int hx = 0; hx < 2; ++hx) {
+          if (hx == 1 && !has_b) continue;
+          if (!mbar_wait(&bar_l_full[hx], nf[hx] & 1, abort_flag)) ok = false;
+          m[hx] = s_max[hx][r];
+          l[hx] = s_inv[hx][r];
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bar_l_empty[hx]);
+          if (!mbar_wait(&bar_o_final[hx], nf[hx] & 1, abort_flag)) ok = false;
+          ++nf[hx];
+        }
+        if (!ok) break;
+        tc::fence_after_sync();
+        const float M = fmaxf(m[0], m[1]);
+        float wa = M == -INFINITY ? 0.f : fast_exp2(m[0] - M), wb = M == -INFINITY ? 0.f : fast_exp2(m[1] - M);
+        const float sum = l[0] * wa + l[1] * wb, inv = sum > 0.f ? 1.f / sum : 0.f;
+        const bool tma = p.out_tma && tq0 + quarter * 32 / G + 32 / G <= Lq;
+        if (!tma) {
+          if (lane == 0) tma_store_wait_read();
+          __syncwarp();
+        }
+        t2_output_split(p, &map_o, tmem + 256 + lane_base, tmem + 384 + lane_base, has_b, bar_o_free, sStage + quarter * 4096, lane,
+                        quarter, wa * inv, wb * inv, tma, q_row, h, tq0, Lq);
+        continue;
+      }
 #pragma unroll 1
       for (int hx = 0; hx < 2; ++hx) {
         if ((hx == 0 ? nA : nB) <= 0) continue;
@@ -772,15 +921,17 @@ int inject_timeout_prefill_tc2() {
   return check_cuda(cudaMemcpyToSymbol(g_prefill_ticket, &stale, sizeof(unsigned int)), "inject_timeout: ticket counter");
 }
 
-// Needs whole query heads groups in a 128-row tile.  The query-block slots are laid out for 2 * QT tokens.
-int launch_prefill_tc2(PrefillParams p, const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v,
+// Needs whole query heads groups in a 128-row tile.  The query-block slots are laid out for 2 * QT tokens, or QT with `split`.
+int launch_prefill_tc2(PrefillParams p, bool split, const CUtensorMap& map_q, const CUtensorMap& map_k, const CUtensorMap& map_v,
                        const CUtensorMap& map_o, const CUtensorMap& map_kc, const CUtensorMap& map_vc, cudaStream_t stream) {
-  p.n_slots = p.total_q / (2 * p.QT) + p.batch;
-  const size_t smem = 1024 + static_cast<size_t>(2 + 2 * kT2Ring) * kT2Tile + 8 * 2048 +
+  p.n_slots = p.total_q / ((split ? 1 : 2) * p.QT) + p.batch;
+  const size_t smem = static_cast<size_t>(2 + 2 * kT2Ring) * kT2Tile + 8 * 2048 +
                       (p.batch <= kT2MaxSeqSmem ? (p.batch + 1) * 6 : 4) + 64;
-  static std::atomic<size_t> configured[2][kMaxDevices];
-  auto* const kernel = p.st_slots ? prefill_attn_tc2_kernel<true> : prefill_attn_tc2_kernel<false>;
-  const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem, configured[p.st_slots != nullptr],
+  static std::atomic<size_t> configured[4][kMaxDevices];
+  const bool store = p.st_slots != nullptr;
+  auto* const kernel = split ? (store ? prefill_attn_tc2_kernel<true, true> : prefill_attn_tc2_kernel<false, true>)
+                             : (store ? prefill_attn_tc2_kernel<true, false> : prefill_attn_tc2_kernel<false, false>);
+  const int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem, configured[2 * split + store],
                                      "prefill_attn(tcgen05): cudaFuncSetAttribute");
   if (rc) return rc;
   const int grid = sm_count();

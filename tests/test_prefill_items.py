@@ -1,0 +1,53 @@
+"""GPU: how the tcgen05 prefill kernel hands out its work -- few items, whose keys the two halves share tile by tile (one tile,
+odd and even numbers of them, rows that see nothing of a half's only tile), and many, in the order of their lengths
+(batches up to the sort's limit, beyond it, and beyond the slot table) -- dense and paged, against the oracle."""
+import pytest
+import torch
+
+from oracle.attention_oracle import prefill_attn_ref
+from workloads import cu_seqlens, default_scale
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+EDGES = [1, 127, 128, 129, 255, 256, 257, 384, 385, 513, 640, 900]
+
+
+@pytest.mark.parametrize("paged", [False, True])
+@pytest.mark.parametrize("h,hkv,lq,lk", [
+    (2, 1, EDGES, None), (1, 1, [1], None), (4, 1, [33], None), (8, 1, [130], None), (16, 8, [1500], None), (128, 1, [70], None),
+    (4, 2, [1, 64, 65, 200], [129, 320, 1000, 201]),         # cached prefixes
+    (2, 1, [300, 0, 70, 300], [100, 50, 1, 257]),            # rows without a visible key
+    (32, 8, EDGES * 4, None), (16, 8, (EDGES * 22)[:256], None), (16, 8, (EDGES * 22)[:257], None),
+    (4, 2, [1 + i % 150 for i in range(1100)], None),
+])
+def test_tcgen05_items(paged, h, hkv, lq, lk):
+    from nanovllm_b200.layers.attention import prefill_attention
+    lk = lk or lq
+    g = torch.Generator().manual_seed(sum(lk) + h)
+    n = sum(lk)
+    q = torch.randn(sum(lq), h, 128, generator=g).to(torch.bfloat16)
+    k = torch.randn(n, hkv, 128, generator=g).to(torch.bfloat16)
+    v = torch.randn(n, hkv, 128, generator=g).to(torch.bfloat16)
+    cu_q, cu_k = cu_seqlens(lq), cu_seqlens(lk)
+    args, bt = (k.to(DEV), v.to(DEV)), None
+    if paged:
+        cols = -(-max(lk) // 256)
+        blocks = sum(-(-m // 256) for m in lk) + 1
+        perm = torch.randperm(blocks, generator=g).tolist()
+        bt = torch.full((len(lk), cols), -1, dtype=torch.int32)
+        kc = torch.full((blocks, 256, hkv, 128), float("nan"), dtype=torch.bfloat16)     # what is not the sequence's own
+        vc = torch.full((blocks, 256, hkv, 128), float("nan"), dtype=torch.bfloat16)
+        at = 0
+        for i, m in enumerate(lk):
+            for c in range(-(-m // 256)):
+                rows = min(256, m - 256 * c)
+                b = perm.pop()
+                bt[i, c] = b
+                kc[b, :rows], vc[b, :rows] = k[at:at + rows], v[at:at + rows]
+                at += rows
+        args, bt = (kc.to(DEV), vc.to(DEV)), bt.to(DEV)
+    scale = default_scale(128)
+    out = prefill_attention(q.to(DEV), *args, cu_q.to(DEV), cu_k.to(DEV), max(lq), max(lk), scale, hkv, bt, kernel_variant=2)
+    torch.cuda.synchronize()
+    ref = prefill_attn_ref(q, k, v, cu_q, cu_k, scale).float()
+    torch.testing.assert_close(out.float().cpu(), ref, atol=2e-2, rtol=1e-2)
