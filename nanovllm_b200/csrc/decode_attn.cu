@@ -43,6 +43,7 @@ constexpr int kDecPending = 8;             // partials written but not yet count
 constexpr int kDecClasses = 64;            // length classes of the sort
 constexpr int kSortRows = kDecPer * kDecWarps;
 constexpr int kDecMinPart = 4;             // tiles: shorter parts would cost more to merge than to stream
+constexpr int kDecOneWaveShare = 12;       // tiles per CTA up to which parts get a CTA each
 constexpr int kPartialSlots = 12;          // of the workspace, per CTA of the grid
 static __device__ int g_status_decode = 0;
 
@@ -182,6 +183,7 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
   __shared__ __align__(16) UnitDesc s_desc[kUnitRing];
   __shared__ __align__(16) UnitDesc s_merge_desc[2];
   __shared__ __align__(16) UnitDesc s_pending[kDecPending];
+  __shared__ int s_parts[kDecWarps];
   __shared__ int s_warp_sums[kDecWarps], s_warp_max[kDecWarps], s_warp_live[kDecWarps];
   __shared__ int s_abort, s_known, s_last, s_decision, s_merge_all;
 
@@ -263,17 +265,36 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
     // Pairs are cut only if the longest one is well above a CTA's equal share of the tiles: whole pairs, longest first,
     // level out well enough below that and leave nothing to merge.  The line is 1.25 shares, or 1.85 where
     // every CTA has at most one pair (short and long ones share an SM then, and the long one gets the SM's bandwidth when
-    // the short one is done).  Above it, pairs longer than 2/3 of a share (and kDecMinPart tiles) are cut into
+    // the short one is done), and 3 tiles, which is what a merge costs (90 sequences of 20 .. 400 tokens, 4 kv heads:
+    // 14.6 -> 11.5 us uncut).  Above it, pairs longer than 2/3 of a share (and kDecMinPart tiles) are cut into
     // equal parts: 1/2 and 1/3 leave parts of a size that do not add up to a share, and cost more merges (measured over
     // batches of 16 .. 500 sequences of 1 .. 8192 tokens).  The parts come first in the order, so that their merging
     // happens while the whole pairs stream.  A part is longer than a third of a share, so there are at most
     // 3 x grid of them: the workspace's kPartialSlots x grid slots hold every partial.
+    // With fewer pairs than CTAs and a small share, the parts are instead as short as they can be with a CTA for
+    // each, 1 .. 1.5 shares: no CTA starts a second unit, and there are half as many partials.  5 sequences of 47 ..
+    // 4381 tokens, 8 kv heads: 21.1 -> 14.2 us; 20 of 500 .. 1500, 4 kv heads: 17.7 -> 13.2; 128 of 30 .. 600, 2 kv heads: 16.3 ->
+    // 12.4.  From kDecOneWaveShare on, levelling through the tickets is as good or better.
     const long long tiles = total * Hkv;
-    const int line = live * Hkv <= static_cast<int>(gridDim.x) ? 185 : 125;
+    const int grid = static_cast<int>(gridDim.x);
+    const bool one_wave = live * Hkv <= grid;
     un.cap = longest;
-    if (static_cast<long long>(longest) * gridDim.x * 100 > line * tiles) {
-      const long long part = 2 * tiles / (3 * static_cast<int>(gridDim.x)) + 1;
+    if (static_cast<long long>(longest) * grid * 100 > (one_wave ? 185 : 125) * tiles && (longest - 3ll) * grid > tiles) {
+      const long long part = 2 * tiles / (3 * grid) + 1;
       un.cap = static_cast<int>(part < kDecMinPart ? kDecMinPart : part < longest ? part : longest);
+      if (one_wave && tiles <= kDecOneWaveShare * grid && longest < 65535) {       // (the same in every thread)
+        const int share = static_cast<int>((tiles + grid - 1) / grid);
+        // each warp counts the parts for one length
+        const int step = (share + 9) / 10, cap = max(kDecMinPart, share + warp * step);
+        int n = 0;
+        for (int i = lane; i < p.batch; i += 32) n += (s_nt[i] + cap - 1) / cap;
+        n = __reduce_add_sync(0xffffffffu, n);
+        if (lane == 0) s_parts[warp] = n;
+        __syncthreads();
+#pragma unroll
+        for (int w = kDecWarps - 1; w >= 0; --w)
+          if (s_parts[w] * Hkv <= grid) un.cap = min(longest, max(kDecMinPart, share + w * step));
+      }
     }
     un.live = live;
     un.split = longest > un.cap;

@@ -1,6 +1,6 @@
 """GPU: how the two decode kernels share out a batch, at the sizes where it can go wrong -- clusters of every size
 (fewer tiles than CTAs, ragged shares), whole pairs just below and above one per CTA, cut pairs (one long sequence
-among short ones), rows without context -- against the CPU oracle."""
+among short ones; few long ones, whose parts get a CTA each), rows without context -- against the CPU oracle."""
 import pytest
 import torch
 
@@ -19,6 +19,8 @@ def _lens(kind, n):
         return torch.randint(0, 700, (n,), generator=g).tolist()
     if kind == "one long":
         return [6000 if i == n // 2 else 1 + i % 130 for i in range(n)]
+    if kind == "spread":
+        return [100 + 2900 * i // n for i in range(n)]
     return [int(kind)] * n                                    # one length
 
 
@@ -27,6 +29,7 @@ def _lens(kind, n):
     ("ragged", 3, 16, 8), ("ragged", 17, 2, 2), ("ragged", 60, 4, 1), ("ragged", 130, 4, 1), ("one long", 5, 16, 8),
     ("513", 3, 32, 2), ("ragged", 9, 5, 1),                                  # 16 and 5 query heads per kv head
     ("equal", 37, 16, 8), ("equal", 149, 4, 2), ("ragged", 296, 1, 1), ("ragged", 297, 1, 1), ("ragged", 512, 4, 1),
+    ("spread", 20, 16, 4), ("spread", 100, 2, 1), ("spread", 148, 4, 2), ("9000", 2, 4, 2), ("9000", 1, 2, 1),   # a CTA per part
     ("one long", 40, 16, 8), ("one long", 300, 4, 1), ("one long", 513, 2, 1), ("0", 200, 2, 1),
 ])
 def test_decode_shares(kind, n, h, hkv):
