@@ -88,8 +88,8 @@ int b200_decode_attn(const void* q, int64_t q_row_stride, const void* k_cache, c
 
 /* b200_store_kvcache(k, v, ..) of one row per sequence and b200_decode_attn as one call, the layer's decode step
  * (nanovllm/layers/attention.py:59-74): row i of k and v goes to flat cache row slot_mapping[i] (-1 and slots outside the
- * cache are skipped), and attention sees the cache with all of the step's rows in place.  A batch with few (sequence,
- * kv head) pairs is one launch, any other the two kernels one after the other. */
+ * cache are skipped), and attention sees the cache with all of the step's rows in place.  Up to 160 sequences, or few
+ * (sequence, kv head) pairs, it is one launch, else the two kernels one after the other. */
 int b200_store_decode_attn(const void* q, int64_t q_row_stride, const void* k, const void* v, int64_t k_row_stride,
                            int64_t v_row_stride, const int32_t* slot_mapping, void* k_cache, void* v_cache,
                            int64_t num_blocks, int32_t block_size, const int32_t* block_tables, int64_t bt_row_stride,

@@ -43,6 +43,11 @@ constexpr int kDecPending = 8;             // partials written but not yet count
 constexpr int kDecClasses = 64;            // length classes of the sort
 constexpr int kSortRows = kDecPer * kDecWarps;
 constexpr int kDecMinPart = 4;             // tiles: shorter parts would cost more to merge than to stream
+// Sequences up to which the cache store rides in the launch (its slots take the place of the other tables' upper halves).  Beyond,
+// going through the slots for every last tile costs what the launch of its own does: eager layer, 128 sequences of 100 .. 2048
+// (16/8 heads) 90.2 -> 87.6 us, 160: 110.6 -> 109.9, 200: 135.3 -> 137.0.
+constexpr int kDecStoreBatch = 160;
+constexpr int kBloomWords = 64, kBloomBits = 11;  // (256 bytes: what static shared memory has left of its 1 KiB)
 constexpr int kDecOneWaveShare = 12;       // tiles per CTA up to which parts get a CTA each
 constexpr int kPartialSlots = 12;          // of the workspace, per CTA of the grid
 static __device__ int g_status_decode = 0;
@@ -161,6 +166,37 @@ __device__ __forceinline__ void dec_store_partial(const DecodeParams& p, int slo
   if (lane == 0) *reinterpret_cast<float2*>(p.ws_ml + (slot * p.G + gq) * 2) = make_float2(r.M, r.L);
 }
 
+// kStore: the step's cache store in the same launch, as in decode_cluster.cu: nobody relies on finding another CTA's row in
+// the cache.  The epilogue warps write the step's rows, and whoever loads a tile that covers any slot of the step puts the
+// new rows into its copy.  Which tiles may do so every CTA knows from a small Bloom filter over the slots' tiles; only for
+// those do the consumer warps go through the slots (eager layer, 37 sequences of 100 .. 1024, 16/8 heads: 19.9 -> 17.1 us).
+__device__ __forceinline__ uint32_t dec_bloom_a(int slot) { return (slot >> 6) & (kBloomWords * 32 - 1); }
+__device__ __forceinline__ uint32_t dec_bloom_b(int slot) { return (static_cast<uint32_t>(slot >> 6) * 2654435761u) >> (32 - kBloomBits); }
+
+// The step's rows among this warp's 16 rows of the tile that starts at slot0.
+__device__ __forceinline__ void dec_patch_rows(const DecodeParams& p, const int* s_slots, unsigned char* stage, int warp, int lane,
+                                               int slot0, int h) {
+  bool any = false;
+  for (int i0 = 0; i0 < p.batch; i0 += 32) {
+    const int slot = i0 + lane < p.batch ? s_slots[i0 + lane] : -1;
+    const int row = slot - slot0 - warp * 16;
+    unsigned found = __ballot_sync(0xffffffffu, slot >= 0 && row >= 0 && row < 16);
+    while (found) {
+      const int src = __ffs(found) - 1;
+      found &= found - 1;
+      const int r = warp * 16 + __shfl_sync(0xffffffffu, row, src), c = lane & 15;
+      *reinterpret_cast<uint4*>(stage + (lane < 16 ? 0 : 2 * kSubTileBytes) + (c >> 3) * kSubTileBytes + r * 128 +
+                                (((c & 7) ^ (r & 7)) << 4)) = step_chunk(p, i0 + src, h, lane);
+      any = true;
+    }
+  }
+  if (any) {
+    fence_proxy_async_smem();
+    __syncwarp();
+  }
+}
+
+template <bool kStore>
 __global__ void __launch_bounds__(kDecThreads, 2)
 decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map_k,
                    const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_k16,
@@ -172,9 +208,11 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
   float* merge_o = reinterpret_cast<float*>(s_q + kUnitRing * G * 128);                           // [n_merge][4][G][128]
   float* merge_ml = merge_o + p.n_merge * kDecConsumerWarps * G * 128;                              // [n_merge][4][G][2]
   unsigned short* s_order = reinterpret_cast<unsigned short*>(merge_ml + p.n_merge * kDecConsumerWarps * G * 2);
-  unsigned short* s_base = s_order + kDecMaxBatch;
-  unsigned short* s_nt = s_base + kDecMaxBatch;
-  unsigned char* s_tail = reinterpret_cast<unsigned char*>(s_nt + kDecMaxBatch);
+  constexpr int kMaxBatch = kStore ? kDecStoreBatch : kDecMaxBatch;
+  unsigned short* s_base = s_order + kMaxBatch;
+  unsigned short* s_nt = s_base + kMaxBatch;
+  unsigned char* s_tail = reinterpret_cast<unsigned char*>(s_nt + kMaxBatch);
+  int* s_slots = reinterpret_cast<int*>(s_tail + kMaxBatch);                 // kStore: [batch], -1 where nothing is stored
   __shared__ __align__(8) uint64_t bar_full[kDecStages];
   __shared__ __align__(8) uint64_t bar_empty[kDecStages];
   __shared__ __align__(8) uint64_t bar_merge_full[2];
@@ -184,6 +222,8 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
   __shared__ __align__(16) UnitDesc s_merge_desc[2];
   __shared__ __align__(16) UnitDesc s_pending[kDecPending];
   __shared__ int s_parts[kDecWarps];
+  __shared__ uint32_t s_bloom[kStore ? kBloomWords : 1];
+  __shared__ int s_patch[kStore ? kDecStages : 1];       // a stage's first slot, or -1: no row of the step in it
   __shared__ int s_warp_sums[kDecWarps], s_warp_max[kDecWarps], s_warp_live[kDecWarps];
   __shared__ int s_abort, s_known, s_last, s_decision, s_merge_all;
 
@@ -232,6 +272,7 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
     const int i0 = tid * per;
     int local[kDecPer];
     int sum = 0, longest = 0, live = 0;
+    if (kStore && tid < kBloomWords) s_bloom[tid] = 0;
 #pragma unroll
     for (int k = 0; k < kDecPer; ++k) {
       int nt = 0;
@@ -254,6 +295,16 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
     if (lane == 0) { s_warp_sums[warp] = sum; s_warp_max[warp] = longest; s_warp_live[warp] = live; }
     __syncthreads();
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if constexpr (kStore) {
+      for (int i = tid; i < p.batch; i += kDecThreads) {
+        const int slot = __ldg(p.st_slots + i);
+        const bool stored = slot >= 0 && slot < p.st_n_slots;
+        s_slots[i] = stored ? slot : -1;
+        if (!stored) continue;
+        atomicOr(&s_bloom[dec_bloom_a(slot) >> 5], 1u << (dec_bloom_a(slot) & 31));
+        atomicOr(&s_bloom[dec_bloom_b(slot) >> 5], 1u << (dec_bloom_b(slot) & 31));
+      }
+    }
     long long total = 0;
     longest = live = 0;
 #pragma unroll
@@ -392,6 +443,16 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
         for (int v = lane; v < p.H * 16; v += 32) o[v] = make_uint4(0, 0, 0, 0);
       }
     }
+    if constexpr (kStore) {
+      for (int i = blockIdx.x; i < p.batch; i += gridDim.x) {
+        const long long slot = s_slots[i];
+        if (slot < 0) continue;
+#pragma unroll 4
+        for (int h = 0; h < Hkv; ++h)
+          *reinterpret_cast<uint4*>((lane < 16 ? p.st_k_cache : p.st_v_cache) + (slot * Hkv + h) * 128 + (lane & 15) * 8) =
+              step_chunk(p, i, h, lane);
+      }
+    }
   }
 
   const int cta = blockIdx.x;
@@ -448,6 +509,10 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
         const bool first = t == cur.t0;
         // descriptor and query rows travel with the unit's first tile
         if (first) s_desc[n_unit % kUnitRing] = cur;
+        if constexpr (kStore) {
+          const uint32_t a = dec_bloom_a(slot0), b = dec_bloom_b(slot0);
+          s_patch[stage] = slot0 >= 0 && ((s_bloom[a >> 5] >> (a & 31)) & (s_bloom[b >> 5] >> (b & 31)) & 1) ? slot0 : -1;
+        }
         mbar_expect_tx(&bar_full[stage], dec_tile_bytes(nslab) + (first ? G * 256 : 0));
         if (first)
           bulk_load_1d(s_q + (n_unit % kUnitRing) * G * 128,
@@ -610,6 +675,10 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
       const uint32_t ph = (it / kDecStages) & 1;
       if (t != d.t0 && !mbar_wait(&bar_full[stage], ph, abort_flag)) { ok = false; break; }
       const int valid = d.len - (t * kTile + warp * 16);  // valid tokens in this warp's 16-token slab
+      if constexpr (kStore) {
+        const int slot0 = s_patch[stage];
+        if (slot0 >= 0 && valid > 0) dec_patch_rows(p, s_slots, stages + stage * kStageBytes, warp, lane, slot0, d.h);
+      }
       if (valid > 0) dec_tile(stages + stage * kStageBytes, warp, lane, valid, p.scale_log2, qa, acc);
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar_empty[stage]);
@@ -775,9 +844,7 @@ static int decode(const void* q, int64_t q_row_stride, const void* k_cache, cons
   if (rc) return rc;
 
   const size_t smem = decode_smem_bytes(G);
-  static std::atomic<size_t> configured[kMaxDevices];
-  rc = ensure_dynamic_smem(reinterpret_cast<const void*>(decode_attn_kernel), smem, configured, "decode_attn: cudaFuncSetAttribute");
-  if (rc) return rc;
+  static std::atomic<size_t> configured[2][kMaxDevices];
 
   unsigned char* ws = static_cast<unsigned char*>(workspace);
   DecodeParams p;
@@ -803,7 +870,7 @@ static int decode(const void* q, int64_t q_row_stride, const void* k_cache, cons
     p.block_tables = block_tables + b0 * bt_row_stride;
     p.st_slots = nullptr;
     const int ctas = decode_cluster_ctas(p.batch, num_kv_heads, G, static_cast<int>(static_cast<long long>(bt_cols) * block_size / kTile));
-    if (store && ctas && p.batch == batch) {
+    if (store && (ctas || batch <= kDecStoreBatch) && p.batch == batch) {
       p.st_slots = store->slots;
       p.st_k = static_cast<const __nv_bfloat16*>(store->k);
       p.st_v = static_cast<const __nv_bfloat16*>(store->v);
@@ -822,7 +889,10 @@ static int decode(const void* q, int64_t q_row_stride, const void* k_cache, cons
       if (rc) return rc;
       continue;
     }
-    const cudaError_t le = launch_early(decode_attn_kernel, grid, kDecThreads, smem, static_cast<cudaStream_t>(stream), p, map_k, map_v, map_k16, map_v16);
+    auto* const kernel = p.st_slots ? decode_attn_kernel<true> : decode_attn_kernel<false>;
+    rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem, configured[p.st_slots != nullptr], "decode_attn: cudaFuncSetAttribute");
+    if (rc) return rc;
+    const cudaError_t le = launch_early(kernel, grid, kDecThreads, smem, static_cast<cudaStream_t>(stream), p, map_k, map_v, map_k16, map_v16);
     g_launches.fetch_add(1);
     rc = check_cuda(le != cudaSuccess ? le : cudaGetLastError(), "decode_attn launch");
     if (rc) return rc;

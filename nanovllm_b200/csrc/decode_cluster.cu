@@ -57,12 +57,6 @@ __device__ __forceinline__ bool cluster_mbar_wait(uint64_t* bar, uint32_t parity
   }
 }
 
-// One 16-byte chunk per lane of head h of the step's row `tok`: lanes 0 .. 15 K, 16 .. 31 V.
-__device__ __forceinline__ uint4 step_chunk(const DecodeParams& p, int tok, int h, int lane) {
-  const __nv_bfloat16* src = lane < 16 ? p.st_k + tok * p.st_k_stride : p.st_v + tok * p.st_v_stride;
-  return __ldg(reinterpret_cast<const uint4*>(src + h * 128 + (lane & 15) * 8));
-}
-
 // kStore: the step's cache store (nanovllm/layers/attention.py:62-63) in the same launch; as one of its own it is half of what
 // an eager step of a small batch costs the host.  Nothing orders this launch's CTAs, so none of them relies on finding
 // another's row in the cache: rank 0 of (sequence i, head h) writes row i of head h to its slot, and whoever loads a tile

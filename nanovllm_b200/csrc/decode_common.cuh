@@ -29,12 +29,18 @@ struct DecodeParams {
   float* ws_ml;   // [slots][G][2]   running max (log2 domain) and sum
   int* counters;  // [batch * Hkv], zero between launches
   unsigned int* ticket;  // unit scheduler, zero between launches
-  // the step's cache store in the same launch (cluster kernel): row i of st_k / st_v to slot st_slots[i]; nullptr: none
+  // the step's cache store in the same launch: row i of st_k / st_v to slot st_slots[i]; nullptr: none
   const int* st_slots;
   const __nv_bfloat16 *st_k, *st_v;
   long long st_k_stride, st_v_stride, st_n_slots;   // elements; slots of the cache
   __nv_bfloat16 *st_k_cache, *st_v_cache;
 };
+
+// One 16-byte chunk per lane of head h of the step's row `tok`: lanes 0 .. 15 K, 16 .. 31 V.
+__device__ __forceinline__ uint4 step_chunk(const DecodeParams& p, int tok, int h, int lane) {
+  const __nv_bfloat16* src = lane < 16 ? p.st_k + tok * p.st_k_stride : p.st_v + tok * p.st_v_stride;
+  return __ldg(reinterpret_cast<const uint4*>(src + h * 128 + (lane & 15) * 8));
+}
 
 // 1-D bulk copy global -> shared, completion counted on an mbarrier (addresses and size multiples of 16).
 __device__ __forceinline__ void bulk_load_1d(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {

@@ -51,7 +51,8 @@ def test_decode_shares(kind, n, h, hkv):
 
 
 @pytest.mark.parametrize("slots", ["own", "anywhere", "holes"])
-@pytest.mark.parametrize("n,h,hkv", [(1, 16, 8), (3, 8, 8), (9, 2, 1), (70, 4, 2), (140, 2, 1), (20, 16, 8)])
+@pytest.mark.parametrize("n,h,hkv", [(1, 16, 8), (3, 8, 8), (9, 2, 1), (70, 4, 2), (140, 2, 1), (20, 16, 8), (37, 16, 8), (160, 8, 4),
+                                     (161, 4, 2), (513, 2, 1)])
 def test_layer_decode_with_store(slots, n, h, hkv):
     """The step's rows stored in the attention launch: at the sequences' ends, in other sequences' blocks (whoever reads such
     a row must see the new one), skipped and outside the cache; a row without context is stored all the same."""
