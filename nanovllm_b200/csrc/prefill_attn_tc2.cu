@@ -45,6 +45,26 @@ static __device__ int g_status_prefill_tc2 = 0;
 
 static __device__ unsigned int g_prefill_ticket = 0;
 
+// The kernel's bounded waits.  Six roles run through their loops at the same time and share the SM's instruction cache, so code
+// size is time here: with these in place of mbar_wait() (a clock read, its 64-bit comparison and a spin counter at each of
+// some thirty places), the output and rescaling loops rolled and the mask taken from bits, 256 prompts of 100 .. 1024 tokens with
+// the store went from 805 to 700 us, 256 of 10 .. 300 without it from 162 to 142.  A failed test comes back after the hardware's own
+// suspension, at the least some 50 ns, so the limit is 0.2 s or more.
+constexpr int kT2WaitLimit = 1 << 22;
+__device__ __forceinline__ bool t2_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+#pragma unroll 1
+  for (int n = 0; n < kT2WaitLimit; ++n) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if (*abort_flag) return false;
+  }
+  *abort_flag = 1;
+  return false;
+}
+// On the S -> softmax -> PV chain: the second test does not come behind a look at the flag (long sequences lose 3 % to it).
+__device__ __forceinline__ bool t2_wait_hot(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return mbar_try_wait(bar, parity) || t2_wait(bar, parity, abort_flag);
+}
+
 struct T2Item {
   int seq;        // -1: no more work
   int h;
@@ -127,7 +147,7 @@ __device__ __forceinline__ void t2_output_tma(const CUtensorMap* map_o, uint32_t
   // eight 16-column chunks, the TMEM load of the next one in flight while one is converted
   uint32_t a[16], b[16];
   tc::ld_32x32b_x16(tmem_o_lane, a);
-#pragma unroll
+#pragma unroll 1      // (code size: t2_wait)
   for (int bx = 0; bx < 4; ++bx) {
     unsigned char* box = stage + (bx & 1) * 2048;
     if (lane == 0) tma_store_wait_read_but_one();        // the store before the previous one has left this box
@@ -382,7 +402,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         if (tk == n_items + gridDim.x - 1) atomicExch(&g_prefill_ticket, 0u);
         // the descriptor is built in its ring slot; only what the loads need stays in registers
         const int is = n_pub % kT2Items;
-        if (!mbar_wait(&bar_item_empty[is], ((n_pub / kT2Items) & 1) ^ 1, abort_flag)) { ok = false; break; }
+        if (!t2_wait(&bar_item_empty[is], ((n_pub / kT2Items) & 1) ^ 1, abort_flag)) { ok = false; break; }
         int seq = -1, h = 0, q_row = 0, k_begin = 0, n = 0;
         bool b_rows = false;                                            // half B holds query rows
         if (tk < n_items) {
@@ -432,7 +452,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         // Q tiles (the buffers are free once every S MMA of the previous item has completed)
         const uint32_t qph = (n_pub & 1) ^ 1;
         for (int hx = 0; hx < 2; ++hx) {
-          if (!mbar_wait(&bar_q_empty[hx], qph, abort_flag)) { ok = false; break; }
+          if (!t2_wait(&bar_q_empty[hx], qph, abort_flag)) { ok = false; break; }
           if (hx == 1 && !b_rows) { mbar_arrive(&bar_q_full[1]); continue; }
           mbar_expect_tx(&bar_q_full[hx], kT2Tile);
           tma_load_3d(sQ + hx * kT2Tile, &map_q, &bar_q_full[hx], 0, h * G, q_row + hx * QT);
@@ -451,7 +471,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         };
         auto load_k = [&](int row0) -> bool {
           const int ks = kt % kRingK;
-          if (!mbar_wait(&bar_k_empty[ks], ((kt / kRingK) & 1) ^ 1, abort_flag)) return false;
+          if (!t2_wait(&bar_k_empty[ks], ((kt / kRingK) & 1) ^ 1, abort_flag)) return false;
           mbar_expect_tx(&bar_k_full[ks], kT2Tile);
           tma_load_3d(sK + ks * kT2Tile, &map_k, &bar_k_full[ks], 0, h, row0);
           tma_load_3d(sK + ks * kT2Tile + kT2Sub, &map_k, &bar_k_full[ks], 64, h, row0);
@@ -460,7 +480,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         };
         auto load_v = [&](int row0) -> bool {
           const int vs = vt % kT2Ring;
-          if (!mbar_wait(&bar_v_empty[vs], ((vt / kT2Ring) & 1) ^ 1, abort_flag)) return false;
+          if (!t2_wait(&bar_v_empty[vs], ((vt / kT2Ring) & 1) ^ 1, abort_flag)) return false;
           mbar_expect_tx(&bar_v_full[vs], kT2Tile);
           tma_load_3d(sV + vs * kT2Tile, &map_v, &bar_v_full[vs], 0, h, row0);
           tma_load_3d(sV + vs * kT2Tile + kT2Sub, &map_v, &bar_v_full[vs], 64, h, row0);
@@ -511,18 +531,18 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       };
       while (ok) {
         const int is = n_item % kT2Items;
-        if (!mbar_wait(&bar_item_full[is], (n_item / kT2Items) & 1, abort_flag)) break;
+        if (!t2_wait(&bar_item_full[is], (n_item / kT2Items) & 1, abort_flag)) break;
         const int seq = s_item[is].seq, nA = s_item[is].n[0], nB = s_item[is].n[1], n = kSplit ? nA + nB : max(nA, nB);
         mbar_arrive(&bar_item_empty[is]);
         if (seq < 0) break;
         const uint32_t qph = n_item & 1;
-        if (!mbar_wait(&bar_q_full[0], qph, abort_flag) || !mbar_wait(&bar_q_full[1], qph, abort_flag)) break;
+        if (!t2_wait(&bar_q_full[0], qph, abort_flag) || !t2_wait(&bar_q_full[1], qph, abort_flag)) break;
         if constexpr (kSplit) {
           // the first S of either half, then PV of step j (half j & 1) and that half's next S; ring places and phases are
           // counted along, the half is a constant of the code: what this thread computes is tensor-core idle time
           auto next_k = [&]() { if (++k_at == kRingK) { k_at = 0; k_ph ^= 1; } };
           for (int j = 0; j < 2 && j < n && ok; ++j) {
-            if (!mbar_wait(&bar_k_full[k_at], k_ph, abort_flag)) { ok = false; break; }
+            if (!t2_wait_hot(&bar_k_full[k_at], k_ph, abort_flag)) { ok = false; break; }
             tc::fence_after_sync();
             issue_s(j, k_at);
             tc::commit(&bar_k_empty[k_at]);
@@ -532,10 +552,10 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
           auto step = [&](auto half, int j) -> bool {
             constexpr int hx = decltype(half)::value;
             const int vslot = vt & 1;
-            if (!mbar_wait(&bar_v_full[vslot], (vt >> 1) & 1, abort_flag)) return false;
-            if (j + 2 < n && !mbar_wait(&bar_k_full[k_at], k_ph, abort_flag)) return false;
-            if (j < 2 && !mbar_wait(&bar_o_free[hx], (no[hx] & 1) ^ 1, abort_flag)) return false;
-            if (!mbar_wait(&bar_p_full[hx], np[hx] & 1, abort_flag)) return false;
+            if (!t2_wait_hot(&bar_v_full[vslot], (vt >> 1) & 1, abort_flag)) return false;
+            if (j + 2 < n && !t2_wait_hot(&bar_k_full[k_at], k_ph, abort_flag)) return false;
+            if (j < 2 && !t2_wait_hot(&bar_o_free[hx], (no[hx] & 1) ^ 1, abort_flag)) return false;
+            if (!t2_wait_hot(&bar_p_full[hx], np[hx] & 1, abort_flag)) return false;
             ++np[hx];
             tc::fence_after_sync();
             issue_pv(hx, vslot, j >= 2);
@@ -562,10 +582,11 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         }
         // first K tile: S for both halves
         if (n > 0) {
-          if (!mbar_wait(&bar_k_full[kt % kT2Ring], (kt / kT2Ring) & 1, abort_flag)) break;
+          if (!t2_wait_hot(&bar_k_full[kt % kT2Ring], (kt / kT2Ring) & 1, abort_flag)) break;
           tc::fence_after_sync();
-          if (nA > 0) issue_s(0, kt % kT2Ring);
-          if (nB > 0) issue_s(1, kt % kT2Ring);
+#pragma unroll 1      // (code size)
+          for (int hx = 0; hx < 2; ++hx)
+            if ((hx ? nB : nA) > 0) issue_s(hx, kt % kT2Ring);
           tc::commit(&bar_k_empty[kt % kT2Ring]);
           ++kt;
         }
@@ -575,18 +596,18 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
           const int vslot = vt % kT2Ring;
           // V_j and the next K tile land long before the softmax is through: their barriers are tested
           // first, so that little but the issue itself stands between a half's P and its MMAs
-          if (!mbar_wait(&bar_v_full[vslot], (vt / kT2Ring) & 1, abort_flag)) { ok = false; break; }
-          if (j + 1 < n && !mbar_wait(&bar_k_full[kt % kT2Ring], (kt / kT2Ring) & 1, abort_flag)) { ok = false; break; }
+          if (!t2_wait_hot(&bar_v_full[vslot], (vt / kT2Ring) & 1, abort_flag)) { ok = false; break; }
+          if (j + 1 < n && !t2_wait_hot(&bar_k_full[kt % kT2Ring], (kt / kT2Ring) & 1, abort_flag)) { ok = false; break; }
           if (j == 0) {
             // the output warpgroup must have taken the previous item's O out of both accumulators
-            if (nA > 0 && !mbar_wait(&bar_o_free[0], (no[0] & 1) ^ 1, abort_flag)) { ok = false; break; }
-            if (nB > 0 && !mbar_wait(&bar_o_free[1], (no[1] & 1) ^ 1, abort_flag)) { ok = false; break; }
+            if (nA > 0 && !t2_wait_hot(&bar_o_free[0], (no[0] & 1) ^ 1, abort_flag)) { ok = false; break; }
+            if (nB > 0 && !t2_wait_hot(&bar_o_free[1], (no[1] & 1) ^ 1, abort_flag)) { ok = false; break; }
           }
           for (int hx = 0; hx < 2 && ok; ++hx) {
             const int nx = hx == 0 ? nA : nB;
             if (j >= nx) continue;
             // O_X += P_X V_j
-            if (!mbar_wait(&bar_p_full[hx], np[hx] & 1, abort_flag)) { ok = false; break; }
+            if (!t2_wait_hot(&bar_p_full[hx], np[hx] & 1, abort_flag)) { ok = false; break; }
             ++np[hx];
             tc::fence_after_sync();
             issue_pv(hx, vslot, j > 0);
@@ -618,7 +639,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
     bool ok = true;
     while (ok) {
       const int is = n_item % kT2Items;
-      if (!mbar_wait(&bar_item_full[is], (n_item / kT2Items) & 1, abort_flag)) break;
+      if (!t2_wait(&bar_item_full[is], (n_item / kT2Items) & 1, abort_flag)) break;
       const int seq = s_item[is].seq, h = s_item[is].h, tq0 = s_item[is].tq0, Lq = s_item[is].Lq, Lk = s_item[is].Lk;
       const int k_begin = s_item[is].k_begin, n = kSplit ? s_item[is].n[0] + s_item[is].n[1] : max(s_item[is].n[0], s_item[is].n[1]);
       __syncwarp();
@@ -634,7 +655,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         const bool mine = j >= j0 && j < j1;
         const int row0 = k_begin + j * kT2Kv, rows = min(min(kT2Kv, Lk - j * kT2Kv), p.st_tokens - row0);
         const int s0 = mine ? t2_store_slots(p, row0, rows, lane) : -1;
-        if (!mbar_wait(&full[slot], (kt / depth) & 1, abort_flag)) { ok = false; break; }
+        if (!t2_wait(&full[slot], (kt / depth) & 1, abort_flag)) { ok = false; break; }
         if (mine) t2_store_tile(p, map, cache, ring + slot * kT2Tile, h, row0, rows, s0, lane);
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[slot]);
@@ -666,7 +687,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
 
     while (ok) {
       const int is = n_item % kT2Items;
-      if (!mbar_wait(&bar_item_full[is], (n_item / kT2Items) & 1, abort_flag)) break;
+      if (!t2_wait(&bar_item_full[is], (n_item / kT2Items) & 1, abort_flag)) break;
       const T2Item it = s_item[is];
       __syncwarp();
       if (lane == 0) mbar_arrive(&bar_item_empty[is]);   // this warp has its copy
@@ -682,7 +703,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       const int first_row_kmax = shift + it.tq0 + row_half * QT;
       float m_used = -INFINITY, l = 0.f;
       for (int j = 0; j < nx; ++j) {
-        if (!mbar_wait(&bar_s_full[hx], ns & 1, abort_flag)) { ok = false; break; }
+        if (!t2_wait_hot(&bar_s_full[hx], ns & 1, abort_flag)) { ok = false; break; }
         ++ns;
         tc::fence_after_sync();
         const int tile = kSplit ? 2 * j + hx : j;        // ... which key tiles this half works on
@@ -697,10 +718,11 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
           const int nvalid = kmax - key0 + 1;           // columns of this row that may be seen
 #pragma unroll
           for (int cch = 0; cch < 4; ++cch) {
-            if (nvalid < (cch + 1) * 32) {              // a chunk that lies wholly below the diagonal costs nothing
+            if (nvalid < (cch + 1) * 32) {
+              const uint32_t keep = nvalid <= cch * 32 ? 0u : (1u << (nvalid - cch * 32)) - 1;              // a chunk that lies wholly below the diagonal costs nothing
 #pragma unroll
               for (int i = 0; i < 32; ++i)
-                if (cch * 32 + i >= nvalid) sv[cch][i] = 0xff800000u;   // -inf
+                if (!((keep >> i) & 1)) sv[cch][i] = 0xff800000u;   // -inf
             }
           }
         }
@@ -730,7 +752,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
           if (__any_sync(0xffffffffu, grow)) {
             const float alpha = grow ? fast_exp2((m_used - m_new) * c) : 1.f;
             if (grow) { m_used = m_new; l *= alpha; }
-#pragma unroll
+#pragma unroll 1          // (code size: t2_wait)
             for (int cch = 0; cch < 8; ++cch) {
               uint32_t v[16];
               tc::ld_32x32b_x16(tmem_o + lane_base + cch * 16, v);
@@ -781,7 +803,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
           // ragged last tile of the sequence: V rows past its end are foreign data; zero them so
           // that 0 * garbage cannot turn into NaN inside the tensor core
           const int vt = vt_base + tile;
-          if (!mbar_wait(&bar_v_full[vt % kT2Ring], (vt / kT2Ring) & 1, abort_flag)) { ok = false; break; }
+          if (!t2_wait_hot(&bar_v_full[vt % kT2Ring], (vt / kT2Ring) & 1, abort_flag)) { ok = false; break; }
           // (Rows are 128 bytes and follow each other, so they are zeroed as one range, thread after thread: a row per
           // thread hits the same banks with every lane and took 2000 cycles.)
           unsigned char* vrow = sV + (vt % kT2Ring) * kT2Tile;
@@ -800,7 +822,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       vt_base += n_all;
       if (nx > 0) {
         // the row's 1 / sum goes to the output warpgroup, which drains O while this one moves on
-        if (!mbar_wait(&bar_l_empty[hx], (n_fin & 1) ^ 1, abort_flag)) { ok = false; break; }
+        if (!t2_wait(&bar_l_empty[hx], (n_fin & 1) ^ 1, abort_flag)) { ok = false; break; }
         if constexpr (kSplit) s_max[hx][r] = m_used == -INFINITY ? -INFINITY : m_used * c;
         s_inv[hx][r] = kSplit ? l : l > 0.f ? 1.f / l : 0.f;
         __syncwarp();
@@ -824,7 +846,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
     bool ok = true;
     while (ok) {
       const int is = n_item % kT2Items;
-      if (!mbar_wait(&bar_item_full[is], (n_item / kT2Items) & 1, abort_flag)) break;
+      if (!t2_wait(&bar_item_full[is], (n_item / kT2Items) & 1, abort_flag)) break;
       const int seq = s_item[is].seq, h = s_item[is].h, q_row = s_item[is].q_row, tq0 = s_item[is].tq0, Lq = s_item[is].Lq;
       const int nA = s_item[is].n[0], nB = s_item[is].n[1];
       __syncwarp();
@@ -838,12 +860,12 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
 #pragma unroll
         for (int hx = 0; hx < 2; ++hx) {
           if (hx == 1 && !has_b) continue;
-          if (!mbar_wait(&bar_l_full[hx], nf[hx] & 1, abort_flag)) ok = false;
+          if (!t2_wait(&bar_l_full[hx], nf[hx] & 1, abort_flag)) ok = false;
           m[hx] = s_max[hx][r];
           l[hx] = s_inv[hx][r];
           __syncwarp();
           if (lane == 0) mbar_arrive(&bar_l_empty[hx]);
-          if (!mbar_wait(&bar_o_final[hx], nf[hx] & 1, abort_flag)) ok = false;
+          if (!t2_wait(&bar_o_final[hx], nf[hx] & 1, abort_flag)) ok = false;
           ++nf[hx];
         }
         if (!ok) break;
@@ -864,11 +886,11 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       for (int hx = 0; hx < 2; ++hx) {
         if ((hx == 0 ? nA : nB) <= 0) continue;
         const uint32_t ph = nf[hx] & 1;
-        if (!mbar_wait(&bar_l_full[hx], ph, abort_flag)) { ok = false; break; }
+        if (!t2_wait(&bar_l_full[hx], ph, abort_flag)) { ok = false; break; }
         const float inv = s_inv[hx][r];
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar_l_empty[hx]);
-        if (!mbar_wait(&bar_o_final[hx], ph, abort_flag)) { ok = false; break; }
+        if (!t2_wait(&bar_o_final[hx], ph, abort_flag)) { ok = false; break; }
         tc::fence_after_sync();
         const int tok_w = tq0 + hx * QT + (quarter * 32) / G;        // first token of this warp's rows
         if (p.out_tma && tok_w + 32 / G <= Lq) {
