@@ -105,22 +105,25 @@ __device__ __forceinline__ int ld_acquire_gpu(const int* ptr) {
   return v;
 }
 
-// Merges into r (query head gq) the partials of n of the pair's parts; `mine` >= 0: all but that slot's (the caller holds
-// it).  Eight partials a trip: their maxima and sums travel together with their rows.
-__device__ __forceinline__ void dec_merge_partials(const DecodeParams& p, int part0, int n, int mine, int gq, int lane, DecPart& r) {
+// Merges the n partials of a pair (query head gq) into r.  `own` >= 0: that part is not in the workspace but in r.  Eight
+// partials a trip, their maxima and sums together with their rows, always in the order of the parts: whichever CTA
+// merges, and from where, depends on timing, so the sums must not.
+__device__ __forceinline__ void dec_merge_partials(const DecodeParams& p, int part0, int n, int own, int gq, int lane, DecPart& r) {
+  const DecPart mine = r;
+  r = dec_nothing();
 #pragma unroll 1
   for (int first = 0; first < n; first += 8) {
     // lane j (mod 8) looks after partial first + j
     const int j = first + (lane & 7);
-    int slot = part0 + (j < n ? j : n - 1) * p.Hkv;
-    if (mine >= 0 && slot >= mine) slot += p.Hkv;
-    const int row = slot * p.G + gq;
-    float2 ml = __ldcg(reinterpret_cast<const float2*>(p.ws_ml + row * 2));
+    const int row = (part0 + (j < n ? j : n - 1) * p.Hkv) * p.G + gq;
+    float2 ml = make_float2(mine.M, mine.L);
+    if (j != own) ml = __ldcg(reinterpret_cast<const float2*>(p.ws_ml + row * 2));
     float4 v[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const int ru = __shfl_sync(0xffffffffu, row, u);
-      if (first + u < n) v[u] = __ldcg(reinterpret_cast<const float4*>(p.ws_o + static_cast<long long>(ru) * 128 + lane * 4));
+      v[u] = mine.v;
+      if (first + u < n && first + u != own) v[u] = __ldcg(reinterpret_cast<const float4*>(p.ws_o + static_cast<long long>(ru) * 128 + lane * 4));
     }
     if (j >= n) ml = make_float2(-INFINITY, 0.f);
     float M = ml.x;
@@ -128,18 +131,19 @@ __device__ __forceinline__ void dec_merge_partials(const DecodeParams& p, int pa
     for (int off = 4; off > 0; off >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, off));
     M = fmaxf(M, r.M);
     const float w = fast_exp2(ml.x - M), w0 = fast_exp2(r.M - M);
-    float L = ml.y * w;
+    float L = __fmul_rn(ml.y, w);
 #pragma unroll
     for (int off = 4; off > 0; off >>= 1) L += __shfl_xor_sync(0xffffffffu, L, off);
     r.M = M;
-    r.L = r.L * w0 + L;
-    r.v.x *= w0; r.v.y *= w0; r.v.z *= w0; r.v.w *= w0;
+    // (written out: the function is expanded in three places, which must not contract products and sums differently)
+    r.L = fmaf(r.L, w0, L);
+    r.v.x = __fmul_rn(r.v.x, w0); r.v.y = __fmul_rn(r.v.y, w0); r.v.z = __fmul_rn(r.v.z, w0); r.v.w = __fmul_rn(r.v.w, w0);
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const float wu = __shfl_sync(0xffffffffu, w, u);
       if (first + u < n) {
-        r.v.x += v[u].x * wu; r.v.y += v[u].y * wu;
-        r.v.z += v[u].z * wu; r.v.w += v[u].w * wu;
+        r.v.x = fmaf(v[u].x, wu, r.v.x); r.v.y = fmaf(v[u].y, wu, r.v.y);
+        r.v.z = fmaf(v[u].z, wu, r.v.z); r.v.w = fmaf(v[u].w, wu, r.v.w);
       }
     }
   }
@@ -716,7 +720,7 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
         if (decision == 2) {
           dec_store_partial(p, d.slot, gq, lane, r);
         } else {
-          if (decision == 1) dec_merge_partials(p, d.part0, d.parts - 1, d.slot, gq, lane, r);
+          if (decision == 1) dec_merge_partials(p, d.part0, d.parts, (d.slot - d.part0) / Hkv, gq, lane, r);
           dec_store_row(out_row + gq * 128, r, lane);
         }
       }

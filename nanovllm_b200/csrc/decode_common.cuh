@@ -184,7 +184,8 @@ __device__ __forceinline__ void dec_hand_off(DecAcc& a, float* mo, float* ml, in
   }
 }
 
-// The consumer warps' states of query head gq combined; lane owns dims [4 * lane, 4 * lane + 4).
+// The consumer warps' states of query head gq combined; lane owns dims [4 * lane, 4 * lane + 4).  (The sums are written
+// out as fused operations: every place this is expanded in must give the same bits.)
 struct DecPart {
   float M, L;
   float4 v;
@@ -200,9 +201,9 @@ __device__ __forceinline__ DecPart dec_combine_warps(const float* mo, const floa
 #pragma unroll
   for (int w = 0; w < WARPS; ++w) {
     const float wgt = fast_exp2(ml[(w * G + gq) * 2] - r.M);
-    r.L += ml[(w * G + gq) * 2 + 1] * wgt;
+    r.L = fmaf(ml[(w * G + gq) * 2 + 1], wgt, r.L);
     const float4 v = *reinterpret_cast<const float4*>(mo + (w * G + gq) * 128 + lane * 4);
-    r.v.x += v.x * wgt; r.v.y += v.y * wgt; r.v.z += v.z * wgt; r.v.w += v.w * wgt;
+    r.v.x = fmaf(v.x, wgt, r.v.x); r.v.y = fmaf(v.y, wgt, r.v.y); r.v.z = fmaf(v.z, wgt, r.v.z); r.v.w = fmaf(v.w, wgt, r.v.w);
   }
   return r;
 }

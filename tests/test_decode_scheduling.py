@@ -91,3 +91,23 @@ def test_layer_decode_with_store(slots, n, h, hkv):
     torch.testing.assert_close(out.float().cpu(), want.float(), atol=2e-2, rtol=1e-2)
     assert torch.equal(att.k_cache.cpu().view(torch.int16), kc.view(torch.int16))
     assert torch.equal(att.v_cache.cpu().view(torch.int16), vc.view(torch.int16))
+
+
+@pytest.mark.parametrize("kind,n,h,hkv", [("one long", 40, 64, 8), ("spread", 256, 2, 1), ("spread", 20, 16, 4), ("spread", 60, 16, 2),
+                                          ("9000", 6, 32, 4), ("one long", 300, 16, 1)])
+def test_cut_pairs_repeat_bit_for_bit(kind, n, h, hkv):
+    """Which CTA brings a pair's last part depends on timing; the order in which its parts are summed must not."""
+    import nanovllm_b200
+    lens = _lens(kind, n)
+    g = torch.Generator().manual_seed(n + 3 * h)
+    bt, nb = make_block_tables(lens, 256, g)
+    gd = torch.Generator(device=DEV).manual_seed(n)
+    kc, vc = (torch.randn(nb, 256, hkv, 128, device=DEV, generator=gd).to(torch.bfloat16) for _ in range(2))
+    q = torch.randn(n, h, 128, device=DEV, generator=gd).to(torch.bfloat16)
+    cl, bt = torch.tensor(lens, dtype=torch.int32, device=DEV), bt.to(DEV)
+    scratch = torch.empty(1 << 28, dtype=torch.uint8, device=DEV)
+    first = nanovllm_b200.decode_attention(q, kc, vc, cl, bt, default_scale(128), hkv)
+    for i in range(60):
+        scratch[:(i % 5) << 25].fill_(i)                      # another state of L2 every time, so other CTAs are late
+        out = nanovllm_b200.decode_attention(q, kc, vc, cl, bt, default_scale(128), hkv)
+        assert torch.equal(out.view(torch.int16), first.view(torch.int16)), f"run {i}"
