@@ -241,6 +241,11 @@ int b200_device_status(void);
  * involved.  The next b200_device_status() must report B200_ERR_TIMEOUT and repair the state. */
 int b200_test_inject_timeout(void);
 
+/* Test hook, never called by the product: one thread waits on a barrier that nobody arrives on until the wait gives
+ * up, once with each of the library's two kinds of timed wait (common; tcgen05 prefill), about a second each.  Fills
+ * seconds[2] (host memory) with what they took, -1 where a wait did not report that it gave up. */
+int b200_test_wait_limits(float* seconds);
+
 #ifdef __cplusplus
 }
 #endif

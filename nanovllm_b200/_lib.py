@@ -53,6 +53,7 @@ SIGNATURES = {
     "b200_launch_count": (c_int64, []),
     "b200_device_status": (c_int32, []),
     "b200_test_inject_timeout": (c_int32, []),
+    "b200_test_wait_limits": (c_int32, [c_void_p]),
 }
 
 

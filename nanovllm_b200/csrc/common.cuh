@@ -65,8 +65,9 @@ inline cudaError_t launch_early(void (*kernel)(Params...), unsigned grid, unsign
 }
 
 // ---------------------------------------------------------------------------------------------
-// Bounded waiting.  Every spin in this library gives up after kSpinLimitCycles (about a second)
-// and reports through a status word instead of hanging the GPU.
+// Bounded waiting.  Every spin in this library gives up after kSpinLimitCycles (about a second; the all-reduce takes
+// its limit from the caller) and reports through a status word instead of hanging the GPU.  In the tcgen05 prefill
+// kernel one role keeps that time for all of them (t2_wait).
 // ---------------------------------------------------------------------------------------------
 constexpr long long kSpinLimitCycles = 2000000000LL;
 

@@ -144,4 +144,9 @@ int b200_test_inject_timeout(void) {
   return b200::inject_timeout_prefill_tc2();
 }
 
+int b200_test_wait_limits(float* seconds) {
+  if (!seconds) return b200::set_error(b200::kErrNullPointer, "test_wait_limits: null pointer");
+  return b200::test_wait_limits(seconds);
+}
+
 }  // extern "C"

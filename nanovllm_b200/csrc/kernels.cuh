@@ -57,5 +57,6 @@ int reset_state_decode_cluster();
 int reset_state_prefill_mma();
 int reset_state_prefill_tc2();
 int inject_timeout_prefill_tc2();   // test hook: leaves the unit as an abandoned launch would
+int test_wait_limits(float* seconds);   // test hook: what the bounded waits (mbar_wait, t2_wait_timed) take to give up
 
 }  // namespace b200

@@ -46,10 +46,14 @@ static __device__ int g_status_prefill_tc2 = 0;
 static __device__ unsigned int g_prefill_ticket = 0;
 
 // The kernel's bounded waits.  Six roles run through their loops at the same time and share the SM's instruction cache, so code
-// size is time here: with these in place of mbar_wait() (a clock read, its 64-bit comparison and a spin counter at each of
+// size is time here: with these in place of mbar_wait() (64-bit clock arithmetic and a spin counter at each of
 // some thirty places), the output and rescaling loops rolled and the mask taken from bits, 256 prompts of 100 .. 1024 tokens with
-// the store went from 805 to 700 us, 256 of 10 .. 300 without it from 162 to 142.  A failed test comes back after the hardware's own
-// suspension, at the least some 50 ns, so the limit is 0.2 s or more.
+// the store went from 805 to 700 us, 256 of 10 .. 300 without it from 162 to 142.
+//
+// How long the hardware suspends a failed test is its own affair, so a count of tests is a limit but not one in time.  The time
+// limit is the producer's, on the low word of the clock: it sets the abort flag, which every other wait looks at after a
+// failed test.  That bounds them all: whatever hangs stops the ring that the producer waits for, and at the end the producer
+// waits until every role has taken the end marker, which it does when it is through with all items.
 constexpr int kT2WaitLimit = 1 << 22;
 __device__ __forceinline__ bool t2_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
 #pragma unroll 1
@@ -59,6 +63,23 @@ __device__ __forceinline__ bool t2_wait(uint64_t* bar, uint32_t parity, volatile
   }
   *abort_flag = 1;
   return false;
+}
+__device__ __forceinline__ uint32_t t2_clock() {
+  uint32_t c;
+  asm volatile("mov.u32 %0, %%clock;" : "=r"(c));
+  return c;
+}
+__device__ __forceinline__ bool t2_wait_timed(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  const uint32_t t0 = t2_clock();
+#pragma unroll 1
+  while (!mbar_try_wait(bar, parity)) {
+    if (*abort_flag) return false;
+    if (t2_clock() - t0 > static_cast<uint32_t>(kSpinLimitCycles)) {
+      *abort_flag = 1;
+      return false;
+    }
+  }
+  return true;
 }
 // On the S -> softmax -> PV chain: the second test does not come behind a look at the flag (long sequences lose 3 % to it).
 __device__ __forceinline__ bool t2_wait_hot(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
@@ -402,7 +423,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         if (tk == n_items + gridDim.x - 1) atomicExch(&g_prefill_ticket, 0u);
         // the descriptor is built in its ring slot; only what the loads need stays in registers
         const int is = n_pub % kT2Items;
-        if (!t2_wait(&bar_item_empty[is], ((n_pub / kT2Items) & 1) ^ 1, abort_flag)) { ok = false; break; }
+        if (!t2_wait_timed(&bar_item_empty[is], ((n_pub / kT2Items) & 1) ^ 1, abort_flag)) { ok = false; break; }
         int seq = -1, h = 0, q_row = 0, k_begin = 0, n = 0;
         bool b_rows = false;                                            // half B holds query rows
         if (tk < n_items) {
@@ -440,7 +461,10 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         }
         s_item[is].seq = seq;
         mbar_arrive(&bar_item_full[is]);                                // an item, or the end marker
-        if (seq < 0) break;
+        if (seq < 0) {
+          t2_wait_timed(&bar_item_empty[is], (n_pub / kT2Items) & 1, abort_flag);     // every role has taken it
+          break;
+        }
         // The Q tiles can only be loaded once the previous item has let go of the buffers, which is when
         // they are needed: start them on their way into L2 now, with the item's first K/V tile.
         tma_prefetch_l2_3d(&map_q, 0, h * G, q_row);
@@ -452,7 +476,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         // Q tiles (the buffers are free once every S MMA of the previous item has completed)
         const uint32_t qph = (n_pub & 1) ^ 1;
         for (int hx = 0; hx < 2; ++hx) {
-          if (!t2_wait(&bar_q_empty[hx], qph, abort_flag)) { ok = false; break; }
+          if (!t2_wait_timed(&bar_q_empty[hx], qph, abort_flag)) { ok = false; break; }
           if (hx == 1 && !b_rows) { mbar_arrive(&bar_q_full[1]); continue; }
           mbar_expect_tx(&bar_q_full[hx], kT2Tile);
           tma_load_3d(sQ + hx * kT2Tile, &map_q, &bar_q_full[hx], 0, h * G, q_row + hx * QT);
@@ -471,7 +495,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         };
         auto load_k = [&](int row0) -> bool {
           const int ks = kt % kRingK;
-          if (!t2_wait(&bar_k_empty[ks], ((kt / kRingK) & 1) ^ 1, abort_flag)) return false;
+          if (!t2_wait_timed(&bar_k_empty[ks], ((kt / kRingK) & 1) ^ 1, abort_flag)) return false;
           mbar_expect_tx(&bar_k_full[ks], kT2Tile);
           tma_load_3d(sK + ks * kT2Tile, &map_k, &bar_k_full[ks], 0, h, row0);
           tma_load_3d(sK + ks * kT2Tile + kT2Sub, &map_k, &bar_k_full[ks], 64, h, row0);
@@ -480,7 +504,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         };
         auto load_v = [&](int row0) -> bool {
           const int vs = vt % kT2Ring;
-          if (!t2_wait(&bar_v_empty[vs], ((vt / kT2Ring) & 1) ^ 1, abort_flag)) return false;
+          if (!t2_wait_timed(&bar_v_empty[vs], ((vt / kT2Ring) & 1) ^ 1, abort_flag)) return false;
           mbar_expect_tx(&bar_v_full[vs], kT2Tile);
           tma_load_3d(sV + vs * kT2Tile, &map_v, &bar_v_full[vs], 0, h, row0);
           tma_load_3d(sV + vs * kT2Tile + kT2Sub, &map_v, &bar_v_full[vs], 64, h, row0);
@@ -941,6 +965,30 @@ int inject_timeout_prefill_tc2() {
   int rc = check_cuda(cudaMemcpyToSymbol(g_status_prefill_tc2, &one, sizeof(int)), "inject_timeout: status word");
   if (rc) return rc;
   return check_cuda(cudaMemcpyToSymbol(g_prefill_ticket, &stale, sizeof(unsigned int)), "inject_timeout: ticket counter");
+}
+
+// Test hook: one thread waits on a barrier that nobody arrives on, with either of the library's waits.
+static __device__ float g_wait_seconds[2];
+static __global__ void wait_limit_kernel() {
+  __shared__ __align__(8) uint64_t bar;
+  __shared__ int s_abort;
+  mbar_init(&bar, 1);
+  mbar_fence_init();
+#pragma unroll 1
+  for (int i = 0; i < 2; ++i) {
+    s_abort = 0;
+    unsigned long long t0, t1;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0)::"memory");
+    const bool arrived = i == 0 ? mbar_wait(&bar, 0, &s_abort) : t2_wait_timed(&bar, 0, &s_abort);
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1)::"memory");
+    g_wait_seconds[i] = !arrived && *const_cast<volatile int*>(&s_abort) ? static_cast<float>(t1 - t0) * 1e-9f : -1.f;
+  }
+}
+int test_wait_limits(float* seconds) {
+  wait_limit_kernel<<<1, 1>>>();
+  int rc = check_cuda(cudaGetLastError(), "test_wait_limits launch");
+  if (rc) return rc;
+  return check_cuda(cudaMemcpyFromSymbol(seconds, g_wait_seconds, sizeof(g_wait_seconds)), "test_wait_limits");
 }
 
 // Needs whole query heads groups in a 128-row tile.  The query-block slots are laid out for 2 * QT tokens, or QT with `split`.

@@ -594,3 +594,14 @@ def test_device_status_recovers_after_an_abandoned_launch(b200):
     torch.cuda.synchronize()
     _close(out, want)                              # a stale ticket counter would have left rows unwritten
     _status_ok()
+
+
+def test_bounded_waits_give_up_after_about_a_second(b200):
+    """Both kinds of wait are bounded in time, from below (2e9 cycles at the 1.965 GHz the clock can reach) and from
+    above (the same at 1 GHz, with as much again for the last suspended test)."""
+    import ctypes
+    seconds = (ctypes.c_float * 2)()
+    from nanovllm_b200 import _lib
+    _lib.check(_lib.load().b200_test_wait_limits(ctypes.cast(seconds, ctypes.c_void_p)))
+    assert all(1.0 < t < 4.0 for t in seconds), list(seconds)
+    _status_ok()
