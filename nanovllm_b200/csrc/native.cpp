@@ -435,9 +435,10 @@ PyObject* py_pack_decode(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   const Tensor* rec = tensor_of(a[1], "record");
   int max_batch, max_blocks, block_size;
   if (!rec || !as_int(a[2], &max_batch) || !as_int(a[3], &max_blocks) || !as_int(a[4], &block_size)) return nullptr;
-  Ref seqs(PySequence_Fast(a[0], "pack() takes a sequence of sequences"));
+  // A tuple of our own: the calls below run Python code, during which another thread may change the caller's list.
+  Ref seqs(PySequence_Tuple(a[0]));
   if (!seqs.o) return nullptr;
-  const Py_ssize_t bs = PySequence_Fast_GET_SIZE(seqs.o);
+  const Py_ssize_t bs = PyTuple_GET_SIZE(seqs.o);
   if (bs > max_batch) {
     PyErr_Format(PyExc_ValueError, "decode batch %zd exceeds the stager's capacity %d", bs, max_batch);
     return nullptr;
@@ -455,7 +456,7 @@ PyObject* py_pack_decode(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   int32_t *const slot = base + 4 * bs, *const len = slot + bs, *const tables = len + bs;
   Py_ssize_t width = 0;
   for (Py_ssize_t i = 0; i < bs; ++i) {
-    PyObject* s = PySequence_Fast_GET_ITEM(seqs.o, i);
+    PyObject* s = PyTuple_GET_ITEM(seqs.o, i);
     Ref table(PyObject_GetAttr(s, s_block_table)), last(PyObject_GetAttr(s, s_last_token));
     if (!table.o || !last.o) return nullptr;
     const Py_ssize_t n = PyObject_Size(s);
@@ -474,7 +475,15 @@ PyObject* py_pack_decode(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       return nullptr;
     }
     for (Py_ssize_t j = 0; j < nb; ++j) {
-      const long id = PyLong_AsLong(PySequence_Fast_GET_ITEM(blocks.o, j));
+      // An id that is no int is asked for its value, which may run Python code: held meanwhile, and the table looked at again.
+      if (j >= PySequence_Fast_GET_SIZE(blocks.o)) {
+        PyErr_SetString(PyExc_RuntimeError, "a block table was shortened while it was read");
+        return nullptr;
+      }
+      PyObject* item = PySequence_Fast_GET_ITEM(blocks.o, j);
+      Py_INCREF(item);
+      const long id = PyLong_AsLong(item);
+      Py_DECREF(item);
       if (id == -1 && PyErr_Occurred()) return nullptr;
       if (id != static_cast<int32_t>(id)) {
         PyErr_SetString(PyExc_OverflowError, "block id does not fit 32 bits");

@@ -8,6 +8,7 @@ captured decode-attention graph replayed after it gives the oracle's attention o
 """
 import os
 import random
+import subprocess
 import sys
 from types import SimpleNamespace
 
@@ -75,6 +76,56 @@ def test_packed_record_equals_prepare_decode(bs):
         stager.pack(_fake_batch(rng, 513))
     with pytest.raises(ValueError):
         stager.pack([FakeSeq(5000, list(range(20)), 1)])
+
+
+_CHANGED_MEANWHILE = """
+import sys
+sys.path[:0] = [%r, %r]
+from test_decode_metadata import FakeSeq, prepare_decode_ref
+from nanovllm_b200.engine.decode_metadata import DecodeMetadataStager
+import numpy as np, torch
+
+class Id:                                             # an id that runs Python code when asked for its value
+    def __init__(self, value, then): self.value, self.then = value, then
+    def __index__(self): self.then(); return self.value
+
+class Meddler(FakeSeq):
+    def __len__(self):                                # what another thread may do while this one is in here
+        self.then()
+        return self.num_tokens
+
+st = DecodeMetadataStager(64, 16, 256)
+what = sys.argv[1]
+seqs = [FakeSeq(300 + i, [2 * i, 2 * i + 1], i) for i in range(40)]
+if what == "list":
+    want = prepare_decode_ref(list(seqs), 256)
+    m = Meddler(300, [0, 1], 0)
+    m.then = lambda: seqs.__delitem__(slice(1, None))
+    seqs[0] = m
+    got = st.record_views(st.pack(seqs))
+    assert all(torch.equal(torch.from_numpy(np.ascontiguousarray(g)), w) for g, w in zip(got, want))
+else:
+    table = [0, 1]
+    table[0] = Id(0, table.clear)
+    seqs[3] = FakeSeq(300, table, 1)
+    try:
+        st.pack(seqs)
+    except RuntimeError:
+        pass
+    else:
+        raise SystemExit("a table that was emptied while it was read went through")
+print("fine")
+"""
+
+
+@pytest.mark.parametrize("what", ["list", "table"])
+def test_pack_while_the_schedulers_objects_change(what):
+    """`len(seq)` runs Python code, in which another thread may come to its turn: the record is that of the sequences the
+    call was given, or the call raises; freed objects are never read (in a child process, which that would end)."""
+    code = _CHANGED_MEANWHILE % (ROOT, os.path.join(ROOT, "tests"))
+    res = subprocess.run([sys.executable, "-c", code, what], capture_output=True, text=True, timeout=300,
+                         env=dict(os.environ, PYTHONPATH=os.path.join(ROOT, "tests", "golden"), PYTHONMALLOC="debug"))
+    assert res.returncode == 0 and res.stdout.endswith("fine\n"), res.stdout + res.stderr
 
 
 @pytest.mark.skipif(not os.path.isdir(os.path.join(REF, "nanovllm")), reason="reference install (baseline/_ref) not present")
