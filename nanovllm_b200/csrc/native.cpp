@@ -447,7 +447,9 @@ PyObject* py_pack_decode(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
               rec->numel() >= static_cast<int64_t>(max_batch) * (6 + static_cast<int64_t>(max_blocks)), "record too small");
   // First sweep: the scheduler's Python objects into C++ (the block tables as flat ids), because where the tables lie
   // in the record depends on the longest one.
-  static thread_local std::vector<int32_t> flat, count;
+  // (The vectors' memory is kept between calls; a call that comes in through one of the objects' own methods finds none.)
+  static thread_local std::vector<int32_t> kept_flat, kept_count;
+  std::vector<int32_t> flat(std::move(kept_flat)), count(std::move(kept_count));
   flat.clear();
   count.clear();
   int32_t* const base = static_cast<int32_t*>(rec->data_ptr());
@@ -508,6 +510,8 @@ PyObject* py_pack_decode(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     std::fill(row + nb, row + width, -1);
     src += nb;
   }
+  kept_flat = std::move(flat);
+  kept_count = std::move(count);
   return Py_BuildValue("nn", bs, width);
   END_HANDLE_TH_ERRORS
 }

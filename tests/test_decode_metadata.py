@@ -104,7 +104,7 @@ if what == "list":
     seqs[0] = m
     got = st.record_views(st.pack(seqs))
     assert all(torch.equal(torch.from_numpy(np.ascontiguousarray(g)), w) for g, w in zip(got, want))
-else:
+elif what == "table":
     table = [0, 1]
     table[0] = Id(0, table.clear)
     seqs[3] = FakeSeq(300, table, 1)
@@ -114,11 +114,19 @@ else:
         pass
     else:
         raise SystemExit("a table that was emptied while it was read went through")
+else:                                                 # a pack within a pack
+    want = prepare_decode_ref(list(seqs), 256)
+    other = DecodeMetadataStager(64, 16, 256)
+    m = Meddler(339, [78, 79], 39)
+    m.then = lambda: other.pack([FakeSeq(10, [5], 1)])
+    seqs[39] = m
+    got = st.record_views(st.pack(seqs))
+    assert all(torch.equal(torch.from_numpy(np.ascontiguousarray(g)), w) for g, w in zip(got, want))
 print("fine")
 """
 
 
-@pytest.mark.parametrize("what", ["list", "table"])
+@pytest.mark.parametrize("what", ["list", "table", "nested"])
 def test_pack_while_the_schedulers_objects_change(what):
     """`len(seq)` runs Python code, in which another thread may come to its turn: the record is that of the sequences the
     call was given, or the call raises; freed objects are never read (in a child process, which that would end)."""
