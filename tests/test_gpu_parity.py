@@ -196,7 +196,7 @@ def test_decode_large_batch_eager_path(b200):
 
 
 def test_decode_config2_shape_repeatable(b200):
-    """BASELINE config 2 at full size; oracle on all 256 rows; two runs agree."""
+    """BASELINE config 2 at full size; oracle on all 256 rows; two runs agree bit for bit."""
     pkg, _ = b200
     g = torch.Generator().manual_seed(2)
     lens = torch.randint(100, 2049, (256,), generator=g).tolist()
@@ -206,8 +206,8 @@ def test_decode_config2_shape_repeatable(b200):
     o2 = pkg.decode_attention(qd, kd, vd, cd, bd, default_scale(128), 8)
     torch.cuda.synchronize()
     _close(o1, decode_attn_ref(q, kc, vc, cl, bt, default_scale(128)))
-    # the split points do not depend on timing, but the merge order of partials does not either
-    _close(o1, o2)
+    # no pair of this batch is cut; for cut pairs see test_decode_scheduling.py
+    assert torch.equal(o1.view(torch.int16), o2.view(torch.int16))
     _status_ok()
 
 
@@ -227,8 +227,8 @@ def _oracle_one_paged_decode(q_row, kc, vc, bt_row, n, hkv, d, bs):
 @pytest.mark.parametrize("tp", [1, 2])
 def test_decode_config4_full_size(b200, tp):
     """BASELINE config 4 at full size: Qwen3-8B geometry (32 query / 8 kv heads at TP1, 16 / 4 at TP2), batch 512,
-    lengths U[512, 8192] (9.4 GB of cache at TP1).  Large enough (>= 256 tiles per CTA) for the ticket-scheduled
-    tail pieces.  The cache is built on the GPU; the oracle runs on a sample of sequences whose blocks are
+    lengths U[512, 8192] (9.4 GB of cache at TP1).  Far more units than CTAs, so nearly all are drawn
+    through tickets.  The cache is built on the GPU; the oracle runs on a sample of sequences whose blocks are
     copied back."""
     pkg, _ = b200
     w = workloads.WORKLOADS["decode_cfg4"]
@@ -245,7 +245,8 @@ def test_decode_config4_full_size(b200, tp):
     out2 = pkg.decode_attention(q, kc, vc, lens.to(DEV), bt.to(DEV), default_scale(d), hkv)
     torch.cuda.synchronize()
     assert torch.isfinite(out1.float()).all()
-    _close(out1, out2)                      # piece assignment differs from run to run; results agree
+    # which CTA takes which unit differs from run to run, the results do not
+    assert torch.equal(out1.view(torch.int16), out2.view(torch.int16))
     for i in list(range(0, 512, 31)) + [511]:
         _close(out1[i:i + 1], _oracle_one_paged_decode(q[i:i + 1], kc, vc, bt[i], int(lens[i]), hkv, d, bs))
     del kc, vc
