@@ -19,6 +19,15 @@
  *  - Block tables are int32 (batch, bt_cols) with row stride bt_row_stride; entries at columns
  *    >= ceil(len / block_size) may hold -1 or stale ids (nanovllm/engine/model_runner.py:119-123,
  *    :203) and are never dereferenced.
+ *  - Early starts (programmatic dependent launch).  b200_store_kvcache, b200_qk_norm_rope_store, b200_decode_attn,
+ *    b200_store_decode_attn and b200_prefill_attn / b200_store_prefill_attn start early behind a kernel that lets its
+ *    dependents do so (griddepcontrol.launch_dependents), and read part of their metadata before they wait for it:
+ *      decode                 context_lens, block_tables; b200_store_decode_attn also slot_mapping
+ *      prefill, tcgen05       cu_seqlens_q, cu_seqlens_k
+ *      store, producer, prefill on mma.sync     nothing
+ *    So a kernel that lets its dependents start early must not write these arrays.  Of this library the store,
+ *    producer, decode and mma.sync prefill kernels do (they write cache rows, q, k and outputs only); the metadata unpack,
+ *    all-reduce and tcgen05 prefill kernels do not.  Behind any other kernel or copy there is nothing to observe.
  *  - Return value: 0 on success; negative = arguments rejected before any launch; positive = a
  *    cudaError_t from the launch.  b200_last_error() describes the last failure of the calling
  *    thread.  Nothing throws, aborts or traps.
@@ -75,11 +84,8 @@ int64_t b200_decode_workspace_bytes(int32_t max_batch, int32_t num_heads, int32_
  * h to kv head h / (num_heads / num_kv_heads); softmax(scale * q k^T) v with fp32 softmax and
  * accumulation; out[i] (num_heads x head_dim, contiguous rows of num_heads * head_dim) in bf16.
  * context_lens[i] <= 0 writes zeros and touches no cache.  The launch geometry depends only on
- * (batch, head geometry), never on device data.  The launch may begin while the previous kernel of
- * the stream is still running if that kernel lets it (programmatic dependent launch: of this library
- * b200_store_kvcache, b200_qk_norm_rope_store and b200_decode_attn itself do); it reads context_lens and
- * block_tables before it waits for that kernel, so a kernel that triggers its dependents early must not be
- * the writer of those two arrays. */
+ * (batch, head geometry, bt_cols), never on device data; the same inputs give the same bits on every call.  Early start:
+ * see above. */
 int b200_decode_attn(const void* q, int64_t q_row_stride, const void* k_cache, const void* v_cache,
                      int64_t num_blocks, int32_t block_size, const int32_t* block_tables, int64_t bt_row_stride,
                      int32_t bt_cols, const int32_t* context_lens, void* out, void* workspace,

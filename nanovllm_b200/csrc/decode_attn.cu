@@ -2,8 +2,8 @@
 // nanovllm/layers/attention.py:71-74).
 //
 // HBM-bound: every K and V byte of every context token is read exactly once.  Design:
-//  * Work unit = one (sequence, kv head) pair, whole, or, where a pair is longer than half of a CTA's equal share of
-//    the batch, one of the equal parts it is cut into.  Persistent CTAs (2 per SM) take the units longest first: the
+//  * Work unit = one (sequence, kv head) pair, whole, or, where the batch's longest pair is well above a CTA's equal share
+//    of the tiles (the rule and its lines stand where the units are laid out), one of the equal parts it is cut into.  Persistent CTAs (2 per SM) take the units longest first: the
 //    first ones statically, the others through an atomic ticket, so that CTAs that stream faster take more and the
 //    short units level the end.  Order and cuts are derived on the device from context_lens by every CTA alike: the
 //    launch geometry never depends on device data, as CUDA-graph replay requires.  (Equal static pieces of
@@ -22,7 +22,7 @@
 //    memory and go on with the next tile; the CTA's last unit they finish themselves.
 //  * An epilogue warp combines the four warps' states and writes the bf16 row, or, for a part of a cut pair, a
 //    partial (m, l, unnormalised O) to the workspace; the last part to arrive (one atomic counter per pair, reset by
-//    that warp) merges the partials.  No CTA ever waits for another; every mbarrier wait is bounded.
+//    that warp) merges the partials in the order of the parts.  No CTA ever waits for another; every mbarrier wait is bounded.
 #include "../../include/b200_attn.h"
 #include "decode_common.cuh"
 
@@ -253,10 +253,10 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
   }
 
   // Launched with programmatic stream serialization: the kernel may start while the previous kernel
-  // of the stream is still running, if that kernel allows it (griddepcontrol.launch_dependents; only
-  // this library's store, producer and decode kernels do, any other kernel has completed before this one
-  // starts).  Those kernels write K/V rows of the cache, query rows and outputs, never the metadata, so
-  // the scan over context_lens and the first block-table reads below run ahead;
+  // of the stream is still running, if that kernel allows it (griddepcontrol.launch_dependents; of this library
+  // the store, producer, decode and mma.sync prefill kernels do; any other kernel has completed before this one
+  // starts).  Those kernels write K/V rows of the cache, query and key rows and outputs, never the metadata, so
+  // the scan over context_lens, the first block-table reads and (kStore) the slots below run ahead;
   // every thread that goes on to touch q, the cache, the output or the workspace first executes
   // griddepcontrol.wait (the consumer warps only touch them after data that was loaded behind it).
 
