@@ -48,7 +48,7 @@ constexpr int kDecMinPart = 4;             // tiles: shorter parts would cost mo
 // (16/8 heads) 90.2 -> 87.6 us, 160: 110.6 -> 109.9, 200: 135.3 -> 137.0.
 constexpr int kDecStoreBatch = 160;
 constexpr int kBloomWords = 64, kBloomBits = 11;  // (256 bytes: what static shared memory has left of its 1 KiB)
-constexpr int kDecOneWaveShare = 12;       // tiles per CTA up to which parts get a CTA each
+constexpr int kDecOneWaveShare = 12;       // tiles per CTA up to which parts get a CTA each (measured where it is used)
 constexpr int kPartialSlots = 12;          // of the workspace, per CTA of the grid
 static __device__ int g_status_decode = 0;
 
@@ -320,7 +320,8 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
     // Pairs are cut only if the longest one is well above a CTA's equal share of the tiles: whole pairs, longest first,
     // level out well enough below that and leave nothing to merge.  The line is 1.25 shares, or 1.85 where
     // every CTA has at most one pair (short and long ones share an SM then, and the long one gets the SM's bandwidth when
-    // the short one is done), and 3 tiles, which is what a merge costs (90 sequences of 20 .. 400 tokens, 4 kv heads:
+    // the short one is done: us per layer with the producer, whole | cut, at 1.46 shares 25.7 | 27.2, 1.73 20.3 | 22.4, 1.93
+    // 26.7 | 26.6, with 32 tiles a share 59.0 | 54.0, 2.05 19.4 | 20.5, 2.3 25.2 | 23.2, 2.9 49.3 | 39.1), and 3 tiles, which is what a merge costs (90 sequences of 20 .. 400 tokens, 4 kv heads:
     // 14.6 -> 11.5 us uncut).  Above it, pairs longer than 2/3 of a share (and kDecMinPart tiles) are cut into
     // equal parts: 1/2 and 1/3 leave parts of a size that do not add up to a share, and cost more merges (measured over
     // batches of 16 .. 500 sequences of 1 .. 8192 tokens).  The parts come first in the order, so that their merging
@@ -329,7 +330,9 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
     // With fewer pairs than CTAs and a small share, the parts are instead as short as they can be with a CTA for
     // each, 1 .. 1.5 shares: no CTA starts a second unit, and there are half as many partials.  5 sequences of 47 ..
     // 4381 tokens, 8 kv heads: 21.1 -> 14.2 us; 20 of 500 .. 1500, 4 kv heads: 17.7 -> 13.2; 128 of 30 .. 600, 2 kv heads: 16.3 ->
-    // 12.4.  From kDecOneWaveShare on, levelling through the tickets is as good or better.
+    // 12.4.  From kDecOneWaveShare on, levelling through the tickets is as good or better unless the longest pair is far above
+    // a share (us per layer with the producer, a CTA for each | through tickets: 4.7 tiles a share 14.8 | 17.6, 9.4
+    // 22.4 | 24.2, 11 24.2 | 24.5, 14.7 30.2 | 29.7, 20.7 38.1 | 38.0, 29.5 52.0 | 50.3; 14.9 with the longest at 9 shares 29.5 | 31.9).
     const long long tiles = total * Hkv;
     const int grid = static_cast<int>(gridDim.x);
     const bool one_wave = live * Hkv <= grid;

@@ -295,7 +295,17 @@ static size_t cluster_smem_bytes(int G, int ctas) {
 // pairs and the capacity of a block-table row.  One CTA per SM and clusters of at most 8 (of 16 only a few fit on the chip
 // at a time), so up to 8 CTAs per pair for 18 pairs, 4 for 37, and so on; and a pair's CTAs must be able to bear the
 // longest pair the table allows: beyond kCluMaxTiles each (8 us at the 66 GB/s that one SM draws) the general
-// kernel, which cuts long pairs as it needs, is the faster one.
+// kernel, which cuts long pairs as it needs, is the faster one.  Both sides, us per layer of a decode graph with the producer
+// in front, this kernel | the general one:
+//   a table of 16 columns (4096 tokens), 16/8 heads, taken here: 1 of 562 tokens 6.9 | 9.0, 4 of 562 7.7 | 9.8, 1 of 4000
+//     10.3 | 11.4, 4 of 500 .. 4000 13.2 | 14.5; but 2 .. 4 of which one has 4000 and the others 200: 13.4 | 11.5;
+//   the same table, left to the general kernel: 6 of 562 8.4 | 10.1, 18 of 562 12.2 | 15.3; but 6 with one of 4000
+//     20.7 | 11.9, 12 of 500 .. 4000 33.9 | 24.7;
+//   40 columns, left to the general kernel from 33 on: 1 of 562 7.2 | 9.0, 4 of 562 7.7 | 9.8; but 4 with one of
+//     4000 13.5 | 11.6, and of 160 columns 2 with one of 30000 61.9 | 32.6.
+// So the line on the table's width is what keeps the worst case near the general kernel's, and it costs short sequences
+// under a wide table 20 %.  Of clusters of 4, 33 fit on the chip at a time: 34 .. 37 pairs, which the line below lets in,
+// take two rounds (4/2 heads, 16 sequences of 562 tokens 7.7 | 9.8, 17 of them 12.3 | 9.9).
 constexpr int kCluMaxTiles = 16;
 int decode_cluster_ctas(int batch, int Hkv, int G, int max_tiles) {
   const int sms = sm_count();

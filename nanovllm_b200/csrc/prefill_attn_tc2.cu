@@ -38,7 +38,12 @@ constexpr int kT2Threads = 512;   // warpgroup 0: TMA producer, MMA issuer, two 
 constexpr int kT2Ring = 2;                   // K ring depth and V ring depth
 constexpr int kT2Items = 4;                  // item descriptors in flight
 constexpr int kT2MaxSeqSmem = 1024;          // sequences whose slot table fits in shared memory
-constexpr int kT2MaxSort = kT2Threads / 2;   // sequences that are put in order of length
+// Sequences that are put in order of length: two threads each, so one round of the block.  Larger batches keep their own order.  What
+// that costs, from batches of up to 256 measured both ways (sorted | the order of a shuffled batch): 64 of 100 .. 1024 tokens
+// 34.7 | 41.6 us at 2/1 heads, 158 | 162 at 16/8; 256 of them 644 | 692 and, at 32/8, 1323 | 1319; 256 of 10 .. 120 at 2/1
+// heads 20.7 | 18.3 (the sort itself takes 2.4 us).  With more than 256 prompts in a step an SM has several items of any
+// length anyway.
+constexpr int kT2MaxSort = kT2Threads / 2;
 constexpr float kT2Rescale = 8.0f;
 
 static __device__ int g_status_prefill_tc2 = 0;
