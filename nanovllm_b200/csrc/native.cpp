@@ -477,15 +477,20 @@ PyObject* py_pack_decode(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       return nullptr;
     }
     for (Py_ssize_t j = 0; j < nb; ++j) {
-      // An id that is no int is asked for its value, which may run Python code: held meanwhile, and the table looked at again.
-      if (j >= PySequence_Fast_GET_SIZE(blocks.o)) {
-        PyErr_SetString(PyExc_RuntimeError, "a block table was shortened while it was read");
-        return nullptr;
-      }
       PyObject* item = PySequence_Fast_GET_ITEM(blocks.o, j);
-      Py_INCREF(item);
-      const long id = PyLong_AsLong(item);
-      Py_DECREF(item);
+      long id;
+      if (PyLong_CheckExact(item)) {
+        id = PyLong_AsLong(item);
+      } else {
+        // It is asked for its value, which may run Python code: held meanwhile, and the table looked at again.
+        Py_INCREF(item);
+        id = PyLong_AsLong(item);
+        Py_DECREF(item);
+        if (PySequence_Fast_GET_SIZE(blocks.o) < nb) {
+          if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "a block table was shortened while it was read");
+          return nullptr;
+        }
+      }
       if (id == -1 && PyErr_Occurred()) return nullptr;
       if (id != static_cast<int32_t>(id)) {
         PyErr_SetString(PyExc_OverflowError, "block id does not fit 32 bits");
