@@ -24,8 +24,8 @@ Besides the contract's keys the line carries
   library_baseline  (N = 1) what the reference's own GPU path achieves on the same box in the same run:
                     flash_attn_with_kvcache / flash_attn_varlen_func / the Triton store_kvcache, called with the
                     argument pattern of nanovllm/layers/attention.py:33-74 on the same tensors
-  secondary         prefill TFLOP/s on BASELINE config 3 (dense); `secondaries` adds its prefix-cache form and,
-                    at every N, decode on BASELINE config 4 (Qwen3-8B geometry, per-GPU and aggregate GB/s)
+  secondary         prefill TFLOP/s on 256 dense prompts of 100 .. 1024 tokens; `secondaries` adds its prefix-cache form and,
+                    at every N, decode of 512 sequences of 512 .. 8192 tokens (Qwen3-8B geometry, per-GPU and aggregate GB/s)
 
 `--impl reference` times the reference's algorithm on the host cores (the CPU restatement under
 oracle/, torch with all host threads) on a bounded sample of the same workload.

@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """End-to-end output tokens/s of the nano-vllm engine with either attention layer
-(BASELINE config 5: the workload of the reference's own bench.py).
+(the workload of the reference's own bench.py).
 
     python bench_e2e.py --attn ours|reference [--fuse-producer] [--fast-metadata] [--tp 1] [--num-seqs 256] [--out FILE]
 

@@ -29,7 +29,7 @@ DT = torch.bfloat16
 
 # name -> spec
 CASES = {
-    # BASELINE config 1 geometry (16/8/128, 64 blocks x 256, lens 100/257/513/1024) in bf16
+    # the smallest engine geometry (16/8/128, 64 blocks x 256, lens 100/257/513/1024) in bf16
     "dec_cfg1": dict(kind="decode", H=16, Hkv=8, D=128, NB=64, lens=[100, 257, 513, 1024], seed=101),
     # one KV head per GPU (Qwen3-8B at TP8: 4 q heads on 1 kv head); block-boundary lengths
     "dec_tp8": dict(kind="decode", H=4, Hkv=1, D=128, NB=24, lens=[1, 255, 256, 257, 2048, 700], seed=102),

@@ -196,7 +196,7 @@ def test_decode_large_batch_eager_path(b200):
 
 
 def test_decode_config2_shape_repeatable(b200):
-    """BASELINE config 2 at full size; oracle on all 256 rows; two runs agree bit for bit."""
+    """256 sequences of 100 .. 2048 tokens, 16/8 heads; oracle on all 256 rows; two runs agree bit for bit."""
     pkg, _ = b200
     g = torch.Generator().manual_seed(2)
     lens = torch.randint(100, 2049, (256,), generator=g).tolist()
@@ -226,7 +226,7 @@ def _oracle_one_paged_decode(q_row, kc, vc, bt_row, n, hkv, d, bs):
 
 @pytest.mark.parametrize("tp", [1, 2])
 def test_decode_config4_full_size(b200, tp):
-    """BASELINE config 4 at full size: Qwen3-8B geometry (32 query / 8 kv heads at TP1, 16 / 4 at TP2), batch 512,
+    """Qwen3-8B geometry (32 query / 8 kv heads at TP1, 16 / 4 at TP2), batch 512,
     lengths U[512, 8192] (9.4 GB of cache at TP1).  Far more units than CTAs, so nearly all are drawn
     through tickets.  The cache is built on the GPU; the oracle runs on a sample of sequences whose blocks are
     copied back."""
@@ -391,7 +391,7 @@ def test_prefill_paged_prefix_poisoned(b200, h, hkv, variant):
 
 
 def test_prefill_config3_scale_and_many_sequences(b200):
-    """BASELINE config 3 at full size (256 sequences, U[100,1024]) against the oracle on a sample of
+    """256 prompts of 100 .. 1024 tokens, dense, against the oracle on a sample of
     sequences, and a batch of more than 1024 short sequences (the slot table no longer fits in shared memory)."""
     pkg, _ = b200
     h, hkv, d = 16, 8, 128
@@ -419,7 +419,7 @@ def test_prefill_config3_scale_and_many_sequences(b200):
 
 
 def test_prefill_config3_prefix_half_full_size(b200):
-    """BASELINE config 3 in its prefix-cache form at full size: 256 sequences U[100, 1024], the second half with a
+    """With a prefix cache: 256 sequences U[100, 1024], the second half with a
     cached prefix of a random whole number of blocks, so the whole batch reads K/V from the paged cache
     (nanovllm/engine/model_runner.py:153-154).  Oracle on 32 sequences, half of them with a prefix."""
     pkg, _ = b200
