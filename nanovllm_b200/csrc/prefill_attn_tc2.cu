@@ -53,7 +53,10 @@ static __device__ unsigned int g_prefill_ticket = 0;
 // The kernel's bounded waits.  Six roles run through their loops at the same time and share the SM's instruction cache, so code
 // size is time here: with these in place of mbar_wait() (64-bit clock arithmetic and a spin counter at each of
 // some thirty places), the output and rescaling loops rolled and the mask taken from bits, 256 prompts of 100 .. 1024 tokens with
-// the store went from 805 to 700 us, 256 of 10 .. 300 without it from 162 to 142.
+// the store went from 805 to 700 us, 256 of 10 .. 300 without it from 162 to 142.  (With 78 KB of code in place of 62 a tcgen05 kernel of
+// this kind waited 2.5 times as long for instructions.)  The form with the store was 78 KB and is 64 with one output path instead of two, shifts for
+// divisions by powers of two, table columns counted along and one copy of the row loop: 256 prompts of 100 .. 1024 tokens
+// 838 -> 794 us with the store, 616 -> 602 without it (57 KB for 63), 64 of 10 .. 300 58 -> 54.
 //
 // How long the hardware suspends a failed test is its own affair, so a count of tests is a limit but not one in time.  The time
 // limit is the producer's, on the low word of the clock: it sets the abort flag, which every other wait looks at after a
@@ -101,60 +104,10 @@ struct T2Item {
   int n[2];       // K/V tiles each half needs (n[1] == 0: half B is empty)
 };
 
-// One 16-column chunk of a warp's 32 rows, scaled, to memory through the staging tile.
-__device__ __forceinline__ void t2_plain_chunk(const PrefillParams& p, const uint32_t (&ov)[16], unsigned char* stage, int lane,
-                                               int quarter, int hx, int cch, float inv, int q_row, int h, int tq0, int Lq) {
-  const int G = p.G, QT = p.QT;
-  const int srow = lane >> 1, sq = lane & 1;             // read-back role: 16 rows x 2 chunks per instruction
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    uint4 w;
-    w.x = pack_bf16(__uint_as_float(ov[8 * i]) * inv, __uint_as_float(ov[8 * i + 1]) * inv);
-    w.y = pack_bf16(__uint_as_float(ov[8 * i + 2]) * inv, __uint_as_float(ov[8 * i + 3]) * inv);
-    w.z = pack_bf16(__uint_as_float(ov[8 * i + 4]) * inv, __uint_as_float(ov[8 * i + 5]) * inv);
-    w.w = pack_bf16(__uint_as_float(ov[8 * i + 6]) * inv, __uint_as_float(ov[8 * i + 7]) * inv);
-    *reinterpret_cast<uint4*>(stage + lane * 32 + ((i ^ ((lane >> 2) & 1)) << 4)) = w;
-  }
-  __syncwarp();
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const int lr = 16 * k + srow;                         // row within the warp's 32
-    const uint4 w = *reinterpret_cast<const uint4*>(stage + lr * 32 + ((sq ^ ((lr >> 2) & 1)) << 4));
-    const int rr = quarter * 32 + lr;                     // row of the 128-row tile
-    const int tk = tq0 + hx * QT + rr / G;
-    if (rr < QT * G && tk < Lq)
-      *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(
-          p.out + (static_cast<long long>(q_row + hx * QT + rr / G) * p.H + h * G + rr % G) * 128) +
-          cch * 32 + sq * 16) = w;
-  }
-  __syncwarp();
-}
-
-// Output of one half of an item, run by the output warpgroup: read the finished O row out of TMEM
-// in 32-column chunks, scale by 1 / row sum and store bf16 rows through a per-warp staging tile so
-// that every store instruction writes 64-byte row segments (a thread owns a whole row: stored
-// directly, each instruction would touch 32 different lines with 16 bytes each).  The accumulator
-// is released as soon as its last chunk is in registers.
-__device__ __forceinline__ void t2_output(const PrefillParams& p, uint32_t tmem_o_lane, uint64_t* bar_o_free,
-                                          unsigned char* stage, int lane, int quarter, int hx,
-                                          float inv, int q_row, int h, int tq0, int Lq) {
-#pragma unroll 1
-  for (int cch = 0; cch < 8; ++cch) {
-    uint32_t ov[16];
-    tc::ld_32x32b_x16(tmem_o_lane + cch * 16, ov);
-    tc::wait_ld();
-    if (cch == 7) {
-      tc::fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_o_free);
-    }
-    t2_plain_chunk(p, ov, stage, lane, quarter, hx, cch, inv, q_row, h, tq0, Lq);
-  }
-}
-
-// The same for a warp whose 32 tile rows are all real query rows: the scaled bf16 rows are laid out
-// in shared memory as two 128-byte-swizzled boxes of 64 dims and leave through two TMA stores, so
-// the warp issues no global store and no read-back at all.  `stage` is 4 KiB, 1024-byte aligned.
+// Output of one half of an item, run by the output warpgroup: a finished O row out of TMEM in chunks of 16 columns, scaled by
+// 1 / row sum and as bf16 into staging boxes in shared memory (32 rows x 32 dims, 2 KiB, 64-byte swizzle; two per warp, used in
+// turn).  Where all 32 rows of the warp are query rows the box leaves through a TMA store, with no global store instruction and no
+// read-back; else row by row, from the same box.  The accumulator is released as soon as its last chunk is in registers.
 __device__ __forceinline__ void t2_stage_chunk(const uint32_t (&ov)[16], unsigned char* box, int lane, int c, float inv) {
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
@@ -166,18 +119,40 @@ __device__ __forceinline__ void t2_stage_chunk(const uint32_t (&ov)[16], unsigne
     *reinterpret_cast<uint4*>(box + lane * 64 + (((2 * c + i) ^ ((lane >> 1) & 3)) << 4)) = w;   // 64-byte swizzle
   }
 }
-// `stage` holds two boxes of 32 rows x 32 dims (2 KiB each, 64-byte swizzle) used in turn, so that
-// a box is written while the TMA engine still reads the one before.
-__device__ __forceinline__ void t2_output_tma(const CUtensorMap* map_o, uint32_t tmem_o_lane, uint64_t* bar_o_free,
-                                              unsigned char* stage, int lane, float inv, int head0, int tok0) {
+// Before a box is written again: the store before the previous one has left it (plain stores are done with it already).
+__device__ __forceinline__ void t2_open_box(bool tma, int lane) {
+  if (tma && lane == 0) tma_store_wait_read_but_one();
+  __syncwarp();
+}
+// `row0`: the output row (token * H + head) of the warp's first tile row, `rows`: how many of its 32 are query rows.
+__device__ __forceinline__ void t2_close_box(const PrefillParams& p, const CUtensorMap* map_o, const unsigned char* box, bool tma, int lane, int gs,
+                                             int bx, int head0, int tok0, int rows) {
+  if (tma) {
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) {
+      tma_store_3d(map_o, box, bx * 32, head0, tok0);
+      tma_store_commit();
+    }
+    return;
+  }
+  __syncwarp();
+#pragma unroll 1
+  for (int lr = lane >> 2; lr < rows; lr += 8) {
+    const uint4 w = *reinterpret_cast<const uint4*>(box + lr * 64 + (((lane & 3) ^ ((lr >> 1) & 3)) << 4));
+    reinterpret_cast<uint4*>(p.out + (static_cast<long long>(tok0 + (lr >> gs)) * p.H + head0 + (lr & ((1 << gs) - 1))) * 128)[bx * 4 + (lane & 3)] = w;
+  }
+  __syncwarp();
+}
+__device__ __forceinline__ void t2_output(const PrefillParams& p, const CUtensorMap* map_o, uint32_t tmem_o_lane, uint64_t* bar_o_free,
+                                          unsigned char* stage, int lane, int gs, float inv, bool tma, int head0, int tok0, int rows) {
   // eight 16-column chunks, the TMEM load of the next one in flight while one is converted
   uint32_t a[16], b[16];
   tc::ld_32x32b_x16(tmem_o_lane, a);
 #pragma unroll 1      // (code size: t2_wait)
   for (int bx = 0; bx < 4; ++bx) {
     unsigned char* box = stage + (bx & 1) * 2048;
-    if (lane == 0) tma_store_wait_read_but_one();        // the store before the previous one has left this box
-    __syncwarp();
+    t2_open_box(tma, lane);
     tc::wait_ld();
     tc::ld_32x32b_x16(tmem_o_lane + bx * 32 + 16, b);
     t2_stage_chunk(a, box, lane, 0, inv);
@@ -191,27 +166,19 @@ __device__ __forceinline__ void t2_output_tma(const CUtensorMap* map_o, uint32_t
       tc::ld_32x32b_x16(tmem_o_lane + bx * 32 + 32, a);
     }
     t2_stage_chunk(b, box, lane, 1, inv);
-    fence_proxy_async_smem();
-    __syncwarp();
-    if (lane == 0) {
-      tma_store_3d(map_o, box, bx * 32, head0, tok0);
-      tma_store_commit();
-    }
+    t2_close_box(p, map_o, box, tma, lane, gs, bx, head0, tok0, rows);
   }
 }
 
 // Output of an item whose keys the halves shared: the same rows lie in both accumulators, each relative to its own half's
 // maximum; `wa` and `wb` bring them together (has_b false: there was one tile, half B has nothing).
 __device__ __forceinline__ void t2_output_split(const PrefillParams& p, const CUtensorMap* map_o, uint32_t tmem_a, uint32_t tmem_b,
-                                                bool has_b, uint64_t* bar_o_free, unsigned char* stage, int lane, int quarter,
-                                                float wa, float wb, bool tma, int q_row, int h, int tq0, int Lq) {
+                                                bool has_b, uint64_t* bar_o_free, unsigned char* stage, int lane, int gs,
+                                                float wa, float wb, bool tma, int head0, int tok0, int rows) {
 #pragma unroll 1
   for (int cch = 0; cch < 8; ++cch) {
     unsigned char* box = stage + ((cch >> 1) & 1) * 2048;
-    if (tma && !(cch & 1)) {
-      if (lane == 0) tma_store_wait_read_but_one();
-      __syncwarp();
-    }
+    if (!(cch & 1)) t2_open_box(tma, lane);
     uint32_t a[16], b[16];
     tc::ld_32x32b_x16(tmem_a + cch * 16, a);
     if (has_b) tc::ld_32x32b_x16(tmem_b + cch * 16, b);
@@ -229,19 +196,8 @@ __device__ __forceinline__ void t2_output_split(const PrefillParams& p, const CU
         if (has_b) mbar_arrive(&bar_o_free[1]);
       }
     }
-    if (tma) {
-      t2_stage_chunk(a, box, lane, cch & 1, 1.f);
-      if (cch & 1) {
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          tma_store_3d(map_o, box, (cch >> 1) * 32, h * p.G, q_row + quarter * 32 / p.G);
-          tma_store_commit();
-        }
-      }
-    } else {
-      t2_plain_chunk(p, a, stage, lane, quarter, 0, cch, 1.f, q_row, h, tq0, Lq);
-    }
+    t2_stage_chunk(a, box, lane, cch & 1, 1.f);
+    if (cch & 1) t2_close_box(p, map_o, box, tma, lane, gs, cch >> 1, head0, tok0, rows);
   }
 }
 
@@ -265,6 +221,7 @@ __device__ __forceinline__ void t2_store_tile(const PrefillParams& p, const CUte
                                               int h, int row0, int rows, int s0, int lane) {
   const int boxes = s0 >= 0 ? rows >> 5 : 0;
   if (lane == 0 && boxes > 0) {
+#pragma unroll 1
     for (int b = 0; b < boxes; ++b) {
       tma_store_3d(map, tile + b * 4096, 0, h, s0 + b * 32);
       tma_store_3d(map, tile + kT2Sub + b * 4096, 64, h, s0 + b * 32);
@@ -288,9 +245,11 @@ __device__ __forceinline__ void t2_store_tile(const PrefillParams& p, const CUte
 __device__ __forceinline__ void t2_store_rows(const PrefillParams& p, const char* src, long long stride, char* cache, int row0,
                                               int row1, int lane) {
   const int vecs = p.Hkv * 16;
+#pragma unroll 1
   for (int r = row0; r < row1; ++r) {
     const long long slot = __ldg(p.st_slots + r);
     if (slot < 0 || slot >= p.st_n_slots) continue;
+#pragma unroll 1
     for (int v = lane; v < vecs; v += 32)
       reinterpret_cast<uint4*>(cache)[slot * vecs + v] = __ldg(reinterpret_cast<const uint4*>(src + r * stride) + v);
   }
@@ -359,7 +318,8 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
   __shared__ int s_abort;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int G = p.G, QT = p.QT, QB = (kSplit ? 1 : 2) * p.QT;
+  // (G divides 128: all of these are powers of two)
+  const int G = p.G, gs = __ffs(p.G) - 1, qs_log = (kSplit ? 7 : 8) - gs, QT = 128 >> gs, QB = 1 << qs_log;
   const bool slot_in_smem = p.batch <= kT2MaxSeqSmem;
 
   if (tid == 0) {
@@ -394,7 +354,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (slot_in_smem && !sorted)
     for (int i = tid; i <= p.batch; i += kT2Threads) {
-      s_slot[i] = __ldg(p.cu_q + i) / QB + i;
+      s_slot[i] = (__ldg(p.cu_q + i) >> qs_log) + i;
       if (i < p.batch) s_order[i] = static_cast<unsigned short>(i);
     }
   if (warp == 1) {
@@ -437,10 +397,10 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
           int lo = 0, hi = p.batch;
           while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
-            const int f = slot_in_smem ? s_slot[mid] : __ldg(p.cu_q + mid) / QB + mid;
+            const int f = slot_in_smem ? s_slot[mid] : (__ldg(p.cu_q + mid) >> qs_log) + mid;
             if (f <= x) lo = mid; else hi = mid;
           }
-          const int qb = x - (slot_in_smem ? s_slot[lo] : __ldg(p.cu_q + lo) / QB + lo);
+          const int qb = x - (slot_in_smem ? s_slot[lo] : (__ldg(p.cu_q + lo) >> qs_log) + lo);
           if (slot_in_smem) lo = s_order[lo];
           const int q_begin = __ldg(p.cu_q + lo);
           const int Lq = __ldg(p.cu_q + lo + 1) - q_begin;
@@ -491,12 +451,19 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         ++n_pub;
         // K and V tiles
         const int* bt_row = p.block_tables ? p.block_tables + seq * p.bt_row_stride : nullptr;
-        auto tile_row = [&](int j) -> int {
-          if (!bt_row) return k_begin + j * kT2Kv;
-          const int tok0 = j * kT2Kv;
-          const int col = tok0 / p.block_size;
-          const long long blk = col < p.bt_cols ? bt_row[col] : -1;
-          return (blk >= 0 && blk < p.num_blocks) ? static_cast<int>(blk * p.block_size + (tok0 - col * p.block_size)) : -kT2Kv;
+        // row of the next tile in turn (paged: the next block when one is through; blocks are multiples of 256 keys)
+        int row_at = k_begin, left = bt_row ? 0 : 0x7fffffff, col = 0;
+        auto next_row = [&]() -> int {
+          if (left == 0) {
+            const long long blk = col < p.bt_cols ? bt_row[col] : -1;
+            ++col;
+            left = p.block_size;
+            row_at = blk >= 0 && blk < p.num_blocks ? static_cast<int>(blk * p.block_size) : -(1 << 30);      // (nowhere: zeros)
+          }
+          const int row = row_at;
+          left -= kT2Kv;
+          row_at += kT2Kv;
+          return row;
         };
         auto load_k = [&](int row0) -> bool {
           const int ks = kt % kRingK;
@@ -518,13 +485,21 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         };
         if constexpr (kSplit) {
           // K two tiles ahead of V: the issuer needs K of step j + 2 in step j
+          int row = 0, v0 = 0, v1 = 0;
+#pragma unroll 1
           for (int j = 0; j < n + 2 && ok; ++j) {
-            if (j < n) ok = load_k(tile_row(j));
-            if (ok && j >= 2) ok = load_v(tile_row(j - 2));
+            if (j < n) {
+              row = next_row();
+              ok = load_k(row);
+            }
+            if (ok && j >= 2) ok = load_v(v0);
+            v0 = v1;
+            v1 = row;
           }
         } else {
+#pragma unroll 1
           for (int j = 0; j < n && ok; ++j) {
-            const int row0 = tile_row(j);
+            const int row0 = next_row();
             ok = load_k(row0) && load_v(row0);
           }
         }
@@ -679,6 +654,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       // start together, the sequence's last item, which loads all tiles, stores them all.
       const int j0 = Lq == Lk ? (tq0 + kT2Kv - 1) / kT2Kv : tq0 + QB >= Lq ? 0 : n;
       const int j1 = Lq == Lk ? min(n, (tq0 + QB + kT2Kv - 1) / kT2Kv) : n;
+#pragma unroll 1
       for (int j = 0; j < n; ++j, ++kt) {
         const int slot = kt % depth;
         const bool mine = j >= j0 && j < j1;
@@ -693,11 +669,11 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
     if (ok) {
       const char* src = is_v ? p.st_v : p.st_k;
       const long long stride = is_v ? p.st_v_stride : p.st_k_stride;
-      for (int i = blockIdx.x; i < p.batch; i += gridDim.x)
-        if (__ldg(p.cu_q + i) == __ldg(p.cu_q + i + 1)) t2_store_rows(p, src, stride, cache, __ldg(p.cu_k + i), __ldg(p.cu_k + i + 1), lane);
-      if (blockIdx.x == 0) {
-        t2_store_rows(p, src, stride, cache, 0, __ldg(p.cu_k), lane);
-        t2_store_rows(p, src, stride, cache, __ldg(p.cu_k + p.batch), p.st_tokens, lane);
+      // (segment g: sequence g - 1; 0 and batch + 1: the rows in front of the first and behind the last)
+#pragma unroll 1
+      for (int g = blockIdx.x; g < p.batch + 2; g += gridDim.x) {
+        const int r0 = g == 0 ? 0 : __ldg(p.cu_k + g - 1), r1 = g > p.batch ? p.st_tokens : __ldg(p.cu_k + g);
+        if (g == 0 || g > p.batch || __ldg(p.cu_q + g - 1) == __ldg(p.cu_q + g)) t2_store_rows(p, src, stride, cache, r0, r1, lane);
       }
     }
   }
@@ -726,8 +702,8 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       const int n_all = kSplit ? it.n[0] + it.n[1] : max(it.n[0], it.n[1]);
       const int row_half = kSplit ? 0 : hx;               // which rows and ...
       const int shift = it.Lk - it.Lq;
-      const int tok = it.tq0 + row_half * QT + r / G;
-      const bool row_ok = r < QT * G && tok < it.Lq;
+      const int tok = it.tq0 + row_half * QT + (r >> gs);
+      const bool row_ok = tok < it.Lq;
       const int kmax = row_ok ? shift + tok : -1;          // last visible key (inclusive)
       const int first_row_kmax = shift + it.tq0 + row_half * QT;
       float m_used = -INFINITY, l = 0.f;
@@ -859,7 +835,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         ++n_fin;
       } else if (row_ok && (!kSplit || n_all == 0) && !(kSplit && hx)) {
         // no visible key at all (Lk < Lq rows): zeros, as the reference's attention library does
-        uint4* dst = reinterpret_cast<uint4*>(p.out + (static_cast<long long>(it.q_row + row_half * QT + r / G) * p.H + it.h * G + r % G) * 128);
+        uint4* dst = reinterpret_cast<uint4*>(p.out + (static_cast<long long>(it.q_row + row_half * QT + (r >> gs)) * p.H + it.h * G + (r & (G - 1))) * 128);
 #pragma unroll
         for (int i = 0; i < 16; ++i) dst[i] = make_uint4(0, 0, 0, 0);
       }
@@ -902,13 +878,14 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         const float M = fmaxf(m[0], m[1]);
         float wa = M == -INFINITY ? 0.f : fast_exp2(m[0] - M), wb = M == -INFINITY ? 0.f : fast_exp2(m[1] - M);
         const float sum = l[0] * wa + l[1] * wb, inv = sum > 0.f ? 1.f / sum : 0.f;
-        const bool tma = p.out_tma && tq0 + quarter * 32 / G + 32 / G <= Lq;
+        const int rows = min(32, (min(Lq - tq0, QT) << gs) - quarter * 32);
+        const bool tma = p.out_tma && rows == 32;
         if (!tma) {
           if (lane == 0) tma_store_wait_read();
           __syncwarp();
         }
-        t2_output_split(p, &map_o, tmem + 256 + lane_base, tmem + 384 + lane_base, has_b, bar_o_free, sStage + quarter * 4096, lane,
-                        quarter, wa * inv, wb * inv, tma, q_row, h, tq0, Lq);
+        t2_output_split(p, &map_o, tmem + 256 + lane_base, tmem + 384 + lane_base, has_b, bar_o_free, sStage + quarter * 4096, lane, gs,
+                        wa * inv, wb * inv, tma, h * G + (G > 32 ? (quarter * 32) & (G - 1) : 0), q_row + (quarter * 32 >> gs), rows);
         continue;
       }
 #pragma unroll 1
@@ -921,16 +898,14 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         if (lane == 0) mbar_arrive(&bar_l_empty[hx]);
         if (!t2_wait(&bar_o_final[hx], ph, abort_flag)) { ok = false; break; }
         tc::fence_after_sync();
-        const int tok_w = tq0 + hx * QT + (quarter * 32) / G;        // first token of this warp's rows
-        if (p.out_tma && tok_w + 32 / G <= Lq) {
-          t2_output_tma(&map_o, tmem + 256 + hx * 128 + lane_base, &bar_o_free[hx], sStage + quarter * 4096, lane, inv,
-                        h * G, q_row + hx * QT + (quarter * 32) / G);
-        } else {
+        const int rows = min(32, (min(Lq - tq0 - hx * QT, QT) << gs) - quarter * 32);      // query rows among this warp's
+        const bool tma = p.out_tma && rows == 32;
+        if (!tma) {
           if (lane == 0) tma_store_wait_read();
           __syncwarp();
-          t2_output(p, tmem + 256 + hx * 128 + lane_base, &bar_o_free[hx], sStage + quarter * 4096, lane, quarter, hx,
-                    inv, q_row, h, tq0, Lq);
         }
+        t2_output(p, &map_o, tmem + 256 + hx * 128 + lane_base, &bar_o_free[hx], sStage + quarter * 4096, lane, gs, inv, tma,
+                  h * G + (G > 32 ? (quarter * 32) & (G - 1) : 0), q_row + hx * QT + (quarter * 32 >> gs), rows);
         ++nf[hx];
       }
     }

@@ -390,6 +390,32 @@ def test_prefill_paged_prefix_poisoned(b200, h, hkv, variant):
     _status_ok()
 
 
+@pytest.mark.parametrize("h,hkv", [(4, 2), (64, 1)])
+@pytest.mark.parametrize("block_size,cols", [(256, None), (512, None), (768, None), (256, 3)])
+def test_prefill_paged_block_sizes(b200, block_size, cols, h, hkv):
+    """Tiles counted along the block table: blocks of two, four and six tiles, the last one ragged; a table that ends before the
+    keys do (the rest reads as zeros)."""
+    pkg, _ = b200
+    g = torch.Generator().manual_seed(block_size + h)
+    lens, prefix = [block_size * 2 + 1, 1025, 127, block_size], [block_size, 0, 0, 0]
+    bt, nb = make_block_tables(lens, block_size, g)
+    kc = torch.randn(nb, block_size, hkv, 128, generator=g).to(torch.bfloat16)
+    vc = torch.randn(nb, block_size, hkv, 128, generator=g).to(torch.bfloat16)
+    lq = [a - b for a, b in zip(lens, prefix)]
+    cu_q, cu_k = torch.tensor([0] + lq).cumsum(0).to(torch.int32), torch.tensor([0] + lens).cumsum(0).to(torch.int32)
+    q = torch.randn(sum(lq), h, 128, generator=g).to(torch.bfloat16)
+    bt = bt[:, :cols].contiguous()
+    out = pkg.prefill_attention(q.to(DEV), kc.to(DEV), vc.to(DEV), cu_q.to(DEV), cu_k.to(DEV), max(lq), max(lens),
+                                default_scale(128), hkv, block_tables=bt.to(DEV), kernel_variant=VARIANTS["tcgen05"])
+    torch.cuda.synchronize()
+    if cols is not None:                                    # the oracle's table: one more block, of zeros
+        need = -(-max(lens) // block_size)
+        bt = torch.cat([bt, torch.full((len(lens), need - cols), nb, dtype=torch.int32)], 1)
+        kc, vc = (torch.cat([c, torch.zeros_like(c[:1])]) for c in (kc, vc))
+    _close(out, prefill_attn_ref(q, kc, vc, cu_q, cu_k, default_scale(128), bt))
+    _status_ok()
+
+
 def test_prefill_config3_scale_and_many_sequences(b200):
     """256 prompts of 100 .. 1024 tokens, dense, against the oracle on a sample of
     sequences, and a batch of more than 1024 short sequences (the slot table no longer fits in shared memory)."""
