@@ -30,6 +30,10 @@ namespace b200 {
 extern std::atomic<long long> g_launches;
 
 constexpr int kDecStages = 3;
+// Tiles that a CTA's first unit has on their way into L2 ahead of the wait (at most 8), while the kernel in front ends and the
+// memory is idle.  Us per layer of a graph with the producer in front at 3 | 5 | 6 | 8: 37 sequences of 100 .. 1024 tokens,
+// 16/8 heads, 18.9 | 18.4 | 18.4 | 19.0; 256 of 100 .. 2048, 2/1 heads, 29.1 | 28.6 | 28.6 | 28.7.
+constexpr int kDecAhead = 5;
 constexpr int kDecProducerWarp = kDecConsumerWarps;
 constexpr int kDecEpilogueWarp = kDecConsumerWarps + 1;
 constexpr int kDecThreads = kDecConsumers + 64;
@@ -149,20 +153,14 @@ __device__ __forceinline__ void dec_merge_partials(const DecodeParams& p, int pa
   }
 }
 
-// L2 prefetch of the full tiles among [t0, t1), which lie in the blocks of table columns col0 and col0 + 1.
+// L2 prefetch of the full tiles among [t0, t1), at most eight, which lie in the blocks of table columns col0 and col0 + 1: a box
+// (half of the K or V rows' columns) per lane.
 __device__ __forceinline__ void dec_prefetch_tiles(const DecodeParams& p, const CUtensorMap& map_k, const CUtensorMap& map_v, int h,
-                                                   int t0, int t1, int len, const int* bt, int col0, int blk0, int blk1) {
-  for (int t = t0; t < t1; ++t) {
-    const int tok0 = t * kTile, col = tok0 / p.block_size;
-    if (tok0 + kTile > len) return;
-    const int blk = col == col0 ? blk0 : col == col0 + 1 ? blk1 : -1;
-    if (blk < 0 || blk >= p.num_blocks) return;
-    const int slot0 = static_cast<int>(blk * static_cast<long long>(p.block_size)) + (tok0 - col * p.block_size);
-    tma_prefetch_l2_3d(&map_k, 0, h, slot0);
-    tma_prefetch_l2_3d(&map_k, 64, h, slot0);
-    tma_prefetch_l2_3d(&map_v, 0, h, slot0);
-    tma_prefetch_l2_3d(&map_v, 64, h, slot0);
-  }
+                                                   int t0, int t1, int len, int lane, int col0, int blk0, int blk1) {
+  const int t = t0 + (lane >> 2), tok0 = t * kTile, col = tok0 / p.block_size;
+  const int blk = col == col0 ? blk0 : col == col0 + 1 ? blk1 : -1;
+  if (t >= t1 || tok0 + kTile > len || blk < 0 || blk >= p.num_blocks) return;
+  tma_prefetch_l2_3d(lane & 2 ? &map_v : &map_k, (lane & 1) * 64, h, static_cast<int>(blk * static_cast<long long>(p.block_size)) + (tok0 - col * p.block_size));
 }
 
 __device__ __forceinline__ void dec_store_partial(const DecodeParams& p, int slot, int gq, int lane, const DecPart& r) {
@@ -470,11 +468,12 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
 
   if (warp == kDecProducerWarp) {
     // =========================== producer warp ===========================
-    if (lane != 0) return;
-    tma_prefetch_desc(&map_k);
-    tma_prefetch_desc(&map_v);
-    tma_prefetch_desc(&map_k16);
-    tma_prefetch_desc(&map_v16);
+    if (lane == 0) {
+      tma_prefetch_desc(&map_k);
+      tma_prefetch_desc(&map_v);
+      tma_prefetch_desc(&map_k16);
+      tma_prefetch_desc(&map_v16);
+    }
     int it = 0, n_unit = 0;
     bool ok = true;
     // The SM's second CTA (ids from the SM count on) counts from the short end, so that long and short units share an SM.
@@ -487,7 +486,8 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
     int cur_blk1 = cur_col0 + 1 < p.bt_cols ? cur_bt[cur_col0 + 1] : -1;
     // Bring the first tiles into L2 while the kernel in front still runs: nothing is read, so it does not matter
     // that that kernel may be writing this step's rows.
-    dec_prefetch_tiles(p, map_k, map_v, cur.h, cur.t0, min(cur.t1, cur.t0 + kDecStages), cur.len, cur_bt, cur_col0, cur_blk0, cur_blk1);
+    dec_prefetch_tiles(p, map_k, map_v, cur.h, cur.t0, min(cur.t1, cur.t0 + kDecAhead), cur.len, lane, cur_col0, cur_blk0, cur_blk1);
+    if (lane != 0) return;
     asm volatile("griddepcontrol.wait;" ::: "memory");   // from here on: query rows and the cache
     while (true) {
       const int last_col = (cur.len - 1) / p.block_size;
