@@ -293,7 +293,7 @@ static size_t cluster_smem_bytes(int G, int ctas) {
 
 // CTAs per (sequence, kv head), or 0: leave the batch to the general kernel.  What is known on the host is the number of
 // pairs and the capacity of a block-table row.  One CTA per SM and clusters of at most 8 (of 16 only a few fit on the chip
-// at a time), so up to 8 CTAs per pair for 18 pairs, 4 for 37, and so on; and a pair's CTAs must be able to bear the
+// at a time), so up to 8 CTAs per pair for 9 pairs, 4 for 33, and so on; and a pair's CTAs must be able to bear the
 // longest pair the table allows: beyond kCluMaxTiles each (8 us at the 66 GB/s that one SM draws) the general
 // kernel, which cuts long pairs as it needs, is the faster one.  Both sides, us per layer of a decode graph with the producer
 // in front, this kernel | the general one:
@@ -304,15 +304,16 @@ static size_t cluster_smem_bytes(int G, int ctas) {
 //   40 columns, left to the general kernel from 33 on: 1 of 562 7.2 | 9.0, 4 of 562 7.7 | 9.8; but 4 with one of
 //     4000 13.5 | 11.6, and of 160 columns 2 with one of 30000 61.9 | 32.6.
 // So the line on the table's width is what keeps the worst case near the general kernel's, and it costs short sequences
-// under a wide table 20 %.  Of clusters of 4, 33 fit on the chip at a time: 34 .. 37 pairs, which the line below lets in,
-// take two rounds (4/2 heads, 16 sequences of 562 tokens 7.7 | 9.8, 17 of them 12.3 | 9.9).
+// under a wide table 20 %.  Of clusters of 4, 33 fit on the chip at a time (what a GPC has left over stays idle): 34 .. 37 pairs would
+// take two rounds and go on clusters of 2, or, under wider tables, to the general kernel.  17 sequences of 562 tokens, 4/2
+// heads, on clusters of 4 | 2 | the general kernel: 11.7 | 7.6 | 9.4 us, 18 of 50 .. 2000 14.4 | 12.4 | 10.6.
 constexpr int kCluMaxTiles = 16;
 int decode_cluster_ctas(int batch, int Hkv, int G, int max_tiles) {
   const int sms = sm_count();
   const long long pairs = static_cast<long long>(batch) * Hkv;
   if (G > kCluMaxG || pairs > sms) return 0;
   int c = 8;
-  while (c > 1 && (c * pairs > (c == 8 ? sms / 2 : sms) || c * G > 32 || c / 2 >= max_tiles)) c /= 2;
+  while (c > 1 && (c * pairs > (c == 8 ? sms / 2 : c == 4 ? sms - sms / 9 : sms) || c * G > 32 || c / 2 >= max_tiles)) c /= 2;
   return max_tiles <= c * kCluMaxTiles ? c : 0;
 }
 

@@ -50,6 +50,12 @@ def test_decode_shares(kind, n, h, hkv):
     _lib.check(_lib.load().b200_device_status())
 
 
+@pytest.mark.parametrize("kind,n,h,hkv", [("562", 33, 2, 1), ("562", 17, 4, 2), ("ragged", 37, 4, 1), ("ragged", 37, 2, 1), ("3000", 17, 4, 2)])
+def test_decode_between_cluster_sizes(kind, n, h, hkv):
+    """The last pairs on clusters of 4, the first on clusters of 2, and a table too wide for those."""
+    test_decode_shares(kind, n, h, hkv)
+
+
 @pytest.mark.parametrize("slots", ["own", "anywhere", "holes"])
 @pytest.mark.parametrize("n,h,hkv", [(1, 16, 8), (3, 8, 8), (9, 2, 1), (70, 4, 2), (140, 2, 1), (20, 16, 8), (37, 16, 8), (160, 8, 4),
                                      (161, 4, 2), (513, 2, 1)])
