@@ -15,37 +15,47 @@ extern std::atomic<long long> g_launches;
 constexpr int kStoreThreads = 256;
 constexpr int kStoreUnroll = 4;
 
+// Index: unsigned while twice the number of vectors fits in it (the division by the row's length is an eighth of the 64-bit
+// one's instructions), else long long.
+template <typename Index>
 __global__ void __launch_bounds__(kStoreThreads)
 store_kvcache_kernel(const char* __restrict__ key, const char* __restrict__ value, long long key_stride_b,
                      long long value_stride_b, char* __restrict__ k_cache, char* __restrict__ v_cache,
-                     const int* __restrict__ slot_mapping, long long total_vecs, int row_vecs, long long n_slots) {
+                     const int* __restrict__ slot_mapping, Index total_vecs, Index row_vecs, long long n_slots) {
   // Let a dependent launch (the decode kernel that follows in the stream) start its prologue
   // now; it still waits for this grid to finish before it reads the cache.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   const long long row_bytes = static_cast<long long>(row_vecs) * 16;
-  const long long step = static_cast<long long>(gridDim.x) * kStoreThreads * kStoreUnroll;
-  for (long long base = static_cast<long long>(blockIdx.x) * kStoreThreads * kStoreUnroll + threadIdx.x;
+  const Index step = static_cast<Index>(gridDim.x) * kStoreThreads * kStoreUnroll;
+  for (Index base = static_cast<Index>(blockIdx.x) * kStoreThreads * kStoreUnroll + threadIdx.x;
        base < total_vecs; base += step) {
-    uint4 data[kStoreUnroll];
+    const char* src[kStoreUnroll];
     char* dst[kStoreUnroll];
 #pragma unroll
     for (int u = 0; u < kStoreUnroll; ++u) {
-      const long long idx = base + static_cast<long long>(u) * kStoreThreads;
+      const Index idx = base + u * kStoreThreads;
       dst[u] = nullptr;
       if (idx < total_vecs) {
-        const long long row = idx / row_vecs;           // (token, K|V) pair
-        const int vec = static_cast<int>(idx - row * row_vecs);
+        const Index row = idx / row_vecs;               // (token, K|V) pair
+        const long long vec = idx - row * row_vecs;
         const long long tok = row >> 1;
         const bool is_v = (row & 1) != 0;
         const long long slot = slot_mapping[tok];
         if (slot >= 0 && slot < n_slots) {
-          const char* src = (is_v ? value + tok * value_stride_b : key + tok * key_stride_b) + vec * 16;
-          data[u] = __ldg(reinterpret_cast<const uint4*>(src));
+          src[u] = (is_v ? value + tok * value_stride_b : key + tok * key_stride_b) + vec * 16;
           dst[u] = (is_v ? v_cache : k_cache) + slot * row_bytes + vec * 16;
         }
       }
     }
+    // The slots are not written by any kernel that lets this one start early, so the first pass has its places by the time
+    // the kernel in front ends; K, V and the cache are touched behind the wait (which costs the later passes nothing).  With the
+    // 32-bit division, per launch in a graph of stores, 8 kv heads: 256 tokens 2.33 -> 1.07 us, 4096 5.45 -> 4.0, 16384 21.9 -> 20.1,
+    // 140000 184.8 -> 185.6; an eager layer of 256 sequences of 100 .. 2048 tokens, store and decode, 170.1 -> 165.9.
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    uint4 data[kStoreUnroll];
+#pragma unroll
+    for (int u = 0; u < kStoreUnroll; ++u)
+      if (dst[u]) data[u] = __ldg(reinterpret_cast<const uint4*>(src[u]));
 #pragma unroll
     for (int u = 0; u < kStoreUnroll; ++u)
       if (dst[u]) *reinterpret_cast<uint4*>(dst[u]) = data[u];
@@ -83,10 +93,13 @@ extern "C" int b200_store_kvcache(const void* key, const void* value, int64_t ke
   if (sms <= 0) return set_error(kErrNoDriver, "store_kvcache: no CUDA device");
   const long long cap = static_cast<long long>(sms) * 16;
   if (blocks > cap) blocks = cap;
-  const cudaError_t le = launch_early(store_kvcache_kernel, static_cast<unsigned>(blocks), kStoreThreads, 0, static_cast<cudaStream_t>(stream),
-                                      static_cast<const char*>(key), static_cast<const char*>(value), ks, vs,
-                                      static_cast<char*>(k_cache), static_cast<char*>(v_cache), slot_mapping, total, row_vecs,
-                                      static_cast<long long>(n_slots));
+  auto launch = [&](auto kernel, auto total_vecs, auto vecs) {
+    return launch_early(kernel, static_cast<unsigned>(blocks), kStoreThreads, 0, static_cast<cudaStream_t>(stream),
+                        static_cast<const char*>(key), static_cast<const char*>(value), ks, vs, static_cast<char*>(k_cache),
+                        static_cast<char*>(v_cache), slot_mapping, total_vecs, vecs, static_cast<long long>(n_slots));
+  };
+  const cudaError_t le = total < (1LL << 31) ? launch(store_kvcache_kernel<unsigned>, static_cast<unsigned>(total), static_cast<unsigned>(row_vecs))
+                                             : launch(store_kvcache_kernel<long long>, total, static_cast<long long>(row_vecs));
   g_launches.fetch_add(1);
   return check_cuda(le != cudaSuccess ? le : cudaGetLastError(), "store_kvcache launch");
 }

@@ -115,6 +115,26 @@ def test_store_bit_exact(b200, dtype, hkv, d, n):
     assert torch.equal(vc.cpu().view(view), v_cache.view(view))
 
 
+@pytest.mark.parametrize("over", [-1, 3])
+def test_store_index_width(b200, over):
+    """Either side of 2^31 16-byte vectors, where the index becomes 64-bit: only the first and the last rows have a slot."""
+    pkg, _ = b200
+    n = (1 << 30) + over
+    k = torch.empty(n, 1, 8, dtype=torch.bfloat16, device=DEV)
+    slots = torch.full((n,), -1, dtype=torch.int32, device=DEV)
+    rows = torch.cat([torch.arange(5), n - 1 - torch.arange(5)])
+    k[rows.to(DEV)] = torch.arange(80, dtype=torch.bfloat16, device=DEV).view(10, 1, 8)
+    slots[rows.to(DEV)] = torch.arange(10, dtype=torch.int32, device=DEV)
+    kc = torch.full((1, 256, 1, 8), -1, dtype=torch.bfloat16, device=DEV)
+    vc = torch.full_like(kc, -2)
+    pkg.store_kvcache(k, k, kc, vc, slots)
+    torch.cuda.synchronize()
+    del k, slots
+    torch.cuda.empty_cache()
+    for c, rest in ((kc, -1), (vc, -2)):
+        assert torch.equal(c[0, :10].float().cpu(), torch.arange(80.).view(10, 1, 8)) and bool((c[0, 10:] == rest).all())
+
+
 def test_store_empty_and_all_skipped(b200):
     pkg, _ = b200
     kc = torch.zeros(2, 256, 2, 128, dtype=torch.bfloat16, device=DEV)
