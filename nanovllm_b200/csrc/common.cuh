@@ -230,6 +230,21 @@ __device__ __forceinline__ unsigned long long f32x2_add(unsigned long long a, un
   return d;
 }
 
+// Loads of what a kernel that is still running when this one starts may write: they stay behind griddepcontrol.wait where they stand
+// behind it, and they are coherent.  __ldg, and a load through a const __restrict__ pointer, promise neither: the compiler
+// may put them wherever address and predicate are known.
+__device__ __forceinline__ uint4 ld_row16(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_u32(const void* p) {
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ int ld_s32(const int* p) { return static_cast<int>(ld_u32(p)); }
+
 __device__ __forceinline__ float ld_cg_f32(const float* p) {
   float v;
   asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p));

@@ -39,7 +39,7 @@ struct DecodeParams {
 // One 16-byte chunk per lane of head h of the step's row `tok`: lanes 0 .. 15 K, 16 .. 31 V.
 __device__ __forceinline__ uint4 step_chunk(const DecodeParams& p, int tok, int h, int lane) {
   const __nv_bfloat16* src = lane < 16 ? p.st_k + tok * p.st_k_stride : p.st_v + tok * p.st_v_stride;
-  return __ldg(reinterpret_cast<const uint4*>(src + h * 128 + (lane & 15) * 8));
+  return ld_row16(src + h * 128 + (lane & 15) * 8);
 }
 
 // 1-D bulk copy global -> shared, completion counted on an mbarrier (addresses and size multiples of 16).

@@ -44,10 +44,10 @@ __device__ __forceinline__ void pf_store_rows(const PrefillParams& p, const char
                                               int h0, int h1, int lane) {
   const int vecs = p.Hkv * 16;
   for (int r = row0; r < row1; ++r) {
-    const long long slot = __ldg(p.st_slots + r);
+    const long long slot = ld_s32(p.st_slots + r);
     if (slot < 0 || slot >= p.st_n_slots) continue;
     for (int v = h0 * 16 + lane; v < h1 * 16; v += 32)
-      reinterpret_cast<uint4*>(cache)[slot * vecs + v] = __ldg(reinterpret_cast<const uint4*>(src + r * stride) + v);
+      reinterpret_cast<uint4*>(cache)[slot * vecs + v] = ld_row16(src + r * stride + v * 16);
   }
 }
 
@@ -145,7 +145,7 @@ prefill_attn_mma_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       const int r0 = max(tq0 - key0, 0), r1 = min(min(tq1 - key0, kPfTile), p.st_tokens - row0);
       int slots[2];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) slots[u] = u * 32 + lane >= r0 && u * 32 + lane < r1 ? __ldg(p.st_slots + row0 + u * 32 + lane) : -1;
+      for (int u = 0; u < 2; ++u) slots[u] = u * 32 + lane >= r0 && u * 32 + lane < r1 ? ld_s32(p.st_slots + row0 + u * 32 + lane) : -1;
       // These are among the CTA's last tiles: once the very last is under way their stages are not loaded again, and each
       // full-barrier is in its tile's phase.
       if (!mbar_wait(&bar_last, 0, abort_flag) || !mbar_wait(&bar_full[t % kPfStages], (t / kPfStages) & 1, abort_flag)) return;
@@ -205,10 +205,10 @@ prefill_attn_mma_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
         p.q + static_cast<long long>(q_begin + tok1) * p.q_row_stride + (h * G + r1 % G) * 128);
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
-      qa[ks][0] = ok0 ? __ldg(q0 + ks * 8 + quad) : 0u;
-      qa[ks][1] = ok1 ? __ldg(q1 + ks * 8 + quad) : 0u;
-      qa[ks][2] = ok0 ? __ldg(q0 + ks * 8 + 4 + quad) : 0u;
-      qa[ks][3] = ok1 ? __ldg(q1 + ks * 8 + 4 + quad) : 0u;
+      qa[ks][0] = ok0 ? ld_u32(q0 + ks * 8 + quad) : 0u;
+      qa[ks][1] = ok1 ? ld_u32(q1 + ks * 8 + quad) : 0u;
+      qa[ks][2] = ok0 ? ld_u32(q0 + ks * 8 + 4 + quad) : 0u;
+      qa[ks][3] = ok1 ? ld_u32(q1 + ks * 8 + 4 + quad) : 0u;
     }
   }
   float o[16][4];

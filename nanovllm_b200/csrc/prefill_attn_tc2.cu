@@ -210,7 +210,7 @@ __device__ __forceinline__ void t2_output_split(const PrefillParams& p, const CU
 __device__ __forceinline__ int t2_store_slots(const PrefillParams& p, int row0, int rows, int lane) {
   int s[4];
 #pragma unroll
-  for (int u = 0; u < 4; ++u) s[u] = u * 32 + lane < rows ? __ldg(p.st_slots + row0 + u * 32 + lane) : 0;
+  for (int u = 0; u < 4; ++u) s[u] = u * 32 + lane < rows ? ld_s32(p.st_slots + row0 + u * 32 + lane) : 0;
   const int s0 = __shfl_sync(0xffffffffu, s[0], 0);
   bool run = s0 >= 0 && s0 + static_cast<long long>(rows) <= p.st_n_slots;
 #pragma unroll
@@ -232,7 +232,7 @@ __device__ __forceinline__ void t2_store_tile(const PrefillParams& p, const CUte
 #pragma unroll 1      // (short code: unrolled four times it costs the kernel 5 %, the hot loops fetch from the same cache)
   for (int e = boxes * 512 + lane; e < rows * 16; e += 32) {
     const int r = e >> 4, c = e & 15;
-    const long long slot = s0 >= 0 ? s0 + r : __ldg(p.st_slots + row0 + r);
+    const long long slot = s0 >= 0 ? s0 + r : ld_s32(p.st_slots + row0 + r);
     if (slot < 0 || slot >= p.st_n_slots) continue;
     *reinterpret_cast<uint4*>(cache + slot * row_bytes + h * 256 + c * 16) =
         *reinterpret_cast<const uint4*>(tile + (c >> 3) * kT2Sub + r * 128 + (((c & 7) ^ (r & 7)) << 4));
@@ -247,11 +247,11 @@ __device__ __forceinline__ void t2_store_rows(const PrefillParams& p, const char
   const int vecs = p.Hkv * 16;
 #pragma unroll 1
   for (int r = row0; r < row1; ++r) {
-    const long long slot = __ldg(p.st_slots + r);
+    const long long slot = ld_s32(p.st_slots + r);
     if (slot < 0 || slot >= p.st_n_slots) continue;
 #pragma unroll 1
     for (int v = lane; v < vecs; v += 32)
-      reinterpret_cast<uint4*>(cache)[slot * vecs + v] = __ldg(reinterpret_cast<const uint4*>(src + r * stride) + v);
+      reinterpret_cast<uint4*>(cache)[slot * vecs + v] = ld_row16(src + r * stride + v * 16);
   }
 }
 

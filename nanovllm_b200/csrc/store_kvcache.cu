@@ -19,9 +19,8 @@ constexpr int kStoreUnroll = 4;
 // one's instructions), else long long.
 template <typename Index>
 __global__ void __launch_bounds__(kStoreThreads)
-store_kvcache_kernel(const char* __restrict__ key, const char* __restrict__ value, long long key_stride_b,
-                     long long value_stride_b, char* __restrict__ k_cache, char* __restrict__ v_cache,
-                     const int* __restrict__ slot_mapping, Index total_vecs, Index row_vecs, long long n_slots) {
+store_kvcache_kernel(const char* key, const char* value, long long key_stride_b,
+                     long long value_stride_b, char* k_cache, char* v_cache, const int* slot_mapping, Index total_vecs, Index row_vecs, long long n_slots) {
   // Let a dependent launch (the decode kernel that follows in the stream) start its prologue
   // now; it still waits for this grid to finish before it reads the cache.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -48,14 +47,16 @@ store_kvcache_kernel(const char* __restrict__ key, const char* __restrict__ valu
       }
     }
     // The slots are not written by any kernel that lets this one start early, so the first pass has its places by the time
-    // the kernel in front ends; K, V and the cache are touched behind the wait (which costs the later passes nothing).  With the
-    // 32-bit division, per launch in a graph of stores, 8 kv heads: 256 tokens 2.33 -> 1.07 us, 4096 5.45 -> 4.0, 16384 21.9 -> 20.1,
-    // 140000 184.8 -> 185.6; an eager layer of 256 sequences of 100 .. 2048 tokens, store and decode, 170.1 -> 165.9.
+    // the kernel in front ends; K, V and the cache are touched behind the wait (which costs the later passes nothing).  Their loads
+    // must not be left to the compiler: through the read-only path it had them ahead of the wait, as the times showed (256 tokens
+    // 1.08 us per launch in a graph of stores, an eager layer of 256 sequences of 100 .. 2048 tokens, store and decode, 160.3 us).
+    // With the 32-bit division, per launch in a graph of stores, 8 kv heads: 256 tokens 2.33 -> 1.34 us, 4096 5.45 -> 4.4,
+    // 16384 21.9 -> 20.9, 140000 184.8 -> 186.7; the eager layer 163.1.
     asm volatile("griddepcontrol.wait;" ::: "memory");
     uint4 data[kStoreUnroll];
 #pragma unroll
     for (int u = 0; u < kStoreUnroll; ++u)
-      if (dst[u]) data[u] = __ldg(reinterpret_cast<const uint4*>(src[u]));
+      if (dst[u]) data[u] = ld_row16(src[u]);
 #pragma unroll
     for (int u = 0; u < kStoreUnroll; ++u)
       if (dst[u]) *reinterpret_cast<uint4*>(dst[u]) = data[u];

@@ -1,0 +1,150 @@
+"""What the kernels read while the kernel in front of them still runs.  GPU: a kernel that lets its dependents start early
+(griddepcontrol.launch_dependents) and writes its arrays only afterwards stands in front of every call; the call must see what
+it wrote.  The same call on the same values with nothing running is the reference, bit for bit."""
+import os
+import re
+
+import pytest
+import torch
+
+from workloads import cu_seqlens, decode_slots, default_scale, make_block_tables
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "nanovllm_b200", "csrc")
+DEV = "cuda:0"
+DELAY = 200_000                  # cycles between the early trigger and the writes (0.1 ms)
+SOURCE = r"""
+extern "C" __global__ void late_copy(const int* src, int* dst, int words, int cycles) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const long long t0 = clock64();
+  while (clock64() - t0 < cycles) {}
+  for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
+}
+"""
+
+
+def test_rows_are_not_read_through_the_read_only_path():
+    """__ldg and const __restrict__ let the compiler move a load ahead of griddepcontrol.wait (and the hardware serve it from a
+    cache that nobody invalidates): in kernels that start early only for arrays that no kernel in front may write."""
+    early = [f for f in sorted(os.listdir(CSRC)) if "griddepcontrol" in open(os.path.join(CSRC, f)).read()]
+    assert len(early) >= 5
+    for f in early + ["decode_common.cuh"]:
+        code = re.sub(r"//.*", "", open(os.path.join(CSRC, f)).read())
+        assert "__restrict__" not in code, f
+        for arg in re.findall(r"__ldg\((.{20})", code):
+            allowed = ("p.cu_q", "p.cu_k") if "prefill" in f else ("p.st_slots",) if f == "decode_attn.cu" else ()
+            assert arg.startswith(allowed) if allowed else False, (f, arg)
+
+
+@pytest.fixture(scope="module")
+def late_copy():
+    kernel = torch.cuda._compile_kernel(SOURCE, "late_copy")
+    return lambda src, dst: kernel(grid=(1, 1, 1), block=(1024, 1, 1), args=[src, dst, src.numel(), DELAY])
+
+
+def _packed(tensors):
+    """The tensors in one buffer of 32-bit words on the device (each at a multiple of 16 bytes), and views of them in it."""
+    sizes = [-(-t.numel() * t.element_size() // 16) * 4 for t in tensors.values()]
+    buf = torch.zeros(sum(sizes), dtype=torch.int32, device=DEV)
+    views, at = {}, 0
+    for (name, t), size in zip(tensors.items(), sizes):
+        words = t.numel() * t.element_size() // 4
+        views[name] = buf[at:at + words].view(t.dtype).view(t.shape)
+        views[name].copy_(t)
+        at += size
+    return buf, views
+
+
+def _compare(late_copy, before, after, prepare, call):
+    """call(views, state) -> the tensors it wrote: with `after` in place and nothing running, and with `before` in place until a
+    kernel that is still running when the call's kernel starts puts `after` there.  `state` is made ahead of that kernel, so
+    that nothing is launched between it and the call's."""
+    with torch.inference_mode():
+        quiet, views = _packed(after)
+        state = prepare()
+        torch.cuda.synchronize()
+        want = call(views, state)
+        for _ in range(3):
+            buf, views = _packed(before)
+            state = prepare()
+            torch.cuda.synchronize()
+            late_copy(quiet, buf)
+            got = call(views, state)
+            torch.cuda.synchronize()
+            assert torch.equal(buf, quiet) and len(got) == len(want)
+            for a, b in zip(got, want):
+                assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+
+
+def _rows(seed, **shapes):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return {k: torch.randn(*s, device=DEV, generator=g).to(torch.bfloat16) for k, s in shapes.items()}
+
+
+def _caches(blocks, hkv):
+    return lambda: tuple(torch.zeros(blocks, 256, hkv, 128, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+
+
+def _layer(h, hkv, caches, call, **context):
+    import nanovllm_b200
+    from nanovllm_b200.utils.context import reset_context, set_context
+    att = nanovllm_b200.Attention(h, 128, default_scale(128), hkv)
+    att.k_cache, att.v_cache = caches
+    set_context(**context)
+    out = call(att)
+    reset_context()
+    return (out, *caches)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,hkv", [(1, 8), (7, 1), (256, 8), (20000, 8)])                  # the last: two passes
+def test_store_behind_a_kernel_that_writes_its_rows(late_copy, n, hkv):
+    import nanovllm_b200
+    slots = torch.arange(n, dtype=torch.int32, device=DEV).flip(0)
+    shape = dict(k=(n, hkv, 128), v=(n, hkv, 128))
+
+    def call(m, caches):
+        nanovllm_b200.store_kvcache(m["k"], m["v"], *caches, slots)
+        return caches
+    _compare(late_copy, _rows(1, **shape), _rows(2, **shape), _caches(n // 256 + 1, hkv), call)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,h,hkv", [(1, 16, 8), (3, 8, 8), (37, 16, 8), (200, 4, 2)])     # clusters, store inside, store in front
+def test_layer_decode_behind_a_kernel_that_writes_its_rows(late_copy, n, h, hkv):
+    g = torch.Generator().manual_seed(n)
+    lens = torch.randint(1, 700, (n,), generator=g).tolist()
+    bt, blocks = make_block_tables(lens, 256, g)
+    ctx = dict(is_prefill=False, slot_mapping=decode_slots(lens, bt, 256).to(DEV), block_tables=bt.to(DEV),
+               context_lens=torch.tensor(lens, dtype=torch.int32, device=DEV))
+    shape = dict(q=(n, h, 128), k=(n, hkv, 128), v=(n, hkv, 128))
+    _compare(late_copy, _rows(1, **shape), _rows(2, **shape), _caches(blocks, hkv),
+             lambda m, caches: _layer(h, hkv, caches, lambda att: att(m["q"], m["k"], m["v"]), **ctx))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("h,hkv,lens", [(16, 8, [137]), (16, 8, [1, 63, 64, 65]), (5, 1, [100, 200]), (16, 8, [700, 31, 2000]),
+                                        (2, 2, [900] * 40)])                               # mma.sync, tcgen05 in both forms
+def test_layer_prefill_behind_a_kernel_that_writes_its_rows(late_copy, h, hkv, lens):
+    n = sum(lens)
+    cu = cu_seqlens(lens).to(DEV)
+    ctx = dict(is_prefill=True, cu_seqlens_q=cu, cu_seqlens_k=cu, max_seqlen_q=max(lens), max_seqlen_k=max(lens),
+               slot_mapping=torch.arange(n, dtype=torch.int32, device=DEV))
+    shape = dict(q=(n, h, 128), k=(n, hkv, 128), v=(n, hkv, 128))
+    _compare(late_copy, _rows(1, **shape), _rows(2, **shape), _caches(n // 256 + 1, hkv),
+             lambda m, caches: _layer(h, hkv, caches, lambda att: att(m["q"], m["k"], m["v"]), **ctx))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 37, 3000])                                               # one head a pass, four heads a pass
+def test_producer_behind_a_kernel_that_writes_its_rows(late_copy, n):
+    from nanovllm_b200.layers.qk_norm_rope import qk_norm_rope_store
+    h, hkv = 16, 8
+    w = _rows(3, q=(128,), k=(128,))
+    table = torch.randn(4096, 1, 128, device=DEV, generator=torch.Generator(device=DEV).manual_seed(4))
+    pos, slots = torch.arange(n, device=DEV), torch.arange(n, dtype=torch.int32, device=DEV)
+    shape = dict(qkv=(n, (h + 2 * hkv) * 128))
+
+    def call(m, caches):
+        q, k, _ = qk_norm_rope_store(m["qkv"], pos, w["q"], w["k"], table, 1e-6, h, hkv, *caches, slots)
+        return (q, k, *caches)
+    _compare(late_copy, _rows(1, **shape), _rows(2, **shape), _caches(n // 256 + 1, hkv), call)
