@@ -25,7 +25,7 @@
  *      decode                 context_lens, block_tables; b200_store_decode_attn also slot_mapping
  *      prefill                cu_seqlens_q, cu_seqlens_k
  *      producer               positions, slot_mapping, the rotary table and the norm weights (for decode-sized batches)
- *      store                  slot_mapping
+ *      store                  nothing (what it reads ahead it reads again)
  *    So a kernel that lets its dependents start early must not write these arrays.  Of this library the store,
  *    producer, decode and mma.sync prefill kernels do (they write cache rows, q, k and outputs only); the metadata unpack,
  *    all-reduce and tcgen05 prefill kernels do not.  Behind any other kernel or copy there is nothing to observe.

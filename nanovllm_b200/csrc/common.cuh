@@ -244,6 +244,14 @@ __device__ __forceinline__ uint32_t ld_u32(const void* p) {
   return v;
 }
 __device__ __forceinline__ int ld_s32(const int* p) { return static_cast<int>(ld_u32(p)); }
+// Past L1: what is read ahead of griddepcontrol.wait, as a hint, and again behind it.
+__device__ __forceinline__ int ld_cg_s32(const int* p) {
+  int v;
+  asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+// A hint, so it may go out before the line is complete: L2 is where it will be completed.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory"); }
 
 __device__ __forceinline__ float ld_cg_f32(const float* p) {
   float v;

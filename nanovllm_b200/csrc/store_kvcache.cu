@@ -26,40 +26,47 @@ store_kvcache_kernel(const char* key, const char* value, long long key_stride_b,
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const long long row_bytes = static_cast<long long>(row_vecs) * 16;
   const Index step = static_cast<Index>(gridDim.x) * kStoreThreads * kStoreUnroll;
+  bool first = true;
   for (Index base = static_cast<Index>(blockIdx.x) * kStoreThreads * kStoreUnroll + threadIdx.x;
        base < total_vecs; base += step) {
     const char* src[kStoreUnroll];
-    char* dst[kStoreUnroll];
+    Index vec[kStoreUnroll];
+    int tok[kStoreUnroll], slot[kStoreUnroll];
+    unsigned is_v = 0;                                  // a bit per vector
 #pragma unroll
     for (int u = 0; u < kStoreUnroll; ++u) {
       const Index idx = base + u * kStoreThreads;
-      dst[u] = nullptr;
+      tok[u] = -1;
       if (idx < total_vecs) {
         const Index row = idx / row_vecs;               // (token, K|V) pair
-        const long long vec = idx - row * row_vecs;
-        const long long tok = row >> 1;
-        const bool is_v = (row & 1) != 0;
-        const long long slot = slot_mapping[tok];
-        if (slot >= 0 && slot < n_slots) {
-          src[u] = (is_v ? value + tok * value_stride_b : key + tok * key_stride_b) + vec * 16;
-          dst[u] = (is_v ? v_cache : k_cache) + slot * row_bytes + vec * 16;
+        vec[u] = idx - row * row_vecs;
+        tok[u] = static_cast<int>(row >> 1);
+        is_v |= static_cast<unsigned>(row & 1) << u;
+        src[u] = (row & 1 ? value + tok[u] * value_stride_b : key + tok[u] * key_stride_b) + static_cast<long long>(vec[u]) * 16;
+        if (first) {
+          const int hint = (threadIdx.x & 7) == 0 ? ld_cg_s32(slot_mapping + tok[u]) : -1;
+          if (hint >= 0 && hint < n_slots) prefetch_l2(src[u]);
         }
       }
     }
-    // The slots are not written by any kernel that lets this one start early, so the first pass has its places by the time
-    // the kernel in front ends; K, V and the cache are touched behind the wait (which costs the later passes nothing).  Their loads
-    // must not be left to the compiler: through the read-only path it had them ahead of the wait, as the times showed (256 tokens
-    // 1.08 us per launch in a graph of stores, an eager layer of 256 sequences of 100 .. 2048 tokens, store and decode, 160.3 us).
-    // With the 32-bit division, per launch in a graph of stores, 8 kv heads: 256 tokens 2.33 -> 1.34 us, 4096 5.45 -> 4.4,
-    // 16384 21.9 -> 20.9, 140000 184.8 -> 186.7; the eager layer 163.1.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // Everything is read behind the wait, so the kernel in front may write any of it.  Ahead of it the first pass finds its
+    // places and, going by what the slots are then, has them and its rows on their way into L2.  Loads of K and V must not be left to
+    // the compiler: through the read-only path it had them ahead of the wait, as the times showed (first figures below).
+    // Us per launch in a graph of stores, 8 kv heads, __ldg | slots ahead of the wait | this form: 256 tokens 1.08 | 1.34 | 1.50,
+    // 4096 4.0 | 4.4 | 5.3, 16384 20.1 | 20.9 | 21.2, 140000 185 | 186.7 | 185.5 (everything behind the wait and a 64-bit division: 2.33,
+    // 5.45, 21.9, 184.8); an eager layer of 256 sequences of 100 .. 2048 tokens, store and decode, 160.3 | 163.1 | 161.6.
+    if (first) asm volatile("griddepcontrol.wait;" ::: "memory");
+    first = false;
+#pragma unroll
+    for (int u = 0; u < kStoreUnroll; ++u) slot[u] = tok[u] >= 0 ? ld_s32(slot_mapping + tok[u]) : -1;
     uint4 data[kStoreUnroll];
 #pragma unroll
     for (int u = 0; u < kStoreUnroll; ++u)
-      if (dst[u]) data[u] = ld_row16(src[u]);
+      if (slot[u] >= 0 && slot[u] < n_slots) data[u] = ld_row16(src[u]);
 #pragma unroll
     for (int u = 0; u < kStoreUnroll; ++u)
-      if (dst[u]) *reinterpret_cast<uint4*>(dst[u]) = data[u];
+      if (slot[u] >= 0 && slot[u] < n_slots)
+        *reinterpret_cast<uint4*>((is_v >> u & 1 ? v_cache : k_cache) + slot[u] * row_bytes + static_cast<long long>(vec[u]) * 16) = data[u];
   }
 }
 

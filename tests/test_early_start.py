@@ -108,6 +108,27 @@ def test_store_behind_a_kernel_that_writes_its_rows(late_copy, n, hkv):
     _compare(late_copy, _rows(1, **shape), _rows(2, **shape), _caches(n // 256 + 1, hkv), call)
 
 
+def _slots(n, total, seed):
+    """n slots of `total` in an order of their own, a fifth of them skipped."""
+    g = torch.Generator().manual_seed(seed)
+    s = torch.randperm(total, generator=g)[:n].to(torch.int32)
+    s[torch.randperm(n, generator=g)[:n // 5]] = -1
+    return s
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,hkv", [(1, 8), (7, 1), (256, 8), (3000, 2), (20000, 8)])
+def test_store_behind_a_kernel_that_writes_its_slots(late_copy, n, hkv):
+    import nanovllm_b200
+    blocks = n // 256 + 2
+    rows = _rows(1, k=(n, hkv, 128), v=(n, hkv, 128))
+
+    def call(m, caches):
+        nanovllm_b200.store_kvcache(rows["k"], rows["v"], *caches, m["slots"])
+        return caches
+    _compare(late_copy, dict(slots=_slots(n, blocks * 256, 2)), dict(slots=_slots(n, blocks * 256, 3)), _caches(blocks, hkv), call)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n,h,hkv", [(1, 16, 8), (3, 8, 8), (37, 16, 8), (200, 4, 2)])     # clusters, store inside, store in front
 def test_layer_decode_behind_a_kernel_that_writes_its_rows(late_copy, n, h, hkv):
