@@ -24,8 +24,7 @@
  *    dependents do so (griddepcontrol.launch_dependents), and read part of their metadata before they wait for it:
  *      decode                 context_lens, block_tables; b200_store_decode_attn also slot_mapping
  *      prefill                cu_seqlens_q, cu_seqlens_k
- *      producer               positions, slot_mapping, the rotary table and the norm weights (for decode-sized batches)
- *      store                  nothing (what it reads ahead it reads again)
+ *      store, producer        nothing (what they read ahead they read again)
  *    So a kernel that lets its dependents start early must not write these arrays.  Of this library the store,
  *    producer, decode and mma.sync prefill kernels do (they write cache rows, q, k and outputs only); the metadata unpack,
  *    all-reduce and tcgen05 prefill kernels do not.  Behind any other kernel or copy there is nothing to observe.

@@ -244,10 +244,25 @@ __device__ __forceinline__ uint32_t ld_u32(const void* p) {
   return v;
 }
 __device__ __forceinline__ int ld_s32(const int* p) { return static_cast<int>(ld_u32(p)); }
+__device__ __forceinline__ long long ld_s64(const long long* p) {
+  long long v;
+  asm volatile("ld.global.s64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+// (32 bytes: the address must be a multiple of that)
+__device__ __forceinline__ void ld_row32(const float* p, float4& a, float4& b) {
+  asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(p) : "memory");
+}
 // Past L1: what is read ahead of griddepcontrol.wait, as a hint, and again behind it.
 __device__ __forceinline__ int ld_cg_s32(const int* p) {
   int v;
   asm volatile("ld.global.cg.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ long long ld_cg_s64(const long long* p) {
+  long long v;
+  asm volatile("ld.global.cg.s64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
 // A hint, so it may go out before the line is complete: L2 is where it will be completed.

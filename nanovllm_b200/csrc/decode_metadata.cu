@@ -27,7 +27,7 @@ unpack_decode_metadata_kernel(const int* __restrict__ packed, int bs, int w, int
                               int* __restrict__ slot_mapping, int* __restrict__ context_lens,
                               int* __restrict__ block_tables) {
   // (No early trigger of dependent launches here: the decode kernels read context_lens and the block
-  // table, the producer positions and slots ahead of their own dependency wait, which is only sound if whatever writes them has completed.)
+  // table ahead of their own dependency wait, which is only sound if whatever writes them has completed.)
   const int tid = blockIdx.x * kMetaThreads + threadIdx.x;
   const int stride = gridDim.x * kMetaThreads;
   const long long* p_ids = reinterpret_cast<const long long*>(packed);

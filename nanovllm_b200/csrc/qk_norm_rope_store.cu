@@ -34,6 +34,7 @@ struct QkNormRopeParams {
   const __nv_bfloat16* k_weight;       // (128)
   const float* cos_sin;                // (max_position, 128): 64 cos then 64 sin
   int max_position;
+  bool wide_table;                     // cos_sin lies at a multiple of 32 bytes
   float eps;
   __nv_bfloat16* q_out;                // (n_tokens, H, 128)
   __nv_bfloat16* k_out;                // (n_tokens, Hkv, 128)
@@ -66,28 +67,50 @@ struct QkTokenCtx {
   unsigned long long cosv[4], sinv[4]; // packed pairs; sin carries the sign of this lane's half (-sin for the first)
 };
 
-__device__ __forceinline__ QkTokenCtx qk_token_ctx(const QkNormRopeParams& p, long long pos, long long slot, int sub) {
+// This lane's part of the table row of a position: eight cos there, eight sin 64 floats on.
+__device__ __forceinline__ const float* qk_table_row(const QkNormRopeParams& p, long long pos, int sub) {
+  pos = pos < 0 ? 0 : (pos >= p.max_position ? p.max_position - 1 : pos);
+  return p.cos_sin + pos * 128 + (sub & 7) * 8;
+}
+
+struct QkTableRow {
+  float4 c0, c1, s0, s1;
+};
+__device__ __forceinline__ float4 qk_float4(const uint4& v) {
+  return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+}
+__device__ __forceinline__ QkTableRow qk_load_table(const QkNormRopeParams& p, long long pos, int sub) {
+  const float* cs = qk_table_row(p, pos, sub);
+  QkTableRow t;
+  if (p.wide_table) {
+    ld_row32(cs, t.c0, t.c1);
+    ld_row32(cs + 64, t.s0, t.s1);
+  } else {
+    t.c0 = qk_float4(ld_row16(cs));
+    t.c1 = qk_float4(ld_row16(cs + 4));
+    t.s0 = qk_float4(ld_row16(cs + 64));
+    t.s1 = qk_float4(ld_row16(cs + 68));
+  }
+  return t;
+}
+
+__device__ __forceinline__ QkTokenCtx qk_token_ctx(const QkNormRopeParams& p, const QkTableRow& t, int slot, int sub) {
   QkTokenCtx c;
   c.slot = slot < p.n_slots ? slot : -1;                 // never write outside the cache
-  pos = pos < 0 ? 0 : (pos >= p.max_position ? p.max_position - 1 : pos);
-  const float* cs = p.cos_sin + pos * 128 + (sub & 7) * 8;
-  const float4 c0 = *reinterpret_cast<const float4*>(cs), c1 = *reinterpret_cast<const float4*>(cs + 4);
-  const float4 s0 = *reinterpret_cast<const float4*>(cs + 64), s1 = *reinterpret_cast<const float4*>(cs + 68);
   // first half:  y1 = x1 * cos - x2 * sin      second half:  y2 = x2 * cos + x1 * sin
   // (negating sin is exact, and a + (-t) rounds like a - t)
   const float sg = sub < 8 ? -1.f : 1.f;
-  c.cosv[0] = f32x2_pack(c0.x, c0.y); c.cosv[1] = f32x2_pack(c0.z, c0.w);
-  c.cosv[2] = f32x2_pack(c1.x, c1.y); c.cosv[3] = f32x2_pack(c1.z, c1.w);
-  c.sinv[0] = f32x2_pack(sg * s0.x, sg * s0.y); c.sinv[1] = f32x2_pack(sg * s0.z, sg * s0.w);
-  c.sinv[2] = f32x2_pack(sg * s1.x, sg * s1.y); c.sinv[3] = f32x2_pack(sg * s1.z, sg * s1.w);
+  c.cosv[0] = f32x2_pack(t.c0.x, t.c0.y); c.cosv[1] = f32x2_pack(t.c0.z, t.c0.w);
+  c.cosv[2] = f32x2_pack(t.c1.x, t.c1.y); c.cosv[3] = f32x2_pack(t.c1.z, t.c1.w);
+  c.sinv[0] = f32x2_pack(sg * t.s0.x, sg * t.s0.y); c.sinv[1] = f32x2_pack(sg * t.s0.z, sg * t.s0.w);
+  c.sinv[2] = f32x2_pack(sg * t.s1.x, sg * t.s1.y); c.sinv[3] = f32x2_pack(sg * t.s1.z, sg * t.s1.w);
   return c;
 }
 
 // One q or k head vector: `raw` holds this lane's 8 elements; `w` the lane's 8 weights as bf16 pairs.
 // Every product and every sum is rounded on its own (mul.rn / add.rn, packed two at a time), in the order the
-// reference's eager arithmetic takes them.
-__device__ __forceinline__ uint4 qk_norm_rope_vector(const uint4& raw, const uint32_t (&w)[4],
-                                                     const QkTokenCtx& c, float eps, unsigned half_mask) {
+// reference's eager arithmetic takes them.  First half: normalised and weighted, exact bf16 values as packed pairs.
+__device__ __forceinline__ void qk_normalise(const uint4& raw, const uint32_t (&w)[4], float eps, unsigned half_mask, uint32_t (&ap)[4]) {
   const uint32_t r[4] = {raw.x, raw.y, raw.z, raw.w};
   unsigned long long x[4];
 #pragma unroll
@@ -100,9 +123,7 @@ __device__ __forceinline__ uint4 qk_norm_rope_vector(const uint4& raw, const uin
   for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(half_mask, ss, o);
   const float rinv = __frsqrt_rn(__fadd_rn(__fmul_rn(ss, 1.f / 128.f), eps));      // (a division by 128 is this product, exactly)
   const unsigned long long rinv2 = f32x2_pack(rinv, rinv);
-  // normalise in fp32, round to bf16, scale by the bf16 weight (rounded to bf16 again); the results are
-  // exact bf16 values, so they travel to the partner lane as packed pairs (4 shuffles instead of 8)
-  uint32_t ap[4];
+  // normalise in fp32, round to bf16, scale by the bf16 weight (rounded to bf16 again)
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     float n0, n1;
@@ -111,6 +132,9 @@ __device__ __forceinline__ uint4 qk_norm_rope_vector(const uint4& raw, const uin
     const __nv_bfloat162 m = __hmul2(__floats2bfloat162_rn(n0, n1), *reinterpret_cast<const __nv_bfloat162*>(&w[i]));
     ap[i] = *reinterpret_cast<const uint32_t*>(&m);
   }
+}
+// Second half: rotated.  (The packed pairs travel to the partner lane, 4 shuffles instead of 8.)
+__device__ __forceinline__ uint4 qk_rotate(const uint32_t (&ap)[4], const QkTokenCtx& c, unsigned half_mask) {
   uint32_t y[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -125,6 +149,19 @@ __device__ __forceinline__ uint4 qk_norm_rope_vector(const uint4& raw, const uin
 __device__ __forceinline__ void qk_weight_pairs(const __nv_bfloat16* wt, int sub, uint32_t (&w)[4]) {
   const uint4 wraw = *reinterpret_cast<const uint4*>(wt + sub * 8);
   w[0] = wraw.x; w[1] = wraw.y; w[2] = wraw.z; w[3] = wraw.w;
+}
+
+// Where a head vector of a token goes (slot -1: not to the cache).
+__device__ __forceinline__ void qk_put_q(const QkNormRopeParams& p, int tok, int hd, int sub, const uint4& out) {
+  *reinterpret_cast<uint4*>(p.q_out + (static_cast<long long>(tok) * p.H + hd) * 128 + sub * 8) = out;
+}
+__device__ __forceinline__ void qk_put_k(const QkNormRopeParams& p, int tok, int hd, int sub, long long slot, const uint4& out) {
+  const int kh = hd - p.H;
+  *reinterpret_cast<uint4*>(p.k_out + (static_cast<long long>(tok) * p.Hkv + kh) * 128 + sub * 8) = out;
+  if (slot >= 0) *reinterpret_cast<uint4*>(p.k_cache + (slot * p.Hkv + kh) * 128 + sub * 8) = out;
+}
+__device__ __forceinline__ void qk_put_v(const QkNormRopeParams& p, int hd, int sub, long long slot, const uint4& raw) {
+  if (slot >= 0) *reinterpret_cast<uint4*>(p.v_cache + (slot * p.Hkv + (hd - p.H - p.Hkv)) * 128 + sub * 8) = raw;     // a bit copy
 }
 
 template <int GROUP>
@@ -144,38 +181,65 @@ qk_norm_rope_store_kernel(const QkNormRopeParams p) {
   const int stride = gridDim.x * (kQkThreads / 16) / groups;              // tokens (the host sees to it that it is >= 1)
   const int tok0 = worker / groups, hd0 = (worker - tok0 * groups) * GROUP;
   const unsigned half_mask = 0xffffu << (threadIdx.x & 16);
-  // Launched with programmatic stream serialization (a decode kernel in front lets it start early).  The projection's rows, the
-  // outputs and the cache are touched behind the wait.  Positions, slots, the rotary table and the norm weights are not written by
-  // any kernel that lets this one start early, so the decode-sized form has them in registers by then, and its row on the way to
-  // L2: what is left behind the wait is one trip.  28 layers of a decode graph, producer and attention: one sequence 201 -> 187 us,
-  // 37 of 100 .. 1024 tokens 564 -> 531, 256 of 100 .. 2048 at 2/1 heads 845 -> 804 (192, 539, 813 without the hint for the row).
+  // Launched with programmatic stream serialization (a decode kernel in front lets it start early).  Everything that counts is read
+  // behind the wait, so the kernel in front may write any of it.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const bool store = p.slot_mapping && p.k_cache && p.v_cache, any = tok0 < stride && tok0 < p.n_tokens;
   uint32_t wq[4], wk[4];
-  long long pos = 0;
+  long long pos;
   int slot = -1;
-  QkTokenCtx c;
-  if (GROUP == 1 && any) {
-    pos = p.positions[tok0];
-    if (store) slot = p.slot_mapping[tok0];
-    if (hd0 < p.H + p.Hkv) {
-      // one head per pass: only the weight of its kind (both sets would cost registers the pass does not have)
-      qk_weight_pairs(hd0 < p.H ? p.q_weight : p.k_weight, sub, wq);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) wk[i] = wq[i];
+  if constexpr (GROUP == 1) {
+    // One pass, one head, and one trip behind the wait: the position is read ahead of it as a hint, and what hangs on it or is known
+    // anyway is on its way into L2.  The table row of the hint comes with everything else (in 32-byte loads: four of 16 bytes
+    // cost a layer 0.2 us); position and row are looked at behind the normalisation, and the row is fetched again if the
+    // position has changed.  28 layers of a decode graph, producer and attention, everything behind the wait | this form | table,
+    // weights, slot and position in registers ahead of the wait, which a kernel in front must then not write: one sequence 201 |
+    // 189 | 187 us, 37 of 100 .. 1024 tokens 564 | 535 | 521, 256 of 100 .. 2048 at 2/1 heads 845 | 803 | 795.
+    const __nv_bfloat16* row = p.qkv + static_cast<long long>(tok0) * p.qkv_row_stride + hd0 * 128 + sub * 8;
+    const __nv_bfloat16* wt = hd0 < p.H ? p.q_weight : p.k_weight;
+    const bool rotated = hd0 < p.H + p.Hkv;
+    long long hint = 0;
+    if (any) {
+      if ((sub & 7) == 0) prefetch_l2(row);
+      // (what many half-warps share is asked for by a few of them: requests for one line queue up)
+      if (store && threadIdx.x == 0) prefetch_l2(p.slot_mapping + tok0);
+      if (blockIdx.x < 2 && threadIdx.x < 4) prefetch_l2((threadIdx.x < 2 ? p.q_weight : p.k_weight) + (threadIdx.x & 1) * 64);
+      if (rotated) {
+        hint = ld_cg_s64(p.positions + tok0);
+        if ((sub & 3) == 0) prefetch_l2(qk_table_row(p, hint, sub) + (sub & 8) * 8);
+      }
     }
-    c = qk_token_ctx(p, pos, slot, sub);
-    // (a hint, so it may go out before the row is complete: L2 is where it will be completed)
-    if ((sub & 7) == 0 && hd0 < heads) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.qkv + static_cast<long long>(tok0) * p.qkv_row_stride + hd0 * 128 + sub * 8));
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!any) return;
+    uint4 out = ld_row16(row);
+    if (rotated) {
+      qk_weight_pairs(wt, sub, wq);
+      QkTableRow t = qk_load_table(p, hint, sub);
+      pos = ld_s64(p.positions + tok0);
+      if (store && hd0 >= p.H) slot = ld_s32(p.slot_mapping + tok0);
+      uint32_t ap[4];
+      qk_normalise(out, wq, p.eps, half_mask, ap);
+      if (pos != hint) t = qk_load_table(p, pos, sub);
+      out = qk_rotate(ap, qk_token_ctx(p, t, slot, sub), half_mask);
+    } else if (store) {
+      slot = ld_s32(p.slot_mapping + tok0);
+    }
+    const long long to = slot < p.n_slots ? slot : -1;       // never write outside the cache
+    if (hd0 < p.H) {
+      qk_put_q(p, tok0, hd0, sub, out);
+    } else if (rotated) {
+      qk_put_k(p, tok0, hd0, sub, to, out);
+    } else {
+      qk_put_v(p, hd0, sub, to, out);
+    }
+    return;
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (!any) return;
-  if (GROUP > 1) {
-    qk_weight_pairs(p.q_weight, sub, wq);
-    qk_weight_pairs(p.k_weight, sub, wk);
-    pos = p.positions[tok0];
-    if (store) slot = p.slot_mapping[tok0];
-  }
+  qk_weight_pairs(p.q_weight, sub, wq);
+  qk_weight_pairs(p.k_weight, sub, wk);
+  pos = p.positions[tok0];
+  if (store) slot = p.slot_mapping[tok0];
   // Position and slot are fetched a token ahead: the table row hangs on the position, and two trips in a row are what a
   // pass would otherwise wait for.
   for (int tok = tok0; tok < p.n_tokens; tok += stride) {
@@ -184,7 +248,13 @@ qk_norm_rope_store_kernel(const QkNormRopeParams p) {
 #pragma unroll
     for (int g = 0; g < GROUP; ++g)
       if (hd0 + g < heads) raw[g] = *reinterpret_cast<const uint4*>(row + (hd0 + g) * 128);
-    if (GROUP > 1 || tok != tok0) c = qk_token_ctx(p, pos, slot, sub);
+    const float* cs = qk_table_row(p, pos, sub);
+    QkTableRow t;
+    t.c0 = *reinterpret_cast<const float4*>(cs);
+    t.c1 = *reinterpret_cast<const float4*>(cs + 4);
+    t.s0 = *reinterpret_cast<const float4*>(cs + 64);
+    t.s1 = *reinterpret_cast<const float4*>(cs + 68);
+    const QkTokenCtx c = qk_token_ctx(p, t, slot, sub);
     if (tok + stride < p.n_tokens) {
       pos = p.positions[tok + stride];
       if (store) slot = p.slot_mapping[tok + stride];
@@ -194,17 +264,15 @@ qk_norm_rope_store_kernel(const QkNormRopeParams p) {
       const int hd = hd0 + g;
       if (hd >= heads) break;
       if (hd >= p.H + p.Hkv) {
-        // v head: a bit copy into the cache
-        if (c.slot >= 0)
-          *reinterpret_cast<uint4*>(p.v_cache + (c.slot * p.Hkv + (hd - p.H - p.Hkv)) * 128 + sub * 8) = raw[g];
+        qk_put_v(p, hd, sub, c.slot, raw[g]);
       } else if (hd < p.H) {
-        const uint4 outw = qk_norm_rope_vector(raw[g], wq, c, p.eps, half_mask);
-        *reinterpret_cast<uint4*>(p.q_out + (static_cast<long long>(tok) * p.H + hd) * 128 + sub * 8) = outw;
+        uint32_t ap[4];
+        qk_normalise(raw[g], wq, p.eps, half_mask, ap);
+        qk_put_q(p, tok, hd, sub, qk_rotate(ap, c, half_mask));
       } else {
-        const int kh = hd - p.H;
-        const uint4 outw = qk_norm_rope_vector(raw[g], wk, c, p.eps, half_mask);
-        *reinterpret_cast<uint4*>(p.k_out + (static_cast<long long>(tok) * p.Hkv + kh) * 128 + sub * 8) = outw;
-        if (c.slot >= 0) *reinterpret_cast<uint4*>(p.k_cache + (c.slot * p.Hkv + kh) * 128 + sub * 8) = outw;
+        uint32_t ap[4];
+        qk_normalise(raw[g], wk, p.eps, half_mask, ap);
+        qk_put_k(p, tok, hd, sub, c.slot, qk_rotate(ap, c, half_mask));
       }
     }
   }
@@ -243,6 +311,7 @@ extern "C" int b200_qk_norm_rope_store(const void* qkv, int64_t qkv_row_stride, 
   p.k_weight = static_cast<const __nv_bfloat16*>(k_weight);
   p.cos_sin = cos_sin_cache;
   p.max_position = max_position;
+  p.wide_table = reinterpret_cast<uintptr_t>(cos_sin_cache) % 32 == 0;
   p.eps = eps;
   p.q_out = static_cast<__nv_bfloat16*>(q_out);
   p.k_out = static_cast<__nv_bfloat16*>(k_out);

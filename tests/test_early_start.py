@@ -169,3 +169,25 @@ def test_producer_behind_a_kernel_that_writes_its_rows(late_copy, n):
         q, k, _ = qk_norm_rope_store(m["qkv"], pos, w["q"], w["k"], table, 1e-6, h, hkv, *caches, slots)
         return (q, k, *caches)
     _compare(late_copy, _rows(1, **shape), _rows(2, **shape), _caches(n // 256 + 1, hkv), call)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shift", [0, 4])                       # the table at a multiple of 32 bytes, and of 16 only
+@pytest.mark.parametrize("n,h,hkv", [(1, 16, 8), (37, 16, 8), (256, 2, 1), (3000, 16, 8)])
+def test_producer_behind_a_kernel_that_writes_everything_else(late_copy, n, h, hkv, shift):
+    from nanovllm_b200.layers.qk_norm_rope import qk_norm_rope_store
+    blocks = n // 256 + 2
+    qkv = _rows(1, qkv=(n, (h + 2 * hkv) * 128))["qkv"]
+
+    def metadata(seed):
+        g = torch.Generator().manual_seed(seed)
+        pos = torch.randint(0, 1000, (n,), generator=g)
+        pos[::5] = torch.arange(0, n, 5) % 1000                  # some stay as they were
+        return dict(pad=torch.zeros(4 + shift, dtype=torch.int32), table=torch.randn(1000, 1, 128, generator=g),
+                    pos=pos, slots=_slots(n, blocks * 256, seed), **_rows(seed, q=(128,), k=(128,)))
+
+    def call(m, caches):
+        assert m["table"].data_ptr() % 32 == (4 + shift) * 4 % 32
+        q, k, _ = qk_norm_rope_store(qkv, m["pos"], m["q"], m["k"], m["table"], 1e-6, h, hkv, *caches, m["slots"])
+        return (q, k, *caches)
+    _compare(late_copy, metadata(2), metadata(3), _caches(blocks, hkv), call)
