@@ -23,8 +23,8 @@
  *    b200_store_decode_attn and b200_prefill_attn / b200_store_prefill_attn start early behind a kernel that lets its
  *    dependents do so (griddepcontrol.launch_dependents), and read part of their metadata before they wait for it:
  *      decode                 context_lens, block_tables; b200_store_decode_attn also slot_mapping
- *      prefill                cu_seqlens_q, cu_seqlens_k
- *      store, producer        nothing (what they read ahead they read again)
+ *      prefill, tcgen05       cu_seqlens_q, cu_seqlens_k
+ *      store, producer, prefill on mma.sync     nothing (what the first two read ahead they read again)
  *    So a kernel that lets its dependents start early must not write these arrays.  Of this library the store,
  *    producer, decode and mma.sync prefill kernels do (they write cache rows, q, k and outputs only); the metadata unpack,
  *    all-reduce and tcgen05 prefill kernels do not.  Behind any other kernel or copy there is nothing to observe.

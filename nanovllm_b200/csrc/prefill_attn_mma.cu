@@ -79,26 +79,25 @@ prefill_attn_mma_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
     mbar_init(&bar_last, 1);
     mbar_fence_init();
   }
-  // Which sequence and query tile this is, ahead of the wait: no kernel that lets this one start early writes cu_seqlens.  Every
-  // CTA waits, those with nothing to do as well, so that this launch ends behind the kernel in front.  Per launch in a graph of
-  // launches, 16/8 heads: 1 prompt of 33 tokens 4.14 -> 3.84 us, 8 of 60 5.5 -> 4.95, 128 of 20 36.6 -> 35.1; 4/2 heads, 32 of 100
-  // 10.9 -> 10.0.
   const int h = blockIdx.x % p.Hkv;
   const int x = p.n_slots - 1 - static_cast<int>(blockIdx.x / p.Hkv);  // later (heavier) tiles first
+  // Everything is read behind the wait, so the kernel in front may write any of it.  Every CTA waits, those with nothing to do as
+  // well, so that this launch ends behind that kernel.  (The search ahead of it, which bars the kernel in front from writing
+  // cu_seqlens: per launch in a graph of launches, 16/8 heads, 1 prompt of 33 tokens 3.99 -> 3.84 us, 8 of 60 5.5 -> 4.95, 128 of 20
+  // 36.0 -> 35.1; as a hint that is checked behind the wait 3.96, 5.5 and 38.3.)
+  asm volatile("griddepcontrol.wait;" ::: "memory");
 
   // slot -> (sequence, query tile): sequence i owns slots [cu_q[i] / QT + i, ... + ceil(Lq_i / QT))
   int lo = 0, hi = p.batch;
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
-    if (__ldg(p.cu_q + mid) / QT + mid <= x) lo = mid; else hi = mid;
+    if (ld_s32(p.cu_q + mid) / QT + mid <= x) lo = mid; else hi = mid;
   }
   const int seq = lo;
-  const int q_begin = __ldg(p.cu_q + seq), q_end = __ldg(p.cu_q + seq + 1);
-  const int Lq = q_end - q_begin;
+  const int q_begin = ld_s32(p.cu_q + seq), q_end = ld_s32(p.cu_q + seq + 1);
+  const int k_begin = ld_s32(p.cu_k + seq);
+  const int Lq = q_end - q_begin, Lk = ld_s32(p.cu_k + seq + 1) - k_begin;
   const int qt = x - (q_begin / QT + seq);
-  const int k_begin = __ldg(p.cu_k + seq);
-  const int Lk = __ldg(p.cu_k + seq + 1) - k_begin;
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   const bool storing = warp > kPfConsumerWarps, st_v = warp == kPfConsumerWarps + 2;
   char* const st_cache = st_v ? p.st_v_cache : p.st_k_cache;
   const char* const st_src = st_v ? p.st_v : p.st_k;
@@ -107,11 +106,11 @@ prefill_attn_mma_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
     if (!p.st_slots) return;
     // rows that belong to no query block: sequences without queries, rows outside cu_seqlens_k
     for (int i = blockIdx.x; i < p.batch; i += gridDim.x)
-      if (__ldg(p.cu_q + i) == __ldg(p.cu_q + i + 1))
-        pf_store_rows(p, st_src, st_stride, st_cache, __ldg(p.cu_k + i), min(__ldg(p.cu_k + i + 1), p.st_tokens), 0, p.Hkv, lane);
+      if (ld_s32(p.cu_q + i) == ld_s32(p.cu_q + i + 1))
+        pf_store_rows(p, st_src, st_stride, st_cache, ld_s32(p.cu_k + i), min(ld_s32(p.cu_k + i + 1), p.st_tokens), 0, p.Hkv, lane);
     if (blockIdx.x == 0) {
-      pf_store_rows(p, st_src, st_stride, st_cache, 0, min(__ldg(p.cu_k), p.st_tokens), 0, p.Hkv, lane);
-      pf_store_rows(p, st_src, st_stride, st_cache, __ldg(p.cu_k + p.batch), p.st_tokens, 0, p.Hkv, lane);
+      pf_store_rows(p, st_src, st_stride, st_cache, 0, min(ld_s32(p.cu_k), p.st_tokens), 0, p.Hkv, lane);
+      pf_store_rows(p, st_src, st_stride, st_cache, ld_s32(p.cu_k + p.batch), p.st_tokens, 0, p.Hkv, lane);
     }
   }
   if (qt < 0 || qt * QT >= Lq) return;
