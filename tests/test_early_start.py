@@ -223,3 +223,78 @@ def test_mma_prefill_behind_a_kernel_that_writes_its_metadata(late_copy, h, hkv,
     cache = tuple(torch.randn(blocks, 256, hkv, 128, device=DEV).to(torch.bfloat16) for _ in range(2))
     for f in (call, layer) if n < 500 and not paged else (call,):          # (the layer takes the other kernel for more)
         _compare(late_copy, metadata(before, 2), metadata(lq, 3), _caches(blocks, hkv), f)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bucket,bs,h,hkv", [(4, 3, 16, 8), (48, 37, 16, 8), (64, 64, 2, 1)])     # a cluster per pair, whole pairs
+def test_graph_of_unpack_producer_and_decode_on_changing_metadata(bucket, bs, h, hkv):
+    """A decode step as one graph, two layers: the record's unpack, then producer and attention of each layer, which start early one
+    behind the other.  Positions, slots, lengths and tables change with every replay; the same calls with a
+    synchronisation behind each are the reference, bit for bit, and the oracles within their tolerances."""
+    import random
+    import nanovllm_b200
+    from nanovllm_b200.engine.decode_metadata import DecodeMetadataStager
+    from nanovllm_b200.layers.qk_norm_rope import qk_norm_rope_store
+    from nanovllm_b200.utils.context import reset_context, set_context
+    from oracle.attention_oracle import decode_attn_ref
+    from oracle.metadata_oracle import prepare_decode_ref
+    from oracle.qk_norm_rope_oracle import qk_norm_rope_ref, rope_cos_sin_cache
+    from test_decode_metadata import FakeSeq, _fake_batch
+    from test_qk_norm_rope import _one_step
+    cols, blocks, layers = 8, 600, 2
+    ints = lambda *s, dtype=torch.int32: torch.zeros(*s, dtype=dtype, device=DEV)  # noqa: E731
+    gv = dict(input_ids=ints(bucket, dtype=torch.int64), positions=ints(bucket, dtype=torch.int64), slot_mapping=ints(bucket) - 1,
+              context_lens=ints(bucket), block_tables=ints(bucket, cols))
+    w = _rows(1, q=(128,), k=(128,))
+    table = rope_cos_sin_cache(128, 4096, 1e6).to(DEV)
+    qkv = torch.zeros(layers, bucket, (h + 2 * hkv) * 128, dtype=torch.bfloat16, device=DEV)
+    shape = (layers, blocks, 256, hkv, 128)
+    stager = DecodeMetadataStager(bucket, cols, 256, DEV)
+    att = nanovllm_b200.Attention(h, 128, default_scale(128), hkv)
+
+    def step(record, kv, sync):
+        stager.unpack_into(record, **gv)
+        sync()
+        out = []
+        for i in range(layers):
+            att.k_cache, att.v_cache = kv["k"][i], kv["v"][i]
+            q, k, v = qk_norm_rope_store(qkv[i], gv["positions"], w["q"], w["k"], table, 1e-6, h, hkv, kv["k"][i], kv["v"][i],
+                                         gv["slot_mapping"])
+            sync()
+            out += [q, k, att(q, k, v, already_stored=True)]
+            sync()
+        return out
+
+    rng = random.Random(bucket)
+
+    def batch():                                                     # (one sequence with a full row of the table: one record size)
+        seqs = _fake_batch(rng, bs - 1, 2000, blocks - cols)
+        return seqs + [FakeSeq(rng.randint(7 * 256 + 1, 8 * 256), list(range(blocks - cols, blocks)), 1)]
+
+    set_context(False, slot_mapping=gv["slot_mapping"], context_lens=gv["context_lens"], block_tables=gv["block_tables"])
+    with torch.inference_mode():
+        replayed, stepped = _rows(2, k=shape, v=shape), _rows(2, k=shape, v=shape)
+        stager.pack(batch())
+        record = stager.to_device().clone()
+        step(record, _rows(2, k=shape, v=shape), lambda: None)       # warm-up, on caches of its own
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = step(record, replayed, lambda: None)
+        for turn in range(4):
+            seqs = batch()
+            stager.pack(seqs)
+            record.copy_(stager.to_device())
+            qkv.copy_(_rows(turn + 3, x=qkv.shape)["x"])
+            torch.cuda.synchronize()
+            graph.replay()
+            torch.cuda.synchronize()
+            want = step(record, stepped, torch.cuda.synchronize)
+            for x, y in zip(got + list(replayed.values()), want + list(stepped.values())):
+                assert torch.equal(x.view(torch.int16), y.view(torch.int16))
+            _, pos, _, lens, bt = prepare_decode_ref(seqs, 256)
+            ref = qk_norm_rope_ref(qkv[0, :bs].cpu(), pos, w["q"].cpu(), w["k"].cpu(), table.cpu(), 1e-6, h, hkv, 128)
+            _one_step(got[0][:bs].cpu(), ref[0])
+            out = decode_attn_ref(got[0][:bs].cpu(), replayed["k"][0].cpu(), replayed["v"][0].cpu(), lens, bt, default_scale(128))
+            torch.testing.assert_close(got[2][:bs].float().cpu(), out.float(), atol=2e-2, rtol=1e-2)
+            assert not got[2][bs:].any()                             # padded rows
+    reset_context()
