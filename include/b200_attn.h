@@ -252,6 +252,11 @@ int b200_test_inject_timeout(void);
  * seconds[2] (host memory) with what they took, -1 where a wait did not report that it gave up. */
 int b200_test_wait_limits(float* seconds);
 
+/* Test hook, never called by the product, needs no device: CTAs per (sequence, kv head) that b200_decode_attn gives a batch of
+ * `pairs` of them, with a block table of max_tiles x 64 tokens, on a chip that holds on_chip[0 .. 3] (host memory) clusters of
+ * 8, 4, 2 and 1 CTAs at a time; 0: the general kernel. */
+int b200_test_cluster_rule(int64_t pairs, int32_t heads_per_kv_head, int32_t max_tiles, const int32_t* on_chip);
+
 #ifdef __cplusplus
 }
 #endif

@@ -54,6 +54,7 @@ SIGNATURES = {
     "b200_device_status": (c_int32, []),
     "b200_test_inject_timeout": (c_int32, []),
     "b200_test_wait_limits": (c_int32, [c_void_p]),
+    "b200_test_cluster_rule": (c_int32, [c_int64, c_int32, c_int32, c_void_p]),
 }
 
 

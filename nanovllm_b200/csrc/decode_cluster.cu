@@ -291,44 +291,86 @@ static size_t cluster_smem_bytes(int G, int ctas) {
          static_cast<size_t>(kCluWarps + ctas) * G * 130 * 4;
 }
 
-// CTAs per (sequence, kv head), or 0: leave the batch to the general kernel.  What is known on the host is the number of
-// pairs and the capacity of a block-table row.  One CTA per SM and clusters of at most 8 (of 16 only a few fit on the chip
-// at a time), so up to 8 CTAs per pair for 9 pairs, 4 for 33, and so on; and a pair's CTAs must be able to bear the
-// longest pair the table allows: beyond kCluMaxTiles each (8 us at the 66 GB/s that one SM draws) the general
-// kernel, which cuts long pairs as it needs, is the faster one.  Both sides, us per layer of a decode graph with the producer
-// in front, this kernel | the general one:
-//   a table of 16 columns (4096 tokens), 16/8 heads, taken here: 1 of 562 tokens 6.9 | 9.0, 4 of 562 7.7 | 9.8, 1 of 4000
-//     10.3 | 11.4, 4 of 500 .. 4000 13.2 | 14.5; but 2 .. 4 of which one has 4000 and the others 200: 13.4 | 11.5;
-//   the same table, left to the general kernel: 6 of 562 8.4 | 10.1, 18 of 562 12.2 | 15.3; but 6 with one of 4000
-//     20.7 | 11.9, 12 of 500 .. 4000 33.9 | 24.7;
-//   40 columns, left to the general kernel from 33 on: 1 of 562 7.2 | 9.0, 4 of 562 7.7 | 9.8; but 4 with one of
-//     4000 13.5 | 11.6, and of 160 columns 2 with one of 30000 61.9 | 32.6.
-// So the line on the table's width is what keeps the worst case near the general kernel's, and it costs short sequences
-// under a wide table 20 %.  Of clusters of 4, 33 fit on the chip at a time (what a GPC has left over stays idle): 34 .. 37 pairs would
-// take two rounds and go on clusters of 2, or, under wider tables, to the general kernel.  17 sequences of 562 tokens, 4/2
-// heads, on clusters of 4 | 2 | the general kernel: 11.7 | 7.6 | 9.4 us, 18 of 50 .. 2000 14.4 | 12.4 | 10.6.
-constexpr int kCluMaxTiles = 16;
+// CTAs per (sequence, kv head), or 0: leave the batch to the general kernel.  What is known on the host is the number of pairs
+// and the width of the block table, not the lengths.
+//
+// Size: the largest of which all pairs are on the chip at once, a second round costs as much as the first.  How many are is the
+// runtime's answer for this kernel (one CTA per SM; what a GPC has left over stays idle): 15 clusters of 8, 33 of 4, 74 of 2
+// on a B200.  Us per layer of a decode graph with the producer in front, one kv head: 13 sequences of 50 .. 2000 tokens on clusters
+// of 8 | 4 7.8 | 8.9, 16 of them 12.5 | 9.1; 33 of 562 on 4 | 2 7.3 | 7.7, 34 of them 11.8 | 7.7; 74 of 562 on 2 | 1
+// 9.5 | 9.1, 75 of them 15.3 | 9.2.  (More than 8 CTAs: of clusters of 16 only a few fit.)
+//
+// Table: a pair's CTAs must be able to bear the longest pair that it allows, which the general kernel cuts as it needs.  Both
+// sides as above, this kernel | the general one, at the line and beyond it, tables filled evenly from 50 tokens on; one
+// sequence filling the table among ones of 200; and sequences of 562 (200) tokens under it, which is what the line costs:
+//   clusters of 8, 128 tiles   9 sequences 13.0 | 12.6; 13.0 | 11.1; 6.3 | 8.3      (64 tiles 9.3 | 10.5; 9.0 | 9.5; 6.3 | 8.3)
+//   clusters of 4, 64 tiles   24 sequences 12.7 | 11.8; 12.6 | 9.8; 7.0 | 9.0       (48 tiles 10.8 | 11.2; 10.5 | 9.6; 7.0 | 8.9)
+//   clusters of 2, 20 tiles   50 sequences 10.1 | 10.6; 9.8 | 9.2; 8.0 | 9.9        (32 tiles 12.8 | 11.8; 12.7 | 9.1; 8.0 | 9.9)
+//   lone CTAs, 16 tiles      110 sequences 12.0 | 12.9; 11.8 | 10.0; 6.4 | 7.8      (75 sequences 11.9 | 10.9; 11.6 | 9.7; 6.5 | 7.6)
+// 16/8 heads, filled evenly: clusters of 2, 32 tiles, 5 sequences 12.1 | 10.9, 9 14.2 | 13.4; lone CTAs, 16 tiles, 12 sequences
+// 11.3 | 11.9, 18 13.2 | 13.8.  So the line lies where tables that are filled stop gaining; clusters of 4 and 8 go beyond that, to
+// the 16 columns of 256 tokens under which an engine of 4096 tokens runs all its batches, short ones for the most part.
+constexpr int kCluSizes = 4;                            // of 8, 4, 2 and 1 CTAs
+constexpr int kCluMaxTiles[kCluSizes] = {128, 64, 20, 16};
+int decode_cluster_rule(long long pairs, int G, int max_tiles, const int* on_chip) {
+  if (G > kCluMaxG) return 0;
+  for (int i = 0; i < kCluSizes; ++i) {
+    const int c = 8 >> i;
+    if (pairs <= on_chip[i] && c * G <= 32 && c / 2 < max_tiles) return max_tiles <= kCluMaxTiles[i] ? c : 0;
+  }
+  return 0;
+}
+
+// Leave for the largest launch there is.
+static int cluster_configure(bool store) {
+  static std::atomic<size_t> configured[2][kMaxDevices];
+  auto* const kernel = store ? decode_cluster_kernel<true> : decode_cluster_kernel<false>;
+  return ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), cluster_smem_bytes(kCluMaxG, 8), configured[store],
+                             "decode_attn(cluster): cudaFuncSetAttribute");
+}
+
+// How many clusters of 8 >> i CTAs the current device holds at a time (0: not known).
+static int clusters_on_chip(int i) {
+  static std::atomic<int> known[kMaxDevices][kCluSizes];
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
+  if ((n = known[dev][i].load(std::memory_order_acquire)) > 0) return n;
+  if (cluster_configure(false)) return 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(8u >> i);
+  cfg.blockDim = dim3(kCluThreads);
+  cfg.dynamicSmemBytes = cluster_smem_bytes(kCluMaxG, 8);  // (one CTA per SM with any number of heads)
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 8u >> i;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, decode_cluster_kernel<false>, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  known[dev][i].store(n, std::memory_order_release);
+  return n;
+}
+
 int decode_cluster_ctas(int batch, int Hkv, int G, int max_tiles) {
-  const int sms = sm_count();
   const long long pairs = static_cast<long long>(batch) * Hkv;
-  if (G > kCluMaxG || pairs > sms) return 0;
-  int c = 8;
-  while (c > 1 && (c * pairs > (c == 8 ? sms / 2 : c == 4 ? sms - sms / 9 : sms) || c * G > 32 || c / 2 >= max_tiles)) c /= 2;
-  return max_tiles <= c * kCluMaxTiles ? c : 0;
+  if (G > kCluMaxG || pairs > sm_count()) return 0;
+  int on_chip[kCluSizes];
+  for (int i = 0; i < kCluSizes; ++i) on_chip[i] = clusters_on_chip(i);
+  return decode_cluster_rule(pairs, G, max_tiles, on_chip);
 }
 
 int launch_decode_cluster(const DecodeParams& p, const CUtensorMap& map_k, const CUtensorMap& map_v, const CUtensorMap& map_k16,
                           const CUtensorMap& map_v16, int ctas_per_pair, cudaStream_t stream) {
-  const size_t smem = cluster_smem_bytes(p.G, ctas_per_pair);
-  static std::atomic<size_t> configured[2][kMaxDevices];
   auto* const kernel = p.st_slots ? decode_cluster_kernel<true> : decode_cluster_kernel<false>;
-  int rc = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem, configured[p.st_slots != nullptr],
-                               "decode_attn(cluster): cudaFuncSetAttribute");
+  const int rc = cluster_configure(p.st_slots != nullptr);
   if (rc) return rc;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(p.batch * p.Hkv * ctas_per_pair));
   cfg.blockDim = dim3(kCluThreads);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = cluster_smem_bytes(p.G, ctas_per_pair);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

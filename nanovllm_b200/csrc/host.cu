@@ -144,6 +144,11 @@ int b200_test_inject_timeout(void) {
   return b200::inject_timeout_prefill_tc2();
 }
 
+int b200_test_cluster_rule(int64_t pairs, int32_t heads_per_kv_head, int32_t max_tiles, const int32_t* on_chip) {
+  if (!on_chip) return b200::set_error(b200::kErrNullPointer, "test_cluster_rule: null pointer");
+  return b200::decode_cluster_rule(pairs, heads_per_kv_head, max_tiles, on_chip);
+}
+
 int b200_test_wait_limits(float* seconds) {
   if (!seconds) return b200::set_error(b200::kErrNullPointer, "test_wait_limits: null pointer");
   return b200::test_wait_limits(seconds);

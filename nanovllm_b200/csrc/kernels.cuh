@@ -57,6 +57,8 @@ int reset_state_decode_cluster();
 int reset_state_prefill_mma();
 int reset_state_prefill_tc2();
 int inject_timeout_prefill_tc2();   // test hook: leaves the unit as an abandoned launch would
+// The rule of decode_cluster_ctas() on a chip that holds on_chip[i] clusters of 8 >> i CTAs at a time, i < 4.
+int decode_cluster_rule(long long pairs, int G, int max_tiles, const int* on_chip);
 int test_wait_limits(float* seconds);   // test hook: what the bounded waits (mbar_wait, t2_wait_timed) take to give up
 
 }  // namespace b200

@@ -78,3 +78,20 @@ def test_product_does_not_import_the_oracle():
             "print(bad); sys.exit(1 if bad else 0)") % ROOT
     res = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True)
     assert res.returncode == 0, res.stdout + res.stderr
+
+
+@pytest.mark.parametrize("on_chip", [(15, 33, 74, 148), (16, 36, 72, 144), (0, 20, 60, 132)])
+def test_decode_clusters_go_by_what_the_chip_holds(lib, on_chip):
+    """Pairs get the largest cluster of which all are on the chip at a time, whatever the chip; no more CTAs than tiles; and the
+    general kernel where the table allows more than a cluster of that size can bear."""
+    arr = (ctypes.c_int32 * 4)(*on_chip)
+    rule = lambda pairs, g, tiles: lib.b200_test_cluster_rule(pairs, g, tiles, arr)  # noqa: E731
+    sizes, line = (8, 4, 2, 1), (128, 64, 20, 16)
+    for i, c in enumerate(sizes):
+        if on_chip[i]:
+            assert rule(on_chip[i], 1, 12) == c
+        assert rule(on_chip[i] + 1, 1, 12) == (sizes[i + 1] if i < 3 else 0)
+        if on_chip[i]:
+            assert rule(on_chip[i], 1, line[i]) == c and rule(on_chip[i], 1, line[i] + 1) == 0
+    assert [rule(1, 2, t) for t in (1, 2, 3, 4, 5)] == [1, 2, 4, 4, 8 if on_chip[0] else 4]
+    assert rule(1, 8, 12) == 4 and rule(1, 9, 12) == 0                       # room for the hand-off of 8 heads, 32 rows in a cluster

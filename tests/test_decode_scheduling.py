@@ -56,6 +56,13 @@ def test_decode_between_cluster_sizes(kind, n, h, hkv):
     test_decode_shares(kind, n, h, hkv)
 
 
+@pytest.mark.parametrize("kind,n,h,hkv", [("ragged", 15, 4, 1), ("ragged", 16, 4, 1), ("8000", 15, 2, 1), ("4000", 33, 2, 1), ("1200", 74, 2, 1),
+                                          ("1300", 74, 2, 1), ("1000", 75, 2, 1), ("1100", 75, 2, 1), ("700", 148, 2, 1), ("700", 149, 2, 1), ("1", 15, 8, 1)])
+def test_decode_at_the_lines_of_the_cluster_rule(kind, n, h, hkv):
+    """The last and the first number of pairs on clusters of a size, the last and the first width of a table."""
+    test_decode_shares(kind, n, h, hkv)
+
+
 @pytest.mark.parametrize("slots", ["own", "anywhere", "holes"])
 @pytest.mark.parametrize("n,h,hkv", [(1, 16, 8), (3, 8, 8), (9, 2, 1), (70, 4, 2), (140, 2, 1), (20, 16, 8), (37, 16, 8), (160, 8, 4),
                                      (161, 4, 2), (513, 2, 1)])
