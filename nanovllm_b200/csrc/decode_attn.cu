@@ -31,9 +31,17 @@ extern std::atomic<long long> g_launches;
 
 constexpr int kDecStages = 3;
 // Tiles that a CTA's first unit has on their way into L2 ahead of the wait (at most 8), while the kernel in front ends and the
-// memory is idle.  Us per layer of a graph with the producer in front at 3 | 5 | 6 | 8: 37 sequences of 100 .. 1024 tokens,
-// 16/8 heads, 18.9 | 18.4 | 18.4 | 19.0; 256 of 100 .. 2048, 2/1 heads, 29.1 | 28.6 | 28.6 | 28.7.
-constexpr int kDecAhead = 5;
+// memory is idle: as many as the ring has stages, or, from kDecAheadShare tiles per CTA on, five.  Us per layer of a graph with the
+// producer in front, by tiles per CTA, at 3 | 5 tiles:
+//   4.4   90 of 20 .. 400 tokens, 8/4 heads      12.9 | 13.4      10.5  200 of 30 .. 900, 4/2          23.3 | 23.2
+//   4.8   256 of 50 .. 600, 2/1                  14.2 | 14.8      12.3  400 of 100 .. 1000, 4/1        27.0 | 26.0
+//   6.2   200 of 30 .. 500, 4/2                  15.9 | 16.7      12.5  50 of 100 .. 1024, 16/8        24.2 | 24.4
+//   7.3   400 of 30 .. 600, 4/1                  18.0 | 18.9      14.9  256 of 100 .. 2048, 2/1        28.9 | 28.5
+//   8.4   200 of 30 .. 700, 4/2                  18.9 | 19.3      15.8  512 of 100 .. 1000, 4/1        30.3 | 29.2
+//   9.4   400 of 30 .. 800, 4/1                  23.5 | 23.0      11.8  12 of 300 .. 9000, 16/4        26.5 | 26.1
+// (6.0, 90 of 500 .. 700, 4/2: 15.4 | 14.9).  Six and eight: the same as five within 0.3 us except 37 of 100 .. 1024, 16/8, at 8
+// (19.1, 20.0) and the last (25.8).  Blocks of 512 and 1024 tokens give the same picture.
+constexpr int kDecAhead = 5, kDecAheadShare = 9;
 constexpr int kDecProducerWarp = kDecConsumerWarps;
 constexpr int kDecEpilogueWarp = kDecConsumerWarps + 1;
 constexpr int kDecThreads = kDecConsumers + 64;
@@ -72,6 +80,7 @@ struct DecUnits {
   const unsigned char* tail;                 // tokens of a sequence's last tile - 1
   int cap;                                   // tiles a part may have
   int live;                                  // sequences with tokens
+  int ahead;                                 // tiles of a CTA's first unit to fetch ahead of the wait
   bool split, wide;                          // some pair is cut; some tile count does not fit 16 bits
   __device__ __forceinline__ UnitDesc get(const DecodeParams& p, int u) const {
     UnitDesc d;
@@ -353,6 +362,7 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
       }
     }
     un.live = live;
+    un.ahead = tiles < static_cast<long long>(kDecAheadShare) * grid ? kDecStages : kDecAhead;
     un.split = longest > un.cap;
     un.wide = longest >= 65535;
     // size classes: without cuts all 64 for the whole pairs, else 32 for the parts and, behind them, 32 for the whole pairs
@@ -486,7 +496,7 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
     int cur_blk1 = cur_col0 + 1 < p.bt_cols ? cur_bt[cur_col0 + 1] : -1;
     // Bring the first tiles into L2 while the kernel in front still runs: nothing is read, so it does not matter
     // that that kernel may be writing this step's rows.
-    dec_prefetch_tiles(p, map_k, map_v, cur.h, cur.t0, min(cur.t1, cur.t0 + kDecAhead), cur.len, lane, cur_col0, cur_blk0, cur_blk1);
+    dec_prefetch_tiles(p, map_k, map_v, cur.h, cur.t0, min(cur.t1, cur.t0 + un.ahead), cur.len, lane, cur_col0, cur_blk0, cur_blk1);
     if (lane != 0) return;
     asm volatile("griddepcontrol.wait;" ::: "memory");   // from here on: query rows and the cache
     while (true) {
