@@ -326,8 +326,8 @@ decode_attn_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map
     }
     // Pairs are cut only if the longest one is well above a CTA's equal share of the tiles: whole pairs, longest first,
     // level out well enough below that and leave nothing to merge.  The line is 1.25 shares, or 1.85 where
-    // every CTA has at most one pair (short and long ones share an SM then, and the long one gets the SM's bandwidth when
-    // the short one is done: us per layer with the producer, whole | cut, at 1.46 shares 25.7 | 27.2, 1.73 20.3 | 22.4, 1.93
+    // every CTA has at most one pair (short and long ones share an SM then, and the long one, which ends the launch, goes
+    // faster when the others are done: a tile takes a CTA 1.38 us while all 296 stream and 0.57 us, its chain, on its own; us per layer with the producer, whole | cut, at 1.46 shares 25.7 | 27.2, 1.73 20.3 | 22.4, 1.93
     // 26.7 | 26.6, with 32 tiles a share 59.0 | 54.0, 2.05 19.4 | 20.5, 2.3 25.2 | 23.2, 2.9 49.3 | 39.1), and 3 tiles, which is what a merge costs (90 sequences of 20 .. 400 tokens, 4 kv heads:
     // 14.6 -> 11.5 us uncut).  Above it, pairs longer than 2/3 of a share (and kDecMinPart tiles) are cut into
     // equal parts: 1/2 and 1/3 leave parts of a size that do not add up to a share, and cost more merges (measured over

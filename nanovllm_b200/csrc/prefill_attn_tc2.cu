@@ -51,12 +51,14 @@ static __device__ int g_status_prefill_tc2 = 0;
 static __device__ unsigned int g_prefill_ticket = 0;
 
 // The kernel's bounded waits.  Six roles run through their loops at the same time and share the SM's instruction cache, so code
-// size is time here: with these in place of mbar_wait() (64-bit clock arithmetic and a spin counter at each of
-// some thirty places), the output and rescaling loops rolled and the mask taken from bits, 256 prompts of 100 .. 1024 tokens with
-// the store went from 805 to 700 us, 256 of 10 .. 300 without it from 162 to 142.  (With 78 KB of code in place of 62 a tcgen05 kernel of
-// this kind waited 2.5 times as long for instructions.)  The form with the store was 78 KB and is 64 with one output path instead of two, shifts for
-// divisions by powers of two, table columns counted along and one copy of the row loop: 256 prompts of 100 .. 1024 tokens
-// 838 -> 794 us with the store, 616 -> 602 without it (57 KB for 63), 64 of 10 .. 300 58 -> 54.
+// size is time here.  Us for 256 prompts of 100 .. 1024 tokens with the store | without it, 256 of 10 .. 300 without it, in four launches
+// after a rest (in 300 launches on end, at the power cap):
+//   mbar_wait() (64-bit clock arithmetic and a spin counter at each of some thirty places), output and rescaling
+//     loops unrolled, a mask by comparisons                                 803 | 657, 167  (885 | 766, 185)
+//   these waits, those loops rolled, the mask from bits of one word         702 | 609, 146  (823 | 725, 170)
+//   one output path instead of two, shifts for divisions by powers of two, table columns counted along and one copy
+//     of the store's row loop: 64 KB of code for 78 with the store          653 | 598, 134  (770 | 713, 159)
+// So the store in the launch costs 55 us; a launch of its own in front of the form without it 181 (782 for both, 884 on end).
 //
 // How long the hardware suspends a failed test is its own affair, so a count of tests is a limit but not one in time.  The time
 // limit is the producer's, on the low word of the clock: it sets the abort flag, which every other wait looks at after a
@@ -202,7 +204,7 @@ __device__ __forceinline__ void t2_output_split(const PrefillParams& p, const CU
 }
 
 // The layer's cache store (nanovllm/layers/attention.py:10-40) on the side.  Attention over dense K and V does not read
-// the cache, so the copy needs no launch of its own in front of it (193 us on 143872 tokens at 16/8 heads), and every
+// the cache, so the copy needs no launch of its own in front of it (193 us on 143872 tokens at 16/8 heads, 55 in this one), and every
 // K and V tile passes through shared memory anyway: the item whose query block is the first to need a tile sends it on,
 // warp 2 the K tiles and warp 3 the V tiles, as TMA stores of 32 rows where the slots run on (they do inside a block),
 // else row by row.  Nothing is read from memory for it but the slots.
