@@ -82,21 +82,27 @@ prefill_attn_mma_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
   const int h = blockIdx.x % p.Hkv;
   const int x = p.n_slots - 1 - static_cast<int>(blockIdx.x / p.Hkv);  // later (heavier) tiles first
   // Everything is read behind the wait, so the kernel in front may write any of it.  Every CTA waits, those with nothing to do as
-  // well, so that this launch ends behind that kernel.  (The search ahead of it, which bars the kernel in front from writing
-  // cu_seqlens: per launch in a graph of launches, 16/8 heads, 1 prompt of 33 tokens 3.99 -> 3.84 us, 8 of 60 5.5 -> 4.95, 128 of 20
-  // 36.0 -> 35.1; as a hint that is checked behind the wait 3.96, 5.5 and 38.3.)
+  // well, so that this launch ends behind that kernel.
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  // slot -> (sequence, query tile): sequence i owns slots [cu_q[i] / QT + i, ... + ceil(Lq_i / QT))
-  int lo = 0, hi = p.batch;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (ld_s32(p.cu_q + mid) / QT + mid <= x) lo = mid; else hi = mid;
+  // slot -> (sequence, query tile): sequence i owns slots [cu_q[i] / QT + i, ... + ceil(Lq_i / QT)).  Each warp looks for itself, 32
+  // places at a time; the last look has the sequence's bounds as well.  Per launch in a graph of launches, a binary search behind the
+  // wait | ahead of it, which bars the kernel in front from writing cu_seqlens | this: 16/8 heads, 1 prompt of 33 tokens 3.98 | 3.85 |
+  // 4.11 us, 8 of 60 5.5 | 4.9 | 5.1, 128 of 20 36.0 | 35.1 | 30.1; 4/2, 32 of 100 10.5 | 10.0 | 9.7; 2/1, 256 of 10 10.7 | 9.5 | 8.1.
+  int seq = 0, left = p.batch;
+  while (left > 31) {
+    const int step = (left + 31) / 32, i = seq + lane * step;
+    const unsigned below = __ballot_sync(0xffffffffu, lane * step < left && ld_s32(p.cu_q + min(i, p.batch)) / QT + i <= x);
+    const int skip = max(__popc(below) - 1, 0) * step;
+    seq += skip;
+    left = min(step, left - skip);
   }
-  const int seq = lo;
-  const int q_begin = ld_s32(p.cu_q + seq), q_end = ld_s32(p.cu_q + seq + 1);
-  const int k_begin = ld_s32(p.cu_k + seq);
-  const int Lq = q_end - q_begin, Lk = ld_s32(p.cu_k + seq + 1) - k_begin;
+  const int cq = ld_s32(p.cu_q + min(seq + lane, p.batch)), ck = ld_s32(p.cu_k + min(seq + lane, p.batch));
+  int at = 0;
+  if (left > 1) at = max(__popc(__ballot_sync(0xffffffffu, lane < left && cq / QT + seq + lane <= x)) - 1, 0);
+  seq += at;
+  const int q_begin = __shfl_sync(0xffffffffu, cq, at), Lq = __shfl_sync(0xffffffffu, cq, at + 1) - q_begin;
+  const int k_begin = __shfl_sync(0xffffffffu, ck, at), Lk = __shfl_sync(0xffffffffu, ck, at + 1) - k_begin;
   const int qt = x - (q_begin / QT + seq);
   const bool storing = warp > kPfConsumerWarps, st_v = warp == kPfConsumerWarps + 2;
   char* const st_cache = st_v ? p.st_v_cache : p.st_k_cache;

@@ -51,3 +51,22 @@ def test_tcgen05_items(paged, h, hkv, lq, lk):
     torch.cuda.synchronize()
     ref = prefill_attn_ref(q, k, v, cu_q, cu_k, scale).float()
     torch.testing.assert_close(out.float().cpu(), ref, atol=2e-2, rtol=1e-2)
+
+
+@pytest.mark.parametrize("h,hkv", [(2, 1), (64, 1)])                 # 64 query tokens to a CTA, one or two
+@pytest.mark.parametrize("batch", [1, 2, 30, 31, 32, 33, 63, 64, 961, 962, 1023, 1100])
+def test_mma_finds_its_sequence(batch, h, hkv):
+    """The mma.sync kernel's search, 32 places at a time: batches around a power of 32, sequences without queries first, last and
+    in a row, a query tile of several sequences and sequences of several tiles."""
+    from nanovllm_b200.layers.attention import prefill_attention
+    g = torch.Generator().manual_seed(batch)
+    lq = [0 if i % 7 in (0, 5, 6) and batch > 2 else 1 + (i * 37) % 3 for i in range(batch)]
+    lq[batch // 2] = 70
+    lk = [m + i % 3 for i, m in enumerate(lq)]
+    n = sum(lk)
+    q = torch.randn(sum(lq), h, 128, generator=g).to(torch.bfloat16)
+    k, v = (torch.randn(n, hkv, 128, generator=g).to(torch.bfloat16) for _ in range(2))
+    cu_q, cu_k = cu_seqlens(lq), cu_seqlens(lk)
+    out = prefill_attention(q.to(DEV), k.to(DEV), v.to(DEV), cu_q.to(DEV), cu_k.to(DEV), max(lq), max(lk), default_scale(128), hkv, None, 1)
+    want = prefill_attn_ref(q, k, v, cu_q, cu_k, default_scale(128))
+    torch.testing.assert_close(out.float().cpu(), want.float(), atol=2e-2, rtol=1e-2)
