@@ -674,7 +674,7 @@ prefill_attn_tc2_kernel(const PrefillParams p, const __grid_constant__ CUtensorM
       // (segment g: sequence g - 1; 0 and batch + 1: the rows in front of the first and behind the last)
 #pragma unroll 1
       for (int g = blockIdx.x; g < p.batch + 2; g += gridDim.x) {
-        const int r0 = g == 0 ? 0 : __ldg(p.cu_k + g - 1), r1 = g > p.batch ? p.st_tokens : __ldg(p.cu_k + g);
+        const int r0 = g == 0 ? 0 : __ldg(p.cu_k + g - 1), r1 = g > p.batch ? p.st_tokens : min(__ldg(p.cu_k + g), p.st_tokens);
         if (g == 0 || g > p.batch || __ldg(p.cu_q + g - 1) == __ldg(p.cu_q + g)) t2_store_rows(p, src, stride, cache, r0, r1, lane);
       }
     }

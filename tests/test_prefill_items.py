@@ -70,3 +70,26 @@ def test_mma_finds_its_sequence(batch, h, hkv):
     out = prefill_attention(q.to(DEV), k.to(DEV), v.to(DEV), cu_q.to(DEV), cu_k.to(DEV), max(lq), max(lk), default_scale(128), hkv, None, 1)
     want = prefill_attn_ref(q, k, v, cu_q, cu_k, default_scale(128))
     torch.testing.assert_close(out.float().cpu(), want.float(), atol=2e-2, rtol=1e-2)
+
+
+@pytest.mark.parametrize("h,hkv,lens", [(16, 8, [60, 70]), (2, 1, [700, 31, 2000]), (2, 2, [900] * 40)])     # mma.sync, tcgen05 in both forms
+def test_store_ends_with_the_rows_of_k(h, hkv, lens):
+    """cu_seqlens_k that run past total_k, in a sequence without queries: rows there are not read, whatever kernel takes the call.
+    (k, v and slots go on behind total_k, so that a store of these rows would show in the cache.)"""
+    from nanovllm_b200 import _lib
+    n, beyond = sum(lens) + 40, 60
+    g = torch.Generator(device=DEV).manual_seed(n)
+    q = torch.randn(sum(lens), h, 128, device=DEV, generator=g).to(torch.bfloat16)
+    k, v = (torch.randn(n + beyond, hkv, 128, device=DEV, generator=g).to(torch.bfloat16) for _ in range(2))
+    kc, vc = (torch.zeros(-(-(n + beyond) // 256), 256, hkv, 128, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    slots = torch.arange(n + beyond, dtype=torch.int32, device=DEV)
+    cu_q, cu_k = cu_seqlens(lens + [0]).to(DEV), cu_seqlens(lens + [40 + beyond]).to(DEV)
+    out = torch.empty_like(q)
+    _lib.check(_lib.load().b200_store_prefill_attn(
+        q.data_ptr(), h * 128, k.data_ptr(), v.data_ptr(), hkv * 128, hkv * 128, n, kc.data_ptr(), vc.data_ptr(), slots.data_ptr(),
+        kc.shape[0] * 256, cu_q.data_ptr(), cu_k.data_ptr(), len(lens) + 1, sum(lens), max(lens), max(lens + [40 + beyond]), out.data_ptr(), h, hkv, 128,
+        default_scale(128), torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    for cache, rows in ((kc, k), (vc, v)):
+        flat = cache.view(-1, hkv, 128)
+        assert torch.equal(flat[:n], rows[:n]) and not flat[n:].any()
