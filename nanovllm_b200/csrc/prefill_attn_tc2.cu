@@ -126,7 +126,7 @@ __device__ __forceinline__ void t2_open_box(bool tma, int lane) {
   if (tma && lane == 0) tma_store_wait_read_but_one();
   __syncwarp();
 }
-// `row0`: the output row (token * H + head) of the warp's first tile row, `rows`: how many of its 32 are query rows.
+// `head0`, `tok0`: head and token of the warp's first tile row, `rows`: how many of its 32 are query rows.
 __device__ __forceinline__ void t2_close_box(const PrefillParams& p, const CUtensorMap* map_o, const unsigned char* box, bool tma, int lane, int gs,
                                              int bx, int head0, int tok0, int rows) {
   if (tma) {
