@@ -115,28 +115,29 @@ def test_store_bit_exact(b200, dtype, hkv, d, n):
     assert torch.equal(vc.cpu().view(view), v_cache.view(view))
 
 
-@pytest.mark.parametrize("over", [-1, 3])
-def test_store_index_width(b200, over):
-    """Either side of 2^31 16-byte vectors, where the index becomes 64-bit: only the first and the last rows have a slot."""
+@pytest.mark.parametrize("over,d", [(-1, 8), (3, 8), (3, 16)])
+def test_store_index_width(b200, over, d):
+    """Either side of 2^31 16-byte vectors, where the index becomes 64-bit, and beyond 2^32, where one of 32 bits would come round: only
+    the first and the last rows have a slot."""
     pkg, _ = b200
     n = (1 << 30) + over
     torch.cuda.empty_cache()
-    free, need = torch.cuda.mem_get_info()[0], n * 20 + (1 << 30)              # k and the slots, and something for the rest
+    free, need = torch.cuda.mem_get_info()[0], n * (2 * d + 4) + (1 << 30)     # k and the slots, and something for the rest
     if free < need:
         pytest.skip(f"needs {need >> 30} GiB of free device memory, {free >> 30} are there")
-    k = torch.empty(n, 1, 8, dtype=torch.bfloat16, device=DEV)
+    k = torch.empty(n, 1, d, dtype=torch.bfloat16, device=DEV)
     slots = torch.full((n,), -1, dtype=torch.int32, device=DEV)
     rows = torch.cat([torch.arange(5), n - 1 - torch.arange(5)])
-    k[rows.to(DEV)] = torch.arange(80, dtype=torch.bfloat16, device=DEV).view(10, 1, 8)
+    k[rows.to(DEV)] = torch.arange(10 * d, dtype=torch.bfloat16, device=DEV).view(10, 1, d)
     slots[rows.to(DEV)] = torch.arange(10, dtype=torch.int32, device=DEV)
-    kc = torch.full((1, 256, 1, 8), -1, dtype=torch.bfloat16, device=DEV)
+    kc = torch.full((1, 256, 1, d), -1, dtype=torch.bfloat16, device=DEV)
     vc = torch.full_like(kc, -2)
     pkg.store_kvcache(k, k, kc, vc, slots)
     torch.cuda.synchronize()
     del k, slots
     torch.cuda.empty_cache()
     for c, rest in ((kc, -1), (vc, -2)):
-        assert torch.equal(c[0, :10].float().cpu(), torch.arange(80.).view(10, 1, 8)) and bool((c[0, 10:] == rest).all())
+        assert torch.equal(c[0, :10].float().cpu(), torch.arange(10. * d).view(10, 1, d)) and bool((c[0, 10:] == rest).all())
 
 
 def test_store_empty_and_all_skipped(b200):
@@ -378,7 +379,7 @@ def _variants(h, hkv):
 
 
 @pytest.mark.parametrize("variant", ["mma", "tcgen05"])
-@pytest.mark.parametrize("h,hkv", [(16, 8), (4, 1), (2, 2), (5, 1), (8, 1), (32, 1), (64, 1)])
+@pytest.mark.parametrize("h,hkv", [(16, 8), (4, 1), (2, 2), (5, 1), (8, 1), (32, 1), (64, 1), (128, 1)])
 def test_prefill_dense_ragged(b200, h, hkv, variant):
     pkg, _ = b200
     if variant not in _variants(h, hkv):
@@ -414,7 +415,7 @@ def test_prefill_paged_prefix_poisoned(b200, h, hkv, variant):
     _status_ok()
 
 
-@pytest.mark.parametrize("h,hkv", [(4, 2), (64, 1)])
+@pytest.mark.parametrize("h,hkv", [(4, 2), (64, 1), (128, 1)])
 @pytest.mark.parametrize("block_size,cols", [(256, None), (512, None), (768, None), (256, 3)])
 def test_prefill_paged_block_sizes(b200, block_size, cols, h, hkv):
     """Tiles counted along the block table: blocks of two, four and six tiles, the last one ragged; a table that ends before the
